@@ -2426,12 +2426,13 @@ __global__ void __launch_bounds__(kThreads, LB) k_batch(BatchParams B)
 struct Workspace {
     int G;                 // grid blocks of the persistent kernel
     int lb;                // register-budget variant (blocks per SM it was built for)
-    // every solver vector lives in one block, the FP64 CG set first, so one L2
-    // access-policy window covers what a solve touches:
-    //   p | q | r | x | s | t | rh | p32 | s32 | p16 | s16 | p8 | s8
-    // (CG, FP64 / mixed: p..x; BiCGSTAB, FP64 / mixed: p..rh; parity mode: all)
+    // every solver vector lives in one block, ordered so that one L2
+    // access-policy window can cover any number of the vectors a solve reuses
+    // most (vec_window):
+    //   x | p | q | r | s | t | rh | p32 | s32 | p16 | s16 | p8 | s8
+    // (CG, FP64 / mixed: x..r; BiCGSTAB, FP64 / mixed: x..rh; parity mode: all)
     char *vecs;
-    size_t cg_bytes, bicg_bytes, all_bytes;
+    size_t vec_bytes, all_bytes;   // one FP64 vector; the whole block
     double *r, *p, *q, *rh, *s, *t, *x;
     float *p32, *s32, *mag_p, *mag_s;
     __half *p16, *s16;
@@ -2573,15 +2574,14 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
     const long long S = std::max(A->tilem, A->tilen) + 1;
     {
         const size_t f = (size_t)L * sizeof(float), d = (size_t)L * sizeof(double), h = (size_t)L * sizeof(__half);
-        w->cg_bytes = 4 * d;
-        w->bicg_bytes = 7 * d;
+        w->vec_bytes = d;
         w->all_bytes = 7 * d + 2 * f + 2 * h + 2 * (size_t)L;
         MF_CUDA_TRY(cudaMalloc((void **)&w->vecs, w->all_bytes));
         char *c = w->vecs;
+        w->x = (double *)c; c += d;
         w->p = (double *)c; c += d;
         w->q = (double *)c; c += d;
         w->r = (double *)c; c += d;
-        w->x = (double *)c; c += d;
         w->s = (double *)c; c += d;
         w->t = (double *)c; c += d;
         w->rh = (double *)c; c += d;
@@ -2726,6 +2726,43 @@ struct L2Window {
     }
 };
 
+// The part of the vector block to keep in L2 for a solve (0 bytes: no window).
+//  * Nothing when the vectors and the matrix stream fit in three quarters of L2
+//    together: the window changed no solve time below that (96^3 CG and
+//    BiCGSTAB, 256^2: within 1 %) and setting it up and back costs 50 us a call.
+//  * Whole vectors only, as many as fit in 7/8 of the persisting set-aside
+//    (72 of 83 MB): a window wider than the set-aside marks part of its lines
+//    streaming, and those thrash (2048^2 CG with all four vectors, 134 MB:
+//    20.5 ms per 100 iterations, 10.5 without a window; 160^3: 3.5 against 3.1).
+//    CG takes r first (read by the SpMV and the update, written by the update),
+//    then q, p and x; BiCGSTAB p, q, r, s, t, rh, then x.
+//    Measured per 24 CG iterations, no window -> this rule: 128^3 1.41 -> 1.23,
+//    144^3 2.18 -> 1.98 (p, q, r), 160^3 3.13 -> 2.82 (q, r), 2048^2 3.22 ->
+//    2.97 (q, r), 2500^2 4.81 -> 4.37 ms (r); 112^3 BiCGSTAB 1.22 -> 1.17.
+struct VecWindow {
+    void *base;
+    size_t bytes;
+};
+
+VecWindow vec_window(const Workspace *w, int mode, int method, size_t matrix_bytes)
+{
+    int dev = 0, l2 = 0, persist = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&persist, cudaDevAttrMaxPersistingL2CacheSize, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return {w->vecs, 0};
+    }
+    const size_t room = (size_t)(persist > 0 ? persist : 0) / 8 * 7, d = w->vec_bytes;
+    const bool bicg = method == MF_METHOD_BICGSTAB;
+    const size_t used = bicg ? 7 : 4;
+    if (mode == MODE_PARITY) return {w->vecs, w->all_bytes <= room ? w->all_bytes : 0};
+    if (used * d + matrix_bytes <= (size_t)l2 / 4 * 3) return {w->vecs, 0};
+    const size_t k = std::min(used, d > 0 ? room / d : 0);
+    char *base = k == used ? w->vecs : bicg ? (char *)w->p : (char *)(w->r + d / sizeof(double)) - k * d;
+    return {base, k * d};
+}
+
 }  // namespace
 
 void mf_solver_free_ws(mf_matrix_s *A)
@@ -2818,9 +2855,11 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     // (the FP64 / mixed modes never touch the narrow shadows: a smaller
     // persisting set-aside leaves more of L2 to the matrix stream -- measured
     // 3.5 % faster on the 128^3 system than a window that included p32)
-    if (opt->l2_window)
-        win.set(s, w->vecs, mode == MODE_PARITY ? w->all_bytes
-                            : opt->method == MF_METHOD_BICGSTAB ? w->bicg_bytes : w->cg_bytes);
+    if (opt->l2_window) {
+        const size_t value = mode != MODE_MIXED ? 8 : P.lean_f16 ? 2 : 4;
+        const VecWindow vw = vec_window(w, mode, opt->method, (size_t)A->slice_entries * (value + 1));
+        if (vw.bytes > 0) win.set(s, vw.base, vw.bytes);
+    }
     const auto t_prepared = std::chrono::steady_clock::now();
     MF_CUDA_TRY(cudaEventRecord(w->e0, s));
     cudaError_t lerr = cudaLaunchCooperativeKernel(solve_kernel(mode, w->lb, opt->method), dim3(w->G), dim3(kThreads), args, 0, s);
