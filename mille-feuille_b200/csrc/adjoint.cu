@@ -47,7 +47,8 @@ extern "C" int mf_value_grad(mf_matrix A, int nrhs, const double *lambda, const 
     const double *dl = lambda, *dx = x;
     double *dg = grad_val, *tmp = nullptr;
     if (!device_ptrs) {
-        MF_CUDA_TRY(cudaMallocAsync((void **)&tmp, (nl + nx + ne) * sizeof(double) + 16, s));
+        const int rc = mf_pool_array(&tmp, (long long)(nl + nx + ne), s);
+        if (rc != MF_SUCCESS) return rc;
         MF_CUDA_TRY(cudaMemcpyAsync(tmp, lambda, nl * sizeof(double), cudaMemcpyHostToDevice, s));
         MF_CUDA_TRY(cudaMemcpyAsync(tmp + nl, x, nx * sizeof(double), cudaMemcpyHostToDevice, s));
         dl = tmp;
@@ -63,7 +64,7 @@ extern "C" int mf_value_grad(mf_matrix A, int nrhs, const double *lambda, const 
     }
     if (!device_ptrs) {
         MF_CUDA_TRY(cudaMemcpyAsync(grad_val, dg, ne * sizeof(double), cudaMemcpyDeviceToHost, s));
-        MF_CUDA_TRY(cudaFreeAsync(tmp, s));
+        mf_pool_free(tmp, s);
     }
     MF_CUDA_TRY(cudaStreamSynchronize(s));
     return MF_SUCCESS;

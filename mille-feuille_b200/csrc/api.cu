@@ -101,8 +101,13 @@ __global__ void k_check_rowptr(const int *rowptr, int n, long long nnz, int *err
     }
 }
 
+// Work on any stream may still use the handle's arrays, so the device is
+// synchronised first (as cudaFree does); the frees themselves are then
+// stream-ordered on an idle device.
 void free_matrix(mf_matrix_s *A)
 {
+    MfDeviceGuard guard(A->dev);
+    if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
     mf_solver_free_ws(A);
     void *ptrs[] = {A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, A->d_tile_ptr, A->d_tile_columnidx,
                     A->d_csr_offset, A->d_csrptr_offset, A->d_tval, A->d_tval_low, A->d_tcol, A->d_tptr,
@@ -111,9 +116,9 @@ void free_matrix(mf_matrix_s *A)
                     A->d_val_i8_ref, A->d_val_i8, A->d_i8_scale, A->d_tile_caps, A->d_seg_ptr, A->d_seg_tile0,
                     A->d_seg_off, A->d_seg_hdr, A->d_seg_tile, A->d_seg_kp, A->d_seg_rowlen, A->d_meta, A->d_v64, A->d_v32, A->d_v16,
                     A->d_v8, A->d_v8ref, A->d_row_cost};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
-    if (A->stage) cudaFree(A->stage);
+    for (void *p : ptrs) mf_pool_free(p, 0);
+    mf_pool_free(A->stage, 0);
+    mf_pool_settle(A->dev);
     delete A;
 }
 
@@ -121,13 +126,16 @@ void free_matrix(mf_matrix_s *A)
 // and grown when a call needs more, so a solve allocates and frees nothing once
 // warm (a stream-ordered allocation per call was returned to the driver at the
 // call's closing synchronisation and mapped again on the next call).
-int stage_get(mf_matrix_s *A, size_t bytes, double **out)
+int stage_get(mf_matrix_s *A, size_t bytes, double **out, cudaStream_t s)
 {
     if (A->stage_bytes < bytes) {
-        if (A->stage) cudaFree(A->stage);
+        if (A->stage) {
+            MF_CUDA_TRY(cudaDeviceSynchronize());   // a call on another stream may still read it
+            mf_pool_free(A->stage, 0);
+        }
         A->stage = nullptr;
         A->stage_bytes = 0;
-        MF_CUDA_TRY(cudaMalloc(&A->stage, bytes));
+        MF_TRY(mf_pool_alloc(&A->stage, bytes, s));
         A->stage_bytes = bytes;
     }
     *out = (double *)A->stage;
@@ -165,12 +173,11 @@ extern "C" int mf_matrix_create(mf_matrix *out, int n_rows, int n_cols, long lon
     const cudaMemcpyKind kind = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     int rc = MF_SUCCESS;
     auto fail = [&](int code) { free_matrix(A); return code; };
-    if (cudaMalloc((void **)&A->d_rowptr, (size_t)(n_rows + 1) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc((void **)&A->d_colidx, (size_t)std::max<long long>(nnz, 1) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc((void **)&A->d_val, (size_t)std::max<long long>(nnz, 1) * sizeof(double)) != cudaSuccess)
-        return fail(MF_ERR_NOMEM);
-    if (val_low && cudaMalloc((void **)&A->d_val_low, (size_t)std::max<long long>(nnz, 1) * sizeof(float)) != cudaSuccess)
-        return fail(MF_ERR_NOMEM);
+    if ((rc = mf_pool_array(&A->d_rowptr, (long long)n_rows + 1, s)) != MF_SUCCESS ||
+        (rc = mf_pool_array(&A->d_colidx, nnz, s)) != MF_SUCCESS ||
+        (rc = mf_pool_array(&A->d_val, nnz, s)) != MF_SUCCESS)
+        return fail(rc);
+    if (val_low && (rc = mf_pool_array(&A->d_val_low, nnz, s)) != MF_SUCCESS) return fail(rc);
     if (cudaMemcpyAsync(A->d_rowptr, rowptr, (size_t)(n_rows + 1) * sizeof(int), kind, s) != cudaSuccess ||
         (nnz > 0 && cudaMemcpyAsync(A->d_colidx, colidx, (size_t)nnz * sizeof(int), kind, s) != cudaSuccess) ||
         (nnz > 0 && cudaMemcpyAsync(A->d_val, val, (size_t)nnz * sizeof(double), kind, s) != cudaSuccess) ||
@@ -178,13 +185,14 @@ extern "C" int mf_matrix_create(mf_matrix *out, int n_rows, int n_cols, long lon
          cudaMemcpyAsync(A->d_val_low, val_low, (size_t)nnz * sizeof(float), kind, s) != cudaSuccess))
         return fail(MF_ERR_CUDA);
     int *d_err = nullptr;
-    if (cudaMalloc((void **)&d_err, sizeof(int)) != cudaSuccess) return fail(MF_ERR_NOMEM);
+    if ((rc = mf_pool_array(&d_err, 1, s)) != MF_SUCCESS) return fail(rc);
     cudaMemsetAsync(d_err, 0, sizeof(int), s);
     if (n_rows > 0) k_check_rowptr<<<(n_rows + 255) / 256, 256, 0, s>>>(A->d_rowptr, n_rows, nnz, d_err);
     int h_err = 0;
     cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) { cudaFree(d_err); return fail(MF_ERR_CUDA); }
-    cudaFree(d_err);
+    const cudaError_t se = cudaStreamSynchronize(s);
+    mf_pool_free(d_err, s);
+    if (se != cudaSuccess) return fail(MF_ERR_CUDA);
     if (h_err) return fail(h_err);
     rc = mf_build_tiles(A, s);
     if (rc != MF_SUCCESS) return fail(rc);
@@ -334,7 +342,7 @@ extern "C" int mf_solve(mf_matrix A, const double *b, double *x, const mf_option
     using clk = std::chrono::steady_clock;
     const auto t0 = clk::now();
     if (!device_ptrs) {
-        MF_TRY(stage_get(A, 2 * nb + 16, &tmp));
+        MF_TRY(stage_get(A, 2 * nb + 16, &tmp, s));
         MF_CUDA_TRY(cudaMemcpyAsync(tmp, b, nb, cudaMemcpyHostToDevice, s));
         db = tmp;
         dx = tmp + A->n_rows;
@@ -372,7 +380,7 @@ extern "C" int mf_solve_multi(mf_matrix A, int nrhs, const double *B, double *X,
     const double *dB = B;
     double *dX = X, *tmp = nullptr;
     if (!device_ptrs) {
-        MF_TRY(stage_get(A, 2 * bytes, &tmp));
+        MF_TRY(stage_get(A, 2 * bytes, &tmp, s));
         MF_CUDA_TRY(cudaMemcpyAsync(tmp, B, bytes, cudaMemcpyHostToDevice, s));
         dB = tmp;
         dX = tmp + (size_t)nrhs * A->n_rows;
@@ -486,7 +494,7 @@ extern "C" int mf_spmv(mf_matrix A, const double *x, double *y, int precision, i
     double *dyp = y;
     double *tmp = nullptr;
     if (!device_ptrs) {
-        MF_TRY(stage_get(A, ((size_t)A->n_cols + A->n_rows) * sizeof(double) + 16, &tmp));
+        MF_TRY(stage_get(A, ((size_t)A->n_cols + A->n_rows) * sizeof(double) + 16, &tmp, s));
         MF_CUDA_TRY(cudaMemcpyAsync(tmp, x, (size_t)A->n_cols * sizeof(double), cudaMemcpyHostToDevice, s));
         dxp = tmp;
         dyp = tmp + A->n_cols;
@@ -527,7 +535,7 @@ extern "C" int mf_debug_spmm(mf_matrix A, const double *X, double *Y, int tensor
     const double *dX = X;
     double *dY = Y, *tmp = nullptr;
     if (!device_ptrs) {
-        MF_TRY(stage_get(A, (nx + ny) * sizeof(double), &tmp));
+        MF_TRY(stage_get(A, (nx + ny) * sizeof(double), &tmp, 0));
         MF_CUDA_TRY(cudaMemcpy(tmp, X, nx * sizeof(double), cudaMemcpyHostToDevice));
         dX = tmp;
         dY = tmp + nx;

@@ -128,6 +128,25 @@ __host__ __device__ __forceinline__ long long mf_slot(long long off, int k, int 
 
 void mf_set_last_cuda_error(cudaError_t e, const char *what, const char *file, int line);
 
+// device memory from the library's private pool of the current device (pool.cu):
+// allocated and freed in stream order.  mf_pool_settle gives memory back once
+// nothing of the device's pool is live.
+int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s);
+void mf_pool_free(void *p, cudaStream_t s);
+void mf_pool_settle(int dev);
+template <typename T>
+inline int mf_pool_array(T **p, long long count, cudaStream_t s)
+{
+    return mf_pool_alloc((void **)p, (size_t)(count > 0 ? count : 1) * sizeof(T), s);
+}
+
+// Makes `dev` current for its lifetime (a handle may be destroyed with another device current).
+struct MfDeviceGuard {
+    explicit MfDeviceGuard(int dev);
+    ~MfDeviceGuard();
+    int old;
+};
+
 // device exclusive scans (scan.cu)
 int mf_scan_i32_to_i32(const int *d_in, int *d_out, long long n, cudaStream_t s);   // out[0..n]
 int mf_scan_i32_to_i64(const int *d_in, long long *d_out, long long n, cudaStream_t s);

@@ -84,11 +84,14 @@ int scan_impl(const TI *d_in, TO *d_out, long long n, cudaStream_t s)
     }
     long long nb = (n + kTile - 1) / kTile;
     TO *sums = nullptr, *sums_scanned = nullptr;
-    MF_CUDA_TRY(cudaMallocAsync((void **)&sums, (size_t)(nb + 1) * sizeof(TO), s));
-    MF_CUDA_TRY(cudaMallocAsync((void **)&sums_scanned, (size_t)(nb + 1) * sizeof(TO), s));
+    int rc = mf_pool_array(&sums, nb + 1, s);
+    if (rc == MF_SUCCESS) rc = mf_pool_array(&sums_scanned, nb + 1, s);
+    if (rc != MF_SUCCESS) {
+        mf_pool_free(sums, s);
+        return rc;
+    }
     k_block_scan<TI, TO><<<(unsigned)nb, kThreads, 0, s>>>(d_in, d_out, sums, n);
     MF_CUDA_TRY(cudaGetLastError());
-    int rc;
     if (nb == 1) {
         MF_CUDA_TRY(cudaMemsetAsync(sums_scanned, 0, sizeof(TO), s));
         MF_CUDA_TRY(cudaMemcpyAsync(sums_scanned + 1, sums, sizeof(TO), cudaMemcpyDeviceToDevice, s));
@@ -104,8 +107,8 @@ int scan_impl(const TI *d_in, TO *d_out, long long n, cudaStream_t s)
         k_set_total<TO><<<1, 1, 0, s>>>(d_out, n, sums_scanned, nb);
         MF_CUDA_TRY(cudaGetLastError());
     }
-    MF_CUDA_TRY(cudaFreeAsync(sums, s));
-    MF_CUDA_TRY(cudaFreeAsync(sums_scanned, s));
+    mf_pool_free(sums, s);
+    mf_pool_free(sums_scanned, s);
     return rc;
 }
 

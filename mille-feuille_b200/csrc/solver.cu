@@ -2458,13 +2458,6 @@ struct Workspace {
     cudaEvent_t *m_ev;     // two timing events per column group
 };
 
-template <typename T>
-int dal(T **p, long long count)
-{
-    MF_CUDA_TRY(cudaMalloc((void **)p, (size_t)(count > 0 ? count : 1) * sizeof(T)));
-    return MF_SUCCESS;
-}
-
 #define MF_TRY(expr)                        \
     do {                                    \
         int _rc = (expr);                   \
@@ -2565,7 +2558,10 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
         *out = w;
         return MF_SUCCESS;
     }
-    if (w) mf_solver_free_ws(A);
+    if (w) {
+        MF_CUDA_TRY(cudaDeviceSynchronize());
+        mf_solver_free_ws(A);
+    }
     w = new Workspace();
     memset(w, 0, sizeof(*w));
     w->G = G;
@@ -2576,7 +2572,7 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
         const size_t f = (size_t)L * sizeof(float), d = (size_t)L * sizeof(double), h = (size_t)L * sizeof(__half);
         w->vec_bytes = d;
         w->all_bytes = 7 * d + 2 * f + 2 * h + 2 * (size_t)L;
-        MF_CUDA_TRY(cudaMalloc((void **)&w->vecs, w->all_bytes));
+        MF_TRY(mf_pool_alloc((void **)&w->vecs, w->all_bytes, s));
         char *c = w->vecs;
         w->x = (double *)c; c += d;
         w->p = (double *)c; c += d;
@@ -2591,16 +2587,18 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
         w->s16 = (__half *)c; c += h;
         w->p8 = (int8_t *)c; c += L;
         w->s8 = (int8_t *)c;
+        // zeros past n_rows: a matrix with more columns than rows gathers there
+        MF_CUDA_TRY(cudaMemsetAsync(w->vecs, 0, w->all_bytes, s));
     }
-    MF_TRY(dal(&w->mag_p, S)); MF_TRY(dal(&w->mag_s, S));
-    MF_TRY(dal(&w->lab_p, S)); MF_TRY(dal(&w->lab_s, S));
-    MF_TRY(dal(&w->red, (long long)kRedKinds * G * kRedWidth));
-    MF_TRY(dal(&w->bar, 1)); MF_TRY(dal(&w->err, 1)); MF_TRY(dal(&w->out, 16));
-    MF_TRY(dal(&w->counts, 16));
-    MF_TRY(dal(&w->phase_ns, 8));
+    MF_TRY(mf_pool_array(&w->mag_p, S, s)); MF_TRY(mf_pool_array(&w->mag_s, S, s));
+    MF_TRY(mf_pool_array(&w->lab_p, S, s)); MF_TRY(mf_pool_array(&w->lab_s, S, s));
+    MF_TRY(mf_pool_array(&w->red, (long long)kRedKinds * G * kRedWidth, s));
+    MF_TRY(mf_pool_array(&w->bar, 1, s)); MF_TRY(mf_pool_array(&w->err, 1, s)); MF_TRY(mf_pool_array(&w->out, 16, s));
+    MF_TRY(mf_pool_array(&w->counts, 16, s));
+    MF_TRY(mf_pool_array(&w->phase_ns, 8, s));
     MF_TRY(exact_tiles(A, w->counts, s));    // counts: scratch before the first solve zeroes it
     w->nhw = G * kWarps * 2;
-    MF_TRY(dal(&w->hw_begin, w->nhw + 1));
+    MF_TRY(mf_pool_array(&w->hw_begin, w->nhw + 1, s));
     MF_CUDA_TRY(cudaEventCreate(&w->e0));
     MF_CUDA_TRY(cudaEventCreate(&w->e1));
     k_partition<<<(w->nhw + 256) / 256, 256, 0, s>>>(A->d_row_cost, A->tilem, w->nhw, w->hw_begin);
@@ -2765,14 +2763,14 @@ VecWindow vec_window(const Workspace *w, int mode, int method, size_t matrix_byt
 
 }  // namespace
 
+// (the caller has synchronised the device)
 void mf_solver_free_ws(mf_matrix_s *A)
 {
     Workspace *w = (Workspace *)A->ws;
     if (!w) return;
     void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->bar, w->err, w->out, w->counts,
                     w->phase_ns, w->hw_begin, w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    for (void *p : ptrs) mf_pool_free(p, 0);
     for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
     delete[] w->m_ev;
     cudaEventDestroy(w->e0);
@@ -3123,10 +3121,9 @@ int mf_spmm_run(mf_matrix_s *A, const double *d_X, double *d_Y, int tensor_cores
     MF_TRY(ws_get(A, 0, &w, s));
     const long long L = A->vec_len;
     double *Xi = nullptr, *Yi = nullptr;
-    MF_TRY(dal(&Xi, L * 8));
-    MF_TRY(dal(&Yi, L * 8));
-    int rc = MF_SUCCESS;
-    do {
+    MF_TRY(mf_pool_array(&Xi, L * 8, s));
+    int rc = mf_pool_array(&Yi, L * 8, s);
+    if (rc == MF_SUCCESS) do {
         if (cudaMemsetAsync(Xi, 0, (size_t)L * 8 * sizeof(double), s) != cudaSuccess) { rc = MF_ERR_CUDA; break; }
         k_interleave<<<592, 256, 0, s>>>(d_X, A->n_cols, (int)L, 8, 0, 8, Xi);
         SolverParams P;
@@ -3149,8 +3146,8 @@ int mf_spmm_run(mf_matrix_s *A, const double *d_X, double *d_Y, int tensor_cores
         cudaEventElapsedTime(&ms, w->e0, w->e1);
         if (elapsed_ms) *elapsed_ms = ms;
     } while (0);
-    cudaFree(Xi);
-    cudaFree(Yi);
+    mf_pool_free(Xi, s);
+    mf_pool_free(Yi, s);
     return rc;
 }
 
@@ -3252,8 +3249,8 @@ int ws_multi(mf_matrix_s *A, Workspace *w, int mode, int nr, cudaStream_t s)
 {
     if (w->m_nr == nr && w->m_vec) return MF_SUCCESS;
     void *old[] = {w->m_vec, w->m_mag, w->m_red, w->m_hw_begin};
-    for (void *p : old)
-        if (p) cudaFree(p);
+    if (w->m_vec) MF_CUDA_TRY(cudaDeviceSynchronize());
+    for (void *p : old) mf_pool_free(p, 0);
     w->m_vec = nullptr; w->m_mag = nullptr; w->m_red = nullptr;
     w->m_hw_begin = nullptr;
     w->m_nr = 0;
@@ -3270,10 +3267,10 @@ int ws_multi(mf_matrix_s *A, Workspace *w, int mode, int nr, cudaStream_t s)
     const int need = (A->tilem + kWarps * 2 - 1) / (kWarps * 2);
     if (need < G) G = need > 0 ? need : 1;
     const long long L = A->vec_len, S = std::max(A->tilem, A->tilen) + 1;
-    MF_TRY(dal(&w->m_vec, 5 * L * nr));
-    MF_TRY(dal(&w->m_mag, S));
-    MF_TRY(dal(&w->m_red, (long long)kRedKinds * G * kRedWidthM));
-    MF_TRY(dal(&w->m_hw_begin, (long long)G * kWarps * 2 + 1));
+    MF_TRY(mf_pool_array(&w->m_vec, 5 * L * nr, s));
+    MF_TRY(mf_pool_array(&w->m_mag, S, s));
+    MF_TRY(mf_pool_array(&w->m_red, (long long)kRedKinds * G * kRedWidthM, s));
+    MF_TRY(mf_pool_array(&w->m_hw_begin, (long long)G * kWarps * 2 + 1, s));
     MF_CUDA_TRY(cudaMemsetAsync(w->m_vec, 0, (size_t)5 * L * nr * sizeof(double), s));
     MF_CUDA_TRY(cudaMemsetAsync(w->m_mag, 0, (size_t)S * sizeof(float), s));
     const int nhw = G * kWarps * 2;
@@ -3287,19 +3284,20 @@ int ws_multi(mf_matrix_s *A, Workspace *w, int mode, int nr, cudaStream_t s)
 constexpr int kOutM = 4 * kMaxNR + 8;    // doubles per column group's result record
 
 // Result slots for `groups` column groups (grown, never shrunk).
-int ws_multi_groups(Workspace *w, int groups)
+int ws_multi_groups(Workspace *w, int groups, cudaStream_t s)
 {
     if (w->m_groups >= groups) return MF_SUCCESS;
-    if (w->m_out) cudaFree(w->m_out);
-    if (w->m_err) cudaFree(w->m_err);
+    if (w->m_out) MF_CUDA_TRY(cudaDeviceSynchronize());
+    mf_pool_free(w->m_out, 0);
+    mf_pool_free(w->m_err, 0);
     w->m_out = nullptr;
     w->m_err = nullptr;
     for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
     delete[] w->m_ev;
     w->m_ev = nullptr;
     w->m_groups = 0;
-    MF_TRY(dal(&w->m_out, (long long)groups * kOutM));
-    MF_TRY(dal(&w->m_err, groups));
+    MF_TRY(mf_pool_array(&w->m_out, (long long)groups * kOutM, s));
+    MF_TRY(mf_pool_array(&w->m_err, groups, s));
     w->m_ev = new cudaEvent_t[2 * groups];
     for (int k = 0; k < 2 * groups; k++) MF_CUDA_TRY(cudaEventCreate(&w->m_ev[k]));
     w->m_groups = groups;
@@ -3346,7 +3344,7 @@ int mf_solver_multi_run(mf_matrix_s *A, int nrhs, const double *d_B, double *d_X
     M.mag = w->m_mag;
     M.red = w->m_red;
     const int groups = (nrhs + nr - 1) / nr;
-    MF_TRY(ws_multi_groups(w, groups));
+    MF_TRY(ws_multi_groups(w, groups, s));
     MF_CUDA_TRY(cudaMemsetAsync(w->m_out, 0, (size_t)groups * kOutM * sizeof(double), s));
     MF_CUDA_TRY(cudaMemsetAsync(w->m_err, 0, (size_t)groups * sizeof(int), s));
     // every column group is enqueued back to back (the interleaved buffers are
@@ -3432,8 +3430,9 @@ struct BatchImpl {
         graph = nullptr;
         graph_key.clear();
         void *p[] = {d_items, d_order, d_bptr, d_blist, d_ctl, d_pool};
-        for (void *q : p)
-            if (q) cudaFree(q);
+        MfDeviceGuard guard(dev);
+        if (d_pool && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+        for (void *q : p) mf_pool_free(q, 0);
         d_items = nullptr; d_order = nullptr; d_bptr = nullptr; d_blist = nullptr; d_ctl = nullptr;
         d_pool = nullptr;
     }
@@ -3520,11 +3519,11 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
     {
         // exact-tile counts of the systems (once per matrix)
         unsigned long long *scratch = nullptr;
-        MF_CUDA_TRY(cudaMalloc((void **)&scratch, 3 * sizeof(*scratch)));
+        MF_TRY(mf_pool_array(&scratch, 3, s));
         int rc = MF_SUCCESS;
         for (mf_matrix_s *A : B.sys)
             if (rc == MF_SUCCESS) rc = exact_tiles(A, scratch, s);
-        cudaFree(scratch);
+        mf_pool_free(scratch, s);
         MF_TRY(rc);
     }
     std::vector<double> cost(B.nitems);
@@ -3563,14 +3562,14 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
         }
     }
     B.pool_bytes = total;
-    MF_CUDA_TRY(cudaMalloc((void **)&B.d_pool, total > 0 ? total : 256));
+    MF_TRY(mf_pool_alloc((void **)&B.d_pool, total > 0 ? total : 256, s));
     MF_CUDA_TRY(cudaMemsetAsync(B.d_pool, 0, total > 0 ? total : 256, s));
     int nteam = 0;
     std::vector<int> ctr_of(B.nitems, -1);
     for (int t = 0; t < B.nitems; t++)
         if (B.it_team[t] > 1) ctr_of[t] = nteam++;
     B.ctl_bytes = sizeof(unsigned) * (size_t)(2 + nteam);
-    MF_CUDA_TRY(cudaMalloc((void **)&B.d_ctl, B.ctl_bytes));
+    MF_TRY(mf_pool_alloc((void **)&B.d_ctl, B.ctl_bytes, s));
     B.h_items.resize(B.nitems);
     for (int t = 0; t < B.nitems; t++) {
         const mf_matrix_s *A = B.sys[B.it_sys[t]];
@@ -3592,10 +3591,10 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
         it.M.nr = B.it_ncol[t];
         it.ctr = it.team > 1 ? B.d_ctl + 2 + ctr_of[t] : nullptr;
     }
-    MF_CUDA_TRY(cudaMalloc((void **)&B.d_items, sizeof(BatchItem) * (size_t)std::max(1, B.nitems)));
-    MF_CUDA_TRY(cudaMalloc((void **)&B.d_order, sizeof(int) * (size_t)std::max(1, B.nqueue)));
-    MF_CUDA_TRY(cudaMalloc((void **)&B.d_bptr, sizeof(int) * (size_t)(B.grid + 1)));
-    MF_CUDA_TRY(cudaMalloc((void **)&B.d_blist, sizeof(int2) * (size_t)std::max<size_t>(1, blist.size())));
+    MF_TRY(mf_pool_array(&B.d_items, B.nitems, s));
+    MF_TRY(mf_pool_array(&B.d_order, B.nqueue, s));
+    MF_TRY(mf_pool_array(&B.d_bptr, B.grid + 1, s));
+    MF_TRY(mf_pool_array(&B.d_blist, (long long)blist.size(), s));
     if (B.nitems > 0)
         MF_CUDA_TRY(cudaMemcpyAsync(B.d_items, B.h_items.data(), sizeof(BatchItem) * B.nitems,
                                     cudaMemcpyHostToDevice, s));
@@ -3737,6 +3736,7 @@ void mf_batch_destroy_impl(mf_batch_s *b)
     if (B.e1) cudaEventDestroy(B.e1);
     if (B.e_in) cudaEventDestroy(B.e_in);
     if (B.own) cudaStreamDestroy(B.own);
+    mf_pool_settle(B.dev);
     delete b;
 }
 
@@ -3893,10 +3893,8 @@ int mf_batch_tune_impl(mf_batch_s *b, int precision, int iters, int *chosen, cud
     int rc = MF_SUCCESS;
     for (size_t k = 0; k < B.sys.size() && rc == MF_SUCCESS; k++) {
         const size_t e = (size_t)B.nrhs[k] * B.sys[k]->n_rows;
-        if (cudaMalloc((void **)&bufB[k], 2 * e * sizeof(double) + 16) != cudaSuccess) {
-            rc = MF_ERR_NOMEM;
-            break;
-        }
+        if ((rc = mf_pool_array(&bufB[k], (long long)(2 * e), run)) != MF_SUCCESS) break;
+        if (cudaStreamSynchronize(run) != cudaSuccess) rc = MF_ERR_CUDA;   // the copy below is not on this stream
         bufX[k] = bufB[k] + e;
         std::vector<double> ones(e, 1.0);
         if (cudaMemcpy(bufB[k], ones.data(), e * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -3939,7 +3937,7 @@ int mf_batch_tune_impl(mf_batch_s *b, int precision, int iters, int *chosen, cud
         }
     }
     for (size_t k = 0; k < B.sys.size(); k++)
-        if (bufB[k]) cudaFree(bufB[k]);
+        mf_pool_free(bufB[k], run);
     if (rc == MF_SUCCESS) rc = batch_build_items(B, best, best_lb, run);
     if (chosen) *chosen = best;
     return rc;

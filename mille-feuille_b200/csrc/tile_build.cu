@@ -545,14 +545,29 @@ int grid_for(long long work, int threads)
     return (int)b;
 }
 
+// an array of the handle
 template <typename T>
 int dalloc(T **p, long long count, cudaStream_t s)
 {
-    (void)s;
-    size_t bytes = (size_t)std::max<long long>(count, 1) * sizeof(T);
-    MF_CUDA_TRY(cudaMalloc((void **)p, bytes));
-    return MF_SUCCESS;
+    return mf_pool_array(p, count, s);
 }
+
+// The build's temporaries: freed in stream order when the build ends, on every path.
+struct Temps {
+    cudaStream_t s;
+    std::vector<void *> all;
+    template <typename T>
+    int get(T **p, long long count)
+    {
+        const int rc = mf_pool_array(p, count, s);
+        if (rc == MF_SUCCESS) all.push_back(*p);
+        return rc;
+    }
+    ~Temps()
+    {
+        for (void *p : all) mf_pool_free(p, s);
+    }
+};
 
 }  // namespace
 
@@ -571,11 +586,12 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     A->tilem = tilem;
     A->tilen = tilen;
     A->vec_len = std::max(tilem, tilen) * MF_BS;
+    Temps tmp{s, {}};
     int *d_err = nullptr, *d_maxes = nullptr, *d_span_base = nullptr, *d_ntiles = nullptr;
-    MF_TRY(dalloc(&d_err, 1, s));
-    MF_TRY(dalloc(&d_maxes, 2, s));
-    MF_TRY(dalloc(&d_span_base, tilem, s));
-    MF_TRY(dalloc(&d_ntiles, tilem + 1, s));
+    MF_TRY(tmp.get(&d_err, 1));
+    MF_TRY(tmp.get(&d_maxes, 2));
+    MF_TRY(tmp.get(&d_span_base, tilem));
+    MF_TRY(tmp.get(&d_ntiles, tilem + 1));
     MF_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
     MF_CUDA_TRY(cudaMemsetAsync(d_maxes, 0, 2 * sizeof(int), s));
     MF_CUDA_TRY(cudaMemsetAsync(d_ntiles, 0, (tilem + 1) * sizeof(int), s));
@@ -602,7 +618,7 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     } else {
         global_mode = 1;
         tgrid = 148 * 4;
-        MF_TRY(dalloc(&gscratch, words_per_warp * (long long)tgrid * kWarps, s));
+        MF_TRY(tmp.get(&gscratch, words_per_warp * (long long)tgrid * kWarps));
     }
     if (smem > 48 * 1024) {
         MF_CUDA_TRY(cudaFuncSetAttribute(k_count_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -653,7 +669,7 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
 
     // nonempty-row lists
     int *d_nzr = nullptr;
-    MF_TRY(dalloc(&d_nzr, tilenum + 1, s));
+    MF_TRY(tmp.get(&d_nzr, tilenum + 1));
     MF_TRY(dalloc(&A->d_nonzero_row_new, tilenum + 1, s));
     MF_TRY(dalloc(&A->d_tile_rowidx, tilenum + 1, s));
     MF_TRY(dalloc(&A->d_block_signal, tilem + 4, s));
@@ -681,8 +697,8 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     }
     // row-block split
     int *d_rbc = nullptr, *d_rbo = nullptr;
-    MF_TRY(dalloc(&d_rbc, tilem + 1, s));
-    MF_TRY(dalloc(&d_rbo, tilem + 1, s));
+    MF_TRY(tmp.get(&d_rbc, tilem + 1));
+    MF_TRY(tmp.get(&d_rbo, tilem + 1));
     if (tilem > 0) {
         k_rowblk_count<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_tile_ptr, tilem, d_rbc);
         MF_CUDA_TRY(cudaGetLastError());
@@ -717,7 +733,7 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     }
     // solver slices
     int *d_nseg = nullptr;
-    MF_TRY(dalloc(&d_nseg, tilem + 1, s));
+    MF_TRY(tmp.get(&d_nseg, tilem + 1));
     MF_TRY(dalloc(&A->d_seg_ptr, tilem + 1, s));
     if (tilem > 0) {
         k_seg_count<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_tile_ptr, tilem, d_nseg);
@@ -733,9 +749,9 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     MF_TRY(dalloc(&A->d_seg_tile0, nseg + 1, s));
     MF_TRY(dalloc(&A->d_seg_kp, nseg + 1, s));
     MF_TRY(dalloc(&A->d_seg_rowlen, (long long)nseg * MF_BS + 1, s));
-    MF_TRY(dalloc(&d_seg_entries, nseg + 1, s));
+    MF_TRY(tmp.get(&d_seg_entries, nseg + 1));
     MF_TRY(dalloc(&A->d_seg_off, nseg + 1, s));
-    MF_TRY(dalloc(&d_cost, tilem + 1, s));
+    MF_TRY(tmp.get(&d_cost, tilem + 1));
     MF_TRY(dalloc(&A->d_row_cost, tilem + 1, s));
     if (tilem > 0) {
         k_seg_shape<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_seg_ptr, A->d_csr_offset, A->d_csrptr_offset,
@@ -776,9 +792,6 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
         MF_CUDA_TRY(cudaGetLastError());
     }
     MF_CUDA_TRY(cudaStreamSynchronize(s));
-    cudaFree(d_err); cudaFree(d_maxes); cudaFree(d_span_base); cudaFree(d_ntiles); cudaFree(d_nzr);
-    cudaFree(d_rbc); cudaFree(d_rbo); cudaFree(d_nseg); cudaFree(d_seg_entries); cudaFree(d_cost);
-    if (gscratch) cudaFree(gscratch);
     A->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
     return MF_SUCCESS;
 }
