@@ -8,8 +8,6 @@
 // No counterpart in the reference, which has no differentiation.
 #include "mf_internal.cuh"
 
-#include <cstdlib>
-#include <cstring>
 #include <vector>
 
 namespace {
@@ -70,46 +68,178 @@ extern "C" int mf_value_grad(mf_matrix A, int nrhs, const double *lambda, const 
     return MF_SUCCESS;
 }
 
-// A^T from A's device CSR copy: a stable counting sort by column on the host
-// (entries of a row of A^T keep the order of A's rows, so the result does not
-// depend on scheduling), then the usual GPU tiling.
+// ------------------------------------------------------------ A^T on the GPU
+// The entries of A (their positions in A's row-major order) are sorted by
+// column with a stable least-significant-digit radix sort, so a row of A^T keeps
+// the order of A's rows and the result does not depend on scheduling.  Columns
+// take ceil(log2(n_cols) / 8) passes of 8 bits; a pass is a digit histogram per
+// block, an exclusive scan over (digit, block), and a scatter in which each warp
+// ranks its entries 32 at a time with __match_any_sync.  The passes move 8 bytes
+// an entry each way (column, position) and are bound by the scattered stores;
+// values are moved once, at the end.  A sort rather than counting columns with
+// atomics and sorting each: its time does not depend on the longest column.
+// 48^3 upwind system (760 K entries): 16 ms for the host's counting sort and its
+// copies before, 0.2 ms for the passes now.
+namespace {
+
+constexpr int kTThreads = 256;
+constexpr int kTWarps = kTThreads / 32;
+constexpr int kTRounds = 16;                         // 32-entry rounds per warp
+constexpr int kTTile = kTThreads * kTRounds;         // entries per block: each warp takes a contiguous run
+constexpr int kDigits = 256;
+
+// rowptr -> the row of every entry (entries counted from row 0's first)
+__global__ void k_entry_rows(const int *__restrict__ rowptr, int n_rows, int *__restrict__ row)
+{
+    const int lane = threadIdx.x & 7;                // 8 lanes per row
+    const int base = rowptr[0];
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; i < n_rows; i += (gridDim.x * blockDim.x) >> 3)
+        for (long long e = rowptr[i] + lane; e < rowptr[i + 1]; e += 8) row[e - base] = i;
+}
+
+__global__ void k_digit_hist(const int *__restrict__ key, int n, int shift, int nblocks, int *__restrict__ hist)
+{
+    __shared__ int h[kDigits];
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const long long b0 = (long long)blockIdx.x * kTTile, b1 = b0 + kTTile < n ? b0 + kTTile : n;
+    for (long long e = b0 + threadIdx.x; e < b1; e += kTThreads)
+        atomicAdd(&h[(key[e] >> shift) & (kDigits - 1)], 1);
+    __syncthreads();
+    hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+}
+
+// pos_in == nullptr: the first pass (entry e is at position e)
+__global__ void k_digit_scatter(const int *__restrict__ key, const int *__restrict__ pos_in, int n, int shift,
+                                int nblocks, const int *__restrict__ start, int *__restrict__ key_out,
+                                int *__restrict__ pos_out)
+{
+    __shared__ int cnt[kTWarps][kDigits];            // next output position of each digit, per warp
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int d = lane; d < kDigits; d += 32) cnt[w][d] = 0;
+    __syncwarp();
+    const long long w0 = (long long)blockIdx.x * kTTile + w * 32 * kTRounds;
+    for (int r = 0; r < kTRounds; r++) {
+        const long long e = w0 + r * 32 + lane;
+        if (e < n) atomicAdd(&cnt[w][(key[e] >> shift) & (kDigits - 1)], 1);
+    }
+    __syncthreads();
+    {
+        int at = start[threadIdx.x * nblocks + blockIdx.x];
+        for (int v = 0; v < kTWarps; v++) {
+            const int c = cnt[v][threadIdx.x];
+            cnt[v][threadIdx.x] = at;
+            at += c;
+        }
+    }
+    __syncthreads();
+    for (int r = 0; r < kTRounds; r++) {
+        const long long e = w0 + r * 32 + lane;
+        const bool act = e < n;
+        const int k = act ? key[e] : 0;
+        const int d = act ? (k >> shift) & (kDigits - 1) : kDigits;
+        const unsigned same = __match_any_sync(0xffffffffu, d);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        const int at = act ? cnt[w][d] : 0;
+        __syncwarp();
+        if (act && rank == 0) cnt[w][d] = at + __popc(same);
+        __syncwarp();
+        if (act) {
+            key_out[at + rank] = k;
+            pos_out[at + rank] = pos_in ? pos_in[e] : (int)e;
+        }
+    }
+}
+
+// row pointers of A^T from the sorted columns: row j starts at the first entry of column >= j
+__global__ void k_sorted_rowptr(const int *__restrict__ key, int n, int n_cols, int *__restrict__ tp)
+{
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= n_cols; j += gridDim.x * blockDim.x) {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key[mid] < j) lo = mid + 1;
+            else hi = mid;
+        }
+        tp[j] = lo;
+    }
+}
+
+__global__ void k_gather_entries(const int *__restrict__ pos, int n, const int *__restrict__ row,
+                                 const double *__restrict__ val, const float *__restrict__ low,
+                                 int *__restrict__ tc, double *__restrict__ tv, float *__restrict__ tl)
+{
+    for (long long e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const int p = pos[e];
+        tc[e] = row[p];
+        tv[e] = val[p];
+        if (tl) tl[e] = low[p];
+    }
+}
+
+struct PoolTemps {
+    cudaStream_t s;
+    std::vector<void *> all;
+    template <typename T>
+    int get(T **p, long long count)
+    {
+        const int rc = mf_pool_array(p, count, s);
+        if (rc == MF_SUCCESS) all.push_back(*p);
+        return rc;
+    }
+    ~PoolTemps()
+    {
+        for (void *p : all) mf_pool_free(p, s);
+    }
+};
+
+}  // namespace
+
+// A handle for A^T, built from A's device CSR copy without leaving the GPU.
 extern "C" int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *stream)
 {
     if (!out || !A) return MF_ERR_INVALID;
     *out = nullptr;
     cudaStream_t s = (cudaStream_t)stream;
-    const int m = A->n_rows, n = A->n_cols;
-    const long long nnz = A->nnz;
-    std::vector<int> rp(m + 1), ci(nnz > 0 ? nnz : 1);
-    std::vector<double> va(nnz > 0 ? nnz : 1);
-    std::vector<float> vl(nnz > 0 ? nnz : 1);
-    MF_CUDA_TRY(cudaMemcpyAsync(rp.data(), A->d_rowptr, (m + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
+    const int m = A->n_rows, n = A->n_cols, nnz = (int)A->nnz;
+    int base = 0;                   // entries of rows [0, m) start here
+    MF_CUDA_TRY(cudaMemcpyAsync(&base, A->d_rowptr, sizeof(int), cudaMemcpyDeviceToHost, s));
     MF_CUDA_TRY(cudaStreamSynchronize(s));
-    const long long base = rp[0];   // entries of rows [0, m) start here
+    const int *colidx = A->d_colidx + base;
+    const int nblocks = (nnz + kTTile - 1) / kTTile;
+    PoolTemps tmp{s, {}};
+    int *row, *key[2], *pos[2], *hist, *start, *tp, *tc;
+    double *tv;
+    float *tl = nullptr;
+    int rc = MF_SUCCESS;
+    if ((rc = tmp.get(&row, nnz)) || (rc = tmp.get(&key[0], nnz)) || (rc = tmp.get(&key[1], nnz)) ||
+        (rc = tmp.get(&pos[0], nnz)) || (rc = tmp.get(&pos[1], nnz)) ||
+        (rc = tmp.get(&hist, (long long)kDigits * nblocks)) || (rc = tmp.get(&start, (long long)kDigits * nblocks + 1)) ||
+        (rc = tmp.get(&tp, (long long)n + 1)) || (rc = tmp.get(&tc, nnz)) || (rc = tmp.get(&tv, nnz)) ||
+        (A->d_val_low && (rc = tmp.get(&tl, nnz))))
+        return rc;
     if (nnz > 0) {
-        MF_CUDA_TRY(cudaMemcpyAsync(ci.data(), A->d_colidx + base, nnz * sizeof(int), cudaMemcpyDeviceToHost, s));
-        MF_CUDA_TRY(cudaMemcpyAsync(va.data(), A->d_val + base, nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
-        if (A->d_val_low)
-            MF_CUDA_TRY(cudaMemcpyAsync(vl.data(), A->d_val_low + base, nnz * sizeof(float), cudaMemcpyDeviceToHost, s));
-    }
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    if (!A->d_val_low)
-        for (long long e = 0; e < nnz; e++) vl[e] = (float)va[e];
-    std::vector<int> tp(n + 1, 0), tc(nnz > 0 ? nnz : 1);
-    std::vector<double> tv(nnz > 0 ? nnz : 1);
-    std::vector<float> tl(nnz > 0 ? nnz : 1);
-    for (long long e = 0; e < nnz; e++) {
-        if (ci[e] < 0 || ci[e] >= n) return MF_ERR_INVALID;
-        tp[ci[e] + 1]++;
-    }
-    for (int j = 0; j < n; j++) tp[j + 1] += tp[j];
-    std::vector<int> cur(tp.begin(), tp.end() - 1);
-    for (int i = 0; i < m; i++)
-        for (long long e = rp[i] - base; e < rp[i + 1] - base; e++) {
-            const int d = cur[ci[e]]++;
-            tc[d] = i;
-            tv[d] = va[e];
-            tl[d] = vl[e];
+        k_entry_rows<<<148 * 8, 256, 0, s>>>(A->d_rowptr, m, row);
+        MF_CUDA_TRY(cudaGetLastError());
+        const int *kin = colidx, *pin = nullptr;
+        int at = 0;
+        for (int shift = 0; shift == 0 || (shift < 31 && ((n - 1) >> shift) > 0); shift += 8, at ^= 1) {
+            k_digit_hist<<<nblocks, kTThreads, 0, s>>>(kin, nnz, shift, nblocks, hist);
+            MF_CUDA_TRY(cudaGetLastError());
+            rc = mf_scan_i32_to_i32(hist, start, (long long)kDigits * nblocks, s);
+            if (rc != MF_SUCCESS) return rc;
+            k_digit_scatter<<<nblocks, kTThreads, 0, s>>>(kin, pin, nnz, shift, nblocks, start, key[at], pos[at]);
+            MF_CUDA_TRY(cudaGetLastError());
+            kin = key[at];
+            pin = pos[at];
         }
-    return mf_matrix_create(out, n, m, nnz, tp.data(), tc.data(), tv.data(), tl.data(), 0, stream);
+        k_sorted_rowptr<<<(n + 256) / 256, 256, 0, s>>>(kin, nnz, n, tp);
+        MF_CUDA_TRY(cudaGetLastError());
+        k_gather_entries<<<148 * 8, 256, 0, s>>>(pin, nnz, row, A->d_val + base,
+                                                 A->d_val_low ? A->d_val_low + base : nullptr, tc, tv, tl);
+        MF_CUDA_TRY(cudaGetLastError());
+    } else {
+        MF_CUDA_TRY(cudaMemsetAsync(tp, 0, ((size_t)n + 1) * sizeof(int), s));
+    }
+    return mf_matrix_create(out, n, m, nnz, tp, tc, tv, tl, 1, stream);
 }
