@@ -13,7 +13,7 @@ only what changed.
 
     python mille-feuille_b200/build.py --check
 
-also builds libmillefeuille_check.so: solver.cu and api.cu compiled with
+also builds libmillefeuille_check.so: the solver files and api.cu compiled with
 MF_CHECK, every kernel index taken from stored data checked against its
 array's extent (MF_ERR_CHECK on a failed check; the access is skipped).  Load
 it with MILLEFEUILLE_LIB=<path> in place of libmillefeuille.so.
@@ -37,8 +37,8 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
            "-ccbin", "g++", "-I", INCLUDE]
-SOURCES = ["pool.cu", "scan.cu", "tile_build.cu", "solver.cu", "api.cu", "adjoint.cu", "mmio.cpp"]
-HEADERS = ["mf_internal.cuh"]
+SOURCES = ["pool.cu", "scan.cu", "tile_build.cu", "solver.cu", "multi.cu", "api.cu", "adjoint.cu", "mmio.cpp"]
+HEADERS = ["mf_internal.cuh", "solver_dev.cuh"]
 
 
 def _newer(src: str, dst: str, deps) -> bool:
@@ -84,7 +84,7 @@ def build(verbose: bool = False, check: bool = False) -> str:
     jobs.append(("api.cu", api_fp64, ("MF_CG_INC_FP64",)))
     swap = {}
     if check:
-        for src in ("solver.cu", "api.cu"):
+        for src in ("solver.cu", "multi.cu", "api.cu"):
             obj = os.path.join(BUILD, src.replace(".cu", "_check.cu.o"))
             swap[src + ".o"] = obj
             jobs.append((src, obj, ("MF_CHECK",)))

@@ -195,6 +195,7 @@ int mf_spmv_noalloc_run(mf_matrix_s *A, const double *d_x, double *d_y, int prec
 int mf_ref_labels_run(const double *d_pold, const double *d_pnew, int nseg, int *d_vis,
                       cudaStream_t s);
 void mf_solver_free_ws(mf_matrix_s *A);
+int mf_ws_get(mf_matrix_s *A, int blocks_per_sm, void **out, cudaStream_t s);
 
 // ------------------------------------------------------- device utilities
 #ifdef __CUDACC__
