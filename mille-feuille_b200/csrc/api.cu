@@ -118,6 +118,8 @@ void free_matrix(mf_matrix_s *A)
                     A->d_v8, A->d_v8ref, A->d_row_cost};
     for (void *p : ptrs) mf_pool_free(p, 0);
     mf_pool_free(A->stage, 0);
+    for (cudaEvent_t e : A->spmv_ev)
+        if (e) cudaEventDestroy(e);
     mf_pool_settle(A->dev);
     delete A;
 }

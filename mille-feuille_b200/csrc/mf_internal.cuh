@@ -81,6 +81,9 @@ struct mf_matrix_s {
     int *d_seg_kp;             // [nseg]
     uint16_t *d_seg_rowlen;    // [nseg*16]
     long long slice_entries;
+    int one_chunk;             // every tile-row is one slice of one chunk (slice number = tile-row)
+    int max_row;               // longest row of a slice
+    cudaEvent_t spmv_ev[2];    // timing events of mf_spmv (made on first use)
     unsigned char *d_meta;
     double *d_v64;
     float *d_v32;
@@ -196,6 +199,10 @@ int mf_ref_labels_run(const double *d_pold, const double *d_pnew, int nseg, int 
                       cudaStream_t s);
 void mf_solver_free_ws(mf_matrix_s *A);
 int mf_ws_get(mf_matrix_s *A, int blocks_per_sm, void **out, cudaStream_t s);
+// solve_rows.cu: the solve kernel of a one-chunk matrix (mode: FP64 / mixed; its
+// longest row), and that file's bounds-check report
+const void *mf_solve_rows_kernel(int mode, int method, int max_row);
+int mf_rows_chk_take();
 
 // ------------------------------------------------------- device utilities
 #ifdef __CUDACC__

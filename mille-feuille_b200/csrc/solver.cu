@@ -1,6 +1,8 @@
-// solver.cu -- host side of the single solves and the standalone products.
+// solver.cu -- host side of the single solves and the standalone products; the
+// kernels of matrices without a one-chunk form (solver_dev.cuh).
 #include "solver_dev.cuh"
 
+#include <atomic>
 #include <chrono>
 #include <mutex>
 #include <vector>
@@ -8,28 +10,30 @@
 namespace {
 
 // ------------------------------------------------------------ standalone SpMV
-// y = A x, one half-warp per tile-row range (same pipeline as the solver).
-template <int MODE, int LB>
+// y = A x, one half-warp per tile-row range (same pipeline as the solver), or
+// tile-rows in turn when every tile-row is one chunk.
+template <int MODE, int LB, int LEN>
 __global__ void __launch_bounds__(kThreads, LB) k_spmv(SolverParams P, int force_pr, double *y, int rows_per_hw)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, half = lane >> 4, i = lane & 15;
     const unsigned hmask = 0xFFFFu << (16 * half);
-    const int hw = (blockIdx.x * kWarps + wib) * 2 + half;
-    const int rb = min(P.tilem, hw * rows_per_hw), re = min(P.tilem, rb + rows_per_hw);
-    if (rb >= re) return;
     XVec X = make_x(P.x, P.p32, nullptr, nullptr, nullptr, nullptr, 0.f);
     X.force_pr = force_pr;
     const int n = P.n;
-    spmv_range<MODE, MODE == MODE_FP64>(P, P.seg_ptr[rb], P.seg_ptr[re], i, hmask, X, nullptr,
-                                        [&](int R, double v) {
+    auto store = [&](int R, double v) {
         const int row = R * MF_BS + i;
         if (row < n) y[row] = v;
-    });
-    for (int R = rb; R < re; R++) {          // tile-rows without tiles: y = 0
-        if (P.seg_ptr[R] != P.seg_ptr[R + 1]) continue;
-        const int row = R * MF_BS + i;
-        if (row < n) y[row] = 0.0;
+    };
+    int rb = 0, re = 0;
+    if (LEN == 0) {
+        const int hw = (blockIdx.x * kWarps + wib) * 2 + half;
+        rb = min(P.tilem, hw * rows_per_hw);
+        re = min(P.tilem, rb + rows_per_hw);
+        if (rb >= re) return;
     }
+    spmv_range<MODE, MODE == MODE_FP64, LEN>(P, P.seg_ptr[rb], P.seg_ptr[re], i, hmask, X, nullptr, store);
+    for (int R = rb; R < re; R++)            // tile-rows without tiles: y = 0
+        if (P.seg_ptr[R] == P.seg_ptr[R + 1]) store(R, 0.0);
 }
 
 __global__ void k_ref_labels(const double *pold, const double *pnew, int nseg, int *vis)
@@ -47,13 +51,13 @@ template <int METH>
 const void *solve_kernel_m(int mode, int lb)
 {
     if (lb == 2) {
-        if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 2, METH>;
-        if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 2, METH>;
-        return (const void *)k_solve<MODE_PARITY, 2, METH>;
+        if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 2, METH, 0>;
+        if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 2, METH, 0>;
+        return (const void *)k_solve<MODE_PARITY, 2, METH, 0>;
     }
-    if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 1, METH>;
-    if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 1, METH>;
-    return (const void *)k_solve<MODE_PARITY, 1, METH>;
+    if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 1, METH, 0>;
+    if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 1, METH, 0>;
+    return (const void *)k_solve<MODE_PARITY, 1, METH, 0>;
 }
 
 const void *solve_kernel(int mode, int lb, int method)
@@ -66,6 +70,13 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
 {
     // blocks_per_sm: 0 = default variant, 1 or 2 = that register-budget variant
     const int lb = (blocks_per_sm == 2) ? 2 : (blocks_per_sm == 1) ? 1 : kDefaultLB;
+    // the workspace of an earlier call with the same variant (its grid depends on
+    // the handle and the device alone)
+    Workspace *w = (Workspace *)A->ws;
+    if (w && w->lb == lb) {
+        *out = w;
+        return MF_SUCCESS;
+    }
     int dev = 0;
     MF_CUDA_TRY(cudaGetDevice(&dev));
     int nsm = 0;
@@ -88,11 +99,6 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
     // small systems: no more blocks than needed for one tile-row per half-warp
     const int need = (A->tilem + kWarps * 2 - 1) / (kWarps * 2);
     if (need < G) G = need > 0 ? need : 1;
-    Workspace *w = (Workspace *)A->ws;
-    if (w && w->G == G && w->lb == lb) {
-        *out = w;
-        return MF_SUCCESS;
-    }
     if (w) {
         MF_CUDA_TRY(cudaDeviceSynchronize());
         mf_solver_free_ws(A);
@@ -128,9 +134,18 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
     MF_TRY(mf_pool_array(&w->mag_p, S, s)); MF_TRY(mf_pool_array(&w->mag_s, S, s));
     MF_TRY(mf_pool_array(&w->lab_p, S, s)); MF_TRY(mf_pool_array(&w->lab_s, S, s));
     MF_TRY(mf_pool_array(&w->red, (long long)kRedKinds * G * kRedWidth, s));
-    MF_TRY(mf_pool_array(&w->bar, 1, s)); MF_TRY(mf_pool_array(&w->err, 1, s)); MF_TRY(mf_pool_array(&w->out, 16, s));
-    MF_TRY(mf_pool_array(&w->counts, 16, s));
-    MF_TRY(mf_pool_array(&w->phase_ns, 8, s));
+    MF_TRY(mf_pool_array(&w->ctl, (long long)kCtlBytes, s));
+    {
+        Readback *rb = (Readback *)(w->ctl + 128);
+        w->bar = (unsigned int *)w->ctl;
+        w->err = &rb->err;
+        w->out = rb->out;
+        w->counts = rb->counts;
+        w->phase_ns = rb->phase_ns;
+    }
+    // column segments past the tile-rows keep magnitude 0 (a matrix with more columns than rows)
+    MF_CUDA_TRY(cudaMemsetAsync(w->mag_p, 0, (size_t)S * sizeof(float), s));
+    MF_CUDA_TRY(cudaMemsetAsync(w->mag_s, 0, (size_t)S * sizeof(float), s));
     MF_TRY(exact_tiles(A, w->counts, s));    // counts: scratch before the first solve zeroes it
     w->nhw = G * kWarps * 2;
     MF_TRY(mf_pool_array(&w->hw_begin, w->nhw + 1, s));
@@ -238,8 +253,7 @@ void mf_solver_free_ws(mf_matrix_s *A)
 {
     Workspace *w = (Workspace *)A->ws;
     if (!w) return;
-    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->bar, w->err, w->out, w->counts,
-                    w->phase_ns, w->hw_begin, w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
+    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
     for (void *p : ptrs) mf_pool_free(p, 0);
     for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
     delete[] w->m_ev;
@@ -265,31 +279,19 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     MF_TRY(ws_get(A, opt->blocks_per_sm, &w, s));
     const long long L = A->vec_len;
     const long long S = std::max(A->tilem, A->tilen) + 1;
-    // zero the padded tails and the state the kernel reads before writing
-    MF_CUDA_TRY(cudaMemsetAsync(w->x, 0, L * sizeof(double), s));
+    // The kernel writes every entry below n_rows before it reads it, and the tails
+    // stay zero from the workspace's creation; parity mode's shadows and labels
+    // start from zero each time.  (Seven fills of whole vectors, and one per result
+    // array, went before each solve: 60 us of launches, and five read-backs after.)
     if (opt->x0_given)
         MF_CUDA_TRY(cudaMemcpyAsync(w->x, d_x, (size_t)A->n_rows * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->p, 0, L * sizeof(double), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->q, 0, L * sizeof(double), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->s, 0, L * sizeof(double), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->t, 0, L * sizeof(double), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->p32, 0, L * sizeof(float), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->s32, 0, L * sizeof(float), s));
     if (mode == MODE_PARITY) {
-        MF_CUDA_TRY(cudaMemsetAsync(w->p16, 0, L * sizeof(__half), s));
-        MF_CUDA_TRY(cudaMemsetAsync(w->s16, 0, L * sizeof(__half), s));
-        MF_CUDA_TRY(cudaMemsetAsync(w->p8, 0, L, s));
-        MF_CUDA_TRY(cudaMemsetAsync(w->s8, 0, L, s));
+        MF_CUDA_TRY(cudaMemsetAsync(w->s, 0, L * sizeof(double), s));
+        MF_CUDA_TRY(cudaMemsetAsync(w->p32, 0, w->all_bytes - 7 * w->vec_bytes, s));   // p32 .. s8
+        MF_CUDA_TRY(cudaMemsetAsync(w->lab_p, 0, S, s));
+        MF_CUDA_TRY(cudaMemsetAsync(w->lab_s, 0, S, s));
     }
-    MF_CUDA_TRY(cudaMemsetAsync(w->mag_p, 0, S * sizeof(float), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->mag_s, 0, S * sizeof(float), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->lab_p, 0, S, s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->lab_s, 0, S, s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->bar, 0, sizeof(unsigned int), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->err, 0, sizeof(int), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->out, 0, 16 * sizeof(double), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->counts, 0, 16 * sizeof(unsigned long long), s));
-    MF_CUDA_TRY(cudaMemsetAsync(w->phase_ns, 0, 8 * sizeof(unsigned long long), s));
+    MF_CUDA_TRY(cudaMemsetAsync(w->ctl, 0, kCtlBytes, s));
     SolverParams P;
     fill_params(P, A, w);
     P.b = d_b;
@@ -335,24 +337,28 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     }
     const auto t_prepared = std::chrono::steady_clock::now();
     MF_CUDA_TRY(cudaEventRecord(w->e0, s));
-    cudaError_t lerr = cudaLaunchCooperativeKernel(solve_kernel(mode, w->lb, opt->method), dim3(w->G), dim3(kThreads), args, 0, s);
+    // One-chunk matrices (the 5- and 7-point stencils) have kernels of their own
+    // in the default two-blocks-per-SM budget; everything else, parity mode and
+    // the one-block variant take the general walks.
+    const bool rows = A->one_chunk && mode != MODE_PARITY && w->lb == 2;
+    const void *kfn = rows ? mf_solve_rows_kernel(mode, opt->method, A->max_row)
+                           : solve_kernel(mode, w->lb, opt->method);
+    cudaError_t lerr = cudaLaunchCooperativeKernel(kfn, dim3(w->G), dim3(kThreads), args, 0, s);
     if (lerr != cudaSuccess) {
         win.reset(s);
         MF_CUDA_TRY(lerr);
     }
     MF_CUDA_TRY(cudaEventRecord(w->e1, s));
-    double out[16];
-    unsigned long long counts[16];
-    int err = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(out, w->out, sizeof(out), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaMemcpyAsync(counts, w->counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaMemcpyAsync(&err, w->err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    unsigned long long phase[8];
-    MF_CUDA_TRY(cudaMemcpyAsync(phase, w->phase_ns, sizeof(phase), cudaMemcpyDeviceToHost, s));
     MF_CUDA_TRY(cudaMemcpyAsync(d_x, w->x, (size_t)A->n_rows * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    Readback rb;
+    MF_CUDA_TRY(cudaMemcpyAsync(&rb, w->ctl + 128, sizeof(rb), cudaMemcpyDeviceToHost, s));
     MF_CUDA_TRY(cudaStreamSynchronize(s));
     win.reset(s);
-    const int chk = chk_take();
+    const double *out = rb.out;
+    const unsigned long long *counts = rb.counts, *phase = rb.phase_ns;
+    int err = rb.err;
+    int chk = chk_take();
+    if (!chk) chk = mf_rows_chk_take();
     if (chk) err = chk;
     const auto t_done = std::chrono::steady_clock::now();
     float ms = 0.f;
@@ -386,44 +392,109 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     return (int)out[6];
 }
 
-// y = A x with every tile in one entry precision (MF_P64 .. MF_P8).
-int mf_spmv_tiles_run(mf_matrix_s *A, const double *d_x, double *d_y, int tile_prec, cudaStream_t s,
-                      double *elapsed_ms)
+namespace {
+
+using SpmvFn = void (*)(SolverParams, int, double *, int);
+
+template <int LEN>
+SpmvFn spmv_kernel_len(bool f64)
 {
-    if (tile_prec < MF_P64 || tile_prec > MF_P8) return MF_ERR_INVALID;
-    // x is read through a padded copy so that column tiles past n_rows read zeros
-    Workspace *w = nullptr;
-    MF_TRY(ws_get(A, 0, &w, s));
-    const long long L = A->vec_len;
-    MF_CUDA_TRY(cudaMemsetAsync(w->x, 0, L * sizeof(double), s));
-    MF_CUDA_TRY(cudaMemcpyAsync(w->x, d_x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    return f64 ? (SpmvFn)k_spmv<MODE_FP64, 2, LEN> : (SpmvFn)k_spmv<MODE_MIXED, 2, LEN>;
+}
+
+// k_spmv for a matrix and stored precision: one-chunk matrices by their longest
+// row (INT8 products need the per-tile scales of the general walk).
+SpmvFn spmv_kernel(const mf_matrix_s *A, int tile_prec, int *variant)
+{
+    const bool f64 = tile_prec == MF_P64;
+    const int len = (!A->one_chunk || tile_prec == MF_P8) ? 0 : A->max_row <= 5 ? 5 : A->max_row <= 7 ? 7 : 8;
+    *variant = (len == 0 ? 0 : len == 5 ? 1 : len == 7 ? 2 : 3) * 2 + (f64 ? 1 : 0);
+    return len == 0 ? spmv_kernel_len<0>(f64) : len == 5 ? spmv_kernel_len<5>(f64)
+           : len == 7 ? spmv_kernel_len<7>(f64) : spmv_kernel_len<8>(f64);
+}
+
+// Blocks per SM of a k_spmv variant on a device (a property of the device and
+// the kernel, asked for once).
+int spmv_resident(int dev, SpmvFn fn, int variant, int *occ)
+{
+    constexpr int kDevs = 64;
+    static std::atomic<int> known[8][kDevs];
+    int o = (dev >= 0 && dev < kDevs) ? known[variant][dev].load(std::memory_order_relaxed) : 0;
+    if (o == 0) {
+        MF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, (const void *)fn, kThreads, 0));
+        if (o < 1) o = 1;
+        if (dev >= 0 && dev < kDevs) known[variant][dev].store(o, std::memory_order_relaxed);
+    }
+    *occ = o;
+    return MF_SUCCESS;
+}
+
+// One wave: resident blocks x SMs, each half-warp a contiguous range of
+// tile-rows (or every stride-th one, spmv_rows).
+int spmv_launch(mf_matrix_s *A, const double *x, double *y, int tile_prec, cudaStream_t s)
+{
     SolverParams P;
-    fill_params(P, A, w);
-    int nsm = 0, dev = 0;
+    fill_params(P, A, nullptr);
+    P.x = const_cast<double *>(x);
+    // gathers reach the columns that have entries, and column 0 of a slice's first tile (padding)
+    P.chk_xlen = A->n_cols;
+    int nsm = 0, dev = 0, occ = 1, variant = 0;
     MF_CUDA_TRY(cudaGetDevice(&dev));
     MF_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    // one wave: resident blocks x SMs, each half-warp a contiguous range of tile-rows
-    const bool f64 = tile_prec == MF_P64;
-    const void *kfn = f64 ? (const void *)k_spmv<MODE_FP64, 2> : (const void *)k_spmv<MODE_MIXED, 2>;
-    int occ = 1;
-    MF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kThreads, 0));
-    if (occ < 1) occ = 1;
+    SpmvFn fn = spmv_kernel(A, tile_prec, &variant);
+    MF_TRY(spmv_resident(dev, fn, variant, &occ));
     const int nhw_max = nsm * occ * kWarps * 2;
     int rows_per_hw = (A->tilem + nhw_max - 1) / nhw_max;
     if (rows_per_hw < 1) rows_per_hw = 1;
     const int nhw = (A->tilem + rows_per_hw - 1) / rows_per_hw;
     int blocks = (nhw + kWarps * 2 - 1) / (kWarps * 2);
     if (blocks < 1) blocks = 1;
-    MF_CUDA_TRY(cudaEventRecord(w->e0, s));
-    if (f64) k_spmv<MODE_FP64, 2><<<blocks, kThreads, 0, s>>>(P, MF_P64, d_y, rows_per_hw);
-    else k_spmv<MODE_MIXED, 2><<<blocks, kThreads, 0, s>>>(P, tile_prec, d_y, rows_per_hw);
+    fn<<<blocks, kThreads, 0, s>>>(P, tile_prec, y, rows_per_hw);
     MF_CUDA_TRY(cudaGetLastError());
-    MF_CUDA_TRY(cudaEventRecord(w->e1, s));
+    return MF_SUCCESS;
+}
+
+// Whether x's n_cols doubles and y's n_rows doubles share memory: the product
+// is then formed from a copy of x.
+bool spmv_overlap(const mf_matrix_s *A, const double *x, const double *y)
+{
+    const uintptr_t x0 = (uintptr_t)x, x1 = x0 + (size_t)A->n_cols * sizeof(double);
+    const uintptr_t y0 = (uintptr_t)y, y1 = y0 + (size_t)A->n_rows * sizeof(double);
+    return x0 < y1 && y0 < x1;
+}
+
+}  // namespace
+
+// y = A x with every tile in one entry precision (MF_P64 .. MF_P8).  The kernel
+// reads the caller's x in place: it gathers no column past n_cols, so the padded
+// copy made before (33 MB moved and a 16.8 MB fill for 128^3: 20 of 75 us) is
+// needed only when y overlaps x.
+int mf_spmv_tiles_run(mf_matrix_s *A, const double *d_x, double *d_y, int tile_prec, cudaStream_t s,
+                      double *elapsed_ms)
+{
+    if (tile_prec < MF_P64 || tile_prec > MF_P8) return MF_ERR_INVALID;
+    for (cudaEvent_t &e : A->spmv_ev)
+        if (!e) MF_CUDA_TRY(cudaEventCreate(&e));
+    double *copy = nullptr;
+    if (spmv_overlap(A, d_x, d_y)) {
+        MF_TRY(mf_pool_array(&copy, A->n_cols, s));
+        const cudaError_t e =
+            cudaMemcpyAsync(copy, d_x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) mf_pool_free(copy, s);
+        MF_CUDA_TRY(e);
+        d_x = copy;
+    }
+    cudaError_t e0 = cudaEventRecord(A->spmv_ev[0], s);
+    const int rc = e0 == cudaSuccess ? spmv_launch(A, d_x, d_y, tile_prec, s) : MF_SUCCESS;
+    if (e0 == cudaSuccess) e0 = cudaEventRecord(A->spmv_ev[1], s);
+    mf_pool_free(copy, s);
+    MF_TRY(rc);
+    MF_CUDA_TRY(e0);
     MF_CUDA_TRY(cudaStreamSynchronize(s));
     MF_TRY(chk_take());
     if (elapsed_ms) {
         float ms = 0.f;
-        MF_CUDA_TRY(cudaEventElapsedTime(&ms, w->e0, w->e1));
+        MF_CUDA_TRY(cudaEventElapsedTime(&ms, A->spmv_ev[0], A->spmv_ev[1]));
         *elapsed_ms = ms;
     }
     return MF_SUCCESS;
@@ -660,29 +731,11 @@ int mf_spmv_noalloc_run(mf_matrix_s *A, const double *d_x, double *d_y, int prec
     if (dev != A->dev) return MF_ERR_INVALID;
     double *x = nullptr;
     MF_TRY(noalloc_scratch(dev, &x));
-    // x, then zeros up to the padded length: every entry the kernel reads is written here
-    MF_CUDA_TRY(cudaMemcpyAsync(x, d_x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (L > A->n_cols)
-        MF_CUDA_TRY(cudaMemsetAsync(x + A->n_cols, 0, (size_t)(L - A->n_cols) * sizeof(double), s));
-    const int fpr = precision == MF_PREC_FP64 ? MF_P64 : MF_P32;
-    SolverParams P;
-    fill_params(P, A, nullptr);
-    P.x = x;
-    int nsm = 0;
-    MF_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const void *kfn = fpr == MF_P64 ? (const void *)k_spmv<MODE_FP64, 2> : (const void *)k_spmv<MODE_MIXED, 2>;
-    int occ = 1;
-    MF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kThreads, 0));
-    if (occ < 1) occ = 1;
-    const int nhw_max = nsm * occ * kWarps * 2;
-    int rows_per_hw = (A->tilem + nhw_max - 1) / nhw_max;
-    if (rows_per_hw < 1) rows_per_hw = 1;
-    const int nhw = (A->tilem + rows_per_hw - 1) / rows_per_hw;
-    int blocks = (nhw + kWarps * 2 - 1) / (kWarps * 2);
-    if (blocks < 1) blocks = 1;
-    if (fpr == MF_P64) k_spmv<MODE_FP64, 2><<<blocks, kThreads, 0, s>>>(P, MF_P64, d_y, rows_per_hw);
-    else k_spmv<MODE_MIXED, 2><<<blocks, kThreads, 0, s>>>(P, MF_P32, d_y, rows_per_hw);
-    MF_CUDA_TRY(cudaGetLastError());
-    return MF_SUCCESS;
+    // the scratch is needed only when y overlaps x
+    if (spmv_overlap(A, d_x, d_y)) {
+        MF_CUDA_TRY(cudaMemcpyAsync(x, d_x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        d_x = x;
+    }
+    return spmv_launch(A, d_x, d_y, precision == MF_PREC_FP64 ? MF_P64 : MF_P32, s);
 }
 

@@ -1,6 +1,6 @@
 // solver_dev.cuh -- the persistent single-kernel CG / BiCGSTAB, the tile walks and
-// the per-handle workspace, shared by solver.cu and multi.cu (each instantiates
-// its own kernels; everything here has internal linkage).
+// the per-handle workspace, shared by solver.cu, solve_rows.cu and multi.cu (each
+// instantiates its own kernels; everything here has internal linkage).
 //
 // One cooperative launch runs the whole solve (the reference's single-kernel
 // design, Mille-feuille-cg.h:1113-1348 / main-cg-mixed.cu:1016-1385 /
@@ -121,6 +121,7 @@ struct SolverParams {
     // through the test_check_limit hook)
     int nseg, ntiles, chk_xlen;
     long long n_payload;
+    long long nnz;
 };
 
 struct Shared {
@@ -128,6 +129,7 @@ struct Shared {
     double bcast[kRedWidth];
     int flag;
     unsigned cnt[kWarps * 2][10];   // per-half-warp tile / entry counters per precision (mixed / parity)
+    unsigned whole[4];              // block 0: products of the whole matrix in one precision (spmv_rows)
     unsigned long long clk_t, clk_acc[5];   // block 0 phase clock
 };
 
@@ -515,10 +517,13 @@ template <> struct LeanChunk<MF_P64> {
         for (int q = 0; q < 4; q++) d[q] = make_double2(0.0, 0.0);
         m = 0ull;
     }
+    // LEN: entries of the longest row; groups past it hold padding only
+    template <int LEN = 8>
     __device__ __forceinline__ void load(const SolverParams &P, long long cb, int i)
     {
 #pragma unroll
-        for (int q = 0; q < 4; q++) d[q] = __ldcs((const double2 *)(P.v64 + cb + 32 * q) + i);
+        for (int q = 0; q < 4; q++)
+            if (2 * q < LEN) d[q] = __ldcs((const double2 *)(P.v64 + cb + 32 * q) + i);
         m = __ldcs((const unsigned long long *)(P.meta + cb) + i);
     }
     __device__ __forceinline__ void values(double (&v)[8]) const
@@ -539,10 +544,11 @@ template <> struct LeanChunk<MF_P32> {
         a = b = make_float4(0.f, 0.f, 0.f, 0.f);
         m = 0ull;
     }
+    template <int LEN = 8>
     __device__ __forceinline__ void load(const SolverParams &P, long long cb, int i)
     {
         a = __ldcs((const float4 *)(P.v32 + cb) + i);
-        b = __ldcs((const float4 *)(P.v32 + cb + 64) + i);
+        if (LEN > 4) b = __ldcs((const float4 *)(P.v32 + cb + 64) + i);
         m = __ldcs((const unsigned long long *)(P.meta + cb) + i);
     }
     __device__ __forceinline__ void values(double (&v)[8]) const
@@ -560,6 +566,7 @@ template <> struct LeanChunk<MF_P16> {
         u = make_uint4(0u, 0u, 0u, 0u);
         m = 0ull;
     }
+    template <int LEN = 8>
     __device__ __forceinline__ void load(const SolverParams &P, long long cb, int i)
     {
         u = __ldcs((const uint4 *)(P.v16 + cb) + i);
@@ -654,6 +661,106 @@ __device__ __forceinline__ void spmv_range_lean(const SolverParams &P, int sb, i
     }
 }
 
+// The walk of a matrix whose every tile-row is one slice of one chunk (rows of
+// up to 8 entries in up to 15 tiles: the 5- and 7-point stencils): tile-row R's
+// payload starts at entry 128 R and its tile words at 16 R, so there are no
+// headers, no slice or chunk counters and nothing to wait for but the chunk.
+//
+// LEN: no row is longer (5, 7 or 8, a template argument).  Entries past it are
+// padding in every row: they are neither loaded (FP64: three of four 16-byte
+// groups with 5), nor gathered, nor multiplied.  A run-time length instead put a
+// branch between the gathers and cost more than it saved (whole 128^3 FP32
+// iterations: 29.4 us with all 8 entries, 34.9 with `j < len`).
+//
+// A block's half-warps take the block's tile-rows in turn (first, first + stride,
+// ... < end): a warp's halves gather from neighbouring rows, and a block sweeps
+// matrix and vectors as one stream instead of 32.  Turns over the whole launch
+// cost 5 % on 128^3: then the update phase touches a row from another SM than
+// the product did.
+//
+// These products move what L2 and DRAM can deliver (128^3 FP32: 11 TB/s through
+// L2 inside a solve; 2048^2 FP64: 6.1 TB/s of DRAM), so bytes and requests count:
+// a TMA ring with mbarriers, asynchronous copies of the epilogue's operands,
+// gathers one step ahead and 3 or 4 blocks per SM were all measured, and none was
+// faster than this walk with the next chunk in registers.
+template <int PR, int LEN, typename Epi>
+__device__ __forceinline__ void spmv_rows(const SolverParams &P, int R, int end, int stride, int i, unsigned hmask,
+                                          const double *x64, Epi &epi)
+{
+    if (R >= end) return;
+    if (!chk_in(CHK_PAYLOAD, (long long)end * 128 - 1, P.n_payload)) return;
+    int tw = load_tw(P, R, i);
+    LeanChunk<PR> cur;
+    cur.zero();
+    cur.template load<LEN>(P, (long long)R * 128, i);
+    for (;;) {
+        const int xb = (tw >> 8) * MF_BS;
+        double xv[LEN];
+#pragma unroll
+        for (int j = 0; j < LEN; j++) {
+            const unsigned mm = (unsigned)(cur.m >> (8 * j)) & 0xFFu;
+            const int xi = __shfl_sync(hmask, xb, (int)(mm >> 4), 16) + (int)(mm & 15u);
+            xv[j] = chk_in(CHK_X, xi, P.chk_xlen) ? x64[xi] : 0.0;
+        }
+        const int Rn = R + stride;
+        LeanChunk<PR> nxt;
+        nxt.zero();
+        if (Rn < end) {
+            nxt.template load<LEN>(P, (long long)Rn * 128, i);
+            tw = load_tw(P, Rn, i);
+        }
+        double v[8];
+        cur.values(v);
+        double acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < LEN; j++) acc = fma(v[j], xv[j], acc);
+        epi(R, acc);
+        if (Rn >= end) return;
+        R = Rn;
+        cur = nxt;
+    }
+}
+
+// The same walk with the precision chosen per slice (or forced to scaled INT8),
+// as slice_dot does.
+template <int LEN, typename Epi>
+__device__ __forceinline__ void spmv_rows_dyn(const SolverParams &P, int R, int end, int stride, int i,
+                                              unsigned hmask, const XVec &X, unsigned *cnt, Epi &epi)
+{
+    if (R < end && !chk_in(CHK_PAYLOAD, (long long)end * 128 - 1, P.n_payload)) return;
+    for (; R < end; R += stride) {
+        const int4 h = P.seg_hdr[R];
+        const int nt = hdr_nt(h);
+        const int tw = load_tw(P, R, i);
+        const float st = load_stat<MODE_MIXED, false>(X, tw, i, nt);
+        const int pr = __reduce_min_sync(hmask, i < nt ? tile_prec<MODE_MIXED, false>(P, tw, st, X) : MF_P8);
+        if (cnt && i == 0 && chk_in(CHK_TILE, (long long)h.x + nt, (long long)P.ntiles + 1)) {
+            cnt[pr] += (unsigned)nt;
+            cnt[5 + pr] += (unsigned)(P.tile_off[h.x + nt] - P.tile_off[h.x]);
+        }
+        double v64[8];
+        float v[8];
+        const long long cb = (long long)R * 128;
+        if (pr == MF_P32) load_chunk<MF_P32>(P, cb, i, LEN, v64, v);
+        else if (pr == MF_P16) load_chunk<MF_P16>(P, cb, i, LEN, v64, v);
+        else load_chunk<MF_P8>(P, cb, i, LEN, v64, v);
+        const float sc =
+            (pr == MF_P8 && i < nt && chk_in(CHK_TILE, h.x + i, P.ntiles)) ? P.i8_scale[h.x + i] : 1.0f;
+        const unsigned long long m8 = __ldcs((const unsigned long long *)(P.meta + cb) + i);
+        double acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < LEN; j++) {
+            const unsigned mm = (unsigned)(m8 >> (8 * j)) & 0xFFu;
+            const int slot = (int)(mm >> 4);
+            const int xi = __shfl_sync(hmask, (tw >> 8) * MF_BS, slot, 16) + (int)(mm & 15u);
+            const float s8 = __shfl_sync(hmask, sc, slot, 16);     // 1 unless the slice runs INT8
+            const double xv = chk_in(CHK_X, xi, P.chk_xlen) ? X.x64[xi] : 0.0;
+            acc = fma((double)(v[j] * s8), xv, acc);
+        }
+        epi(R, acc);
+    }
+}
+
 // y = A x over the half-warp's slices [sb, se); epi(R, y) is called once per
 // tile-row (after its last slice) with the row sum of lane i.
 // F64: every tile in FP64 (the FP64 residual replacement and the FP64 SpMV).
@@ -665,10 +772,30 @@ __device__ __forceinline__ void spmv_range_lean(const SolverParams &P, int sb, i
 // together with that slice's own loads; the precision statistic (mixed /
 // parity) is loaded one slice ahead once the tile word is in.  A slice then
 // waits for two round trips: values + index word, then the gathered x.
-template <int MODE, bool F64, typename Epi>
+// LEN > 0: a one-chunk matrix with rows of up to LEN entries (spmv_rows; the
+// range is then the block's own tile-rows in a solve, all of them in turn in the
+// standalone product, and sb, se are not used).
+template <int MODE, bool F64, int LEN, typename Epi>
 __device__ __forceinline__ void spmv_range(const SolverParams &P, int sb, int se, int i, unsigned hmask,
-                                           const XVec &X, unsigned *cnt, Epi epi)
+                                           const XVec &X, unsigned *cnt, Epi epi, unsigned *whole = nullptr)
 {
+    if constexpr (LEN > 0) {
+        const int h = (int)(threadIdx.x >> 4);
+        const int *hb = P.hw_begin ? P.hw_begin + blockIdx.x * kWarps * 2 : nullptr;
+        const int R = hb ? hb[0] + h : (int)blockIdx.x * kWarps * 2 + h;
+        const int end = hb ? hb[kWarps * 2] : P.tilem;
+        const int stride = hb ? kWarps * 2 : (int)gridDim.x * kWarps * 2;
+        if constexpr (MODE == MODE_FP64 || F64) {
+            spmv_rows<MF_P64, LEN>(P, R, end, stride, i, hmask, X.x64, epi);
+        } else {
+            const int pr = (X.force_pr < 0 && !X.dyn) ? X.lean_pr : X.force_pr;
+            if (pr == MF_P32) spmv_rows<MF_P32, LEN>(P, R, end, stride, i, hmask, X.x64, epi);
+            else if (pr == MF_P16) spmv_rows<MF_P16, LEN>(P, R, end, stride, i, hmask, X.x64, epi);
+            else spmv_rows_dyn<LEN>(P, R, end, stride, i, hmask, X, cnt, epi);
+            if (whole && (pr == MF_P32 || pr == MF_P16) && blockIdx.x == 0 && threadIdx.x == 0) whole[pr]++;
+        }
+        return;
+    }
     if (sb >= se) return;
     if (!chk_in(CHK_SLICE, sb, P.nseg) || !chk_in(CHK_SLICE, se - 1, P.nseg)) return;
     // the FP64 mode takes the pipelined walk too (128^3 FP64 CG 62.0 -> 60.3 ms);
@@ -914,7 +1041,9 @@ __device__ __forceinline__ int relaxed_precision(const SolverParams &P, double r
 // each gets its own register allocation: the kernel sits at the 64-register
 // limit of two 512-thread blocks per SM, and code in one method's branch
 // moves spills into the other's hot loop.
-template <int MODE, int LB, int METH>
+// LEN > 0: for one-chunk matrices with rows of up to LEN entries (spmv_rows); these
+// instantiations hold none of the general walks.
+template <int MODE, int LB, int METH, int LEN>
 __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
 {
     __shared__ Shared sh;
@@ -924,6 +1053,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     // the host derives the totals from the SpMV count)
     unsigned *cnt = (MODE == MODE_FP64) ? nullptr : sh.cnt[c.wib * 2 + c.half];
     if (cnt && c.i < 10) cnt[c.i] = 0u;
+    if (threadIdx.x < 4) sh.whole[threadIdx.x] = 0u;
     int nspmv = 0;
     __syncwarp();
     PhaseClock clk;
@@ -955,13 +1085,14 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                 P.r[row] = rv;
                 P.p[row] = rv;
                 if (bicg) P.rh[row] = rv;
+                else P.q[row] = 0.0;               // the first q = w + 0 q
             }
             publish_dir<MODE>(R, row, valid, rv, 0.0, P.p32, P.p16, P.p8, P.mag_p, P.lab_p, bmax, c.hmask, false,
                               &bmin);
             pb += rv * rv;
         };
-        spmv_range<MODE, true>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, init_row);
-        for (int R = c.rbeg; R < c.rend; R++)
+        spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, init_row);
+        for (int R = c.rbeg; LEN == 0 && R < c.rend; R++)
             if (P.seg_ptr[R] == P.seg_ptr[R + 1]) init_row(R, 0.0);
         nspmv++;
     } else {
@@ -974,6 +1105,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                 P.r[row] = bv;
                 P.p[row] = bv;
                 if (bicg) P.rh[row] = bv;
+                else P.q[row] = 0.0;               // the first q = w + 0 q
             }
             // parity mode: labels start all FP64 (cudaMemset(d_vis, 0), main-cg-mixed.cu:2828)
             publish_dir<MODE>(R, row, valid, bv, 0.0, P.p32, P.p16, P.p8, P.mag_p, P.lab_p, bmax, c.hmask, false,
@@ -1044,7 +1176,8 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
 
     // tile-rows without slices (all-zero rows) get no SpMV epilogue
     bool has_empty = false;
-    for (int R = c.rbeg; R < c.rend && !has_empty; R++) has_empty = P.seg_ptr[R] == P.seg_ptr[R + 1];
+    if (LEN == 0)
+        for (int R = c.rbeg; R < c.rend && !has_empty; R++) has_empty = P.seg_ptr[R] == P.seg_ptr[R + 1];
     double beta2 = 0.0;
     // mixed CG: uniform reduced precision of the next SpMV (relaxed_precision)
     int prA = (MODE == MODE_MIXED) ? relaxed_precision(P, rr, bb) : MF_P32;
@@ -1062,7 +1195,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             XVec XA = make_x(P.r, nullptr, nullptr, nullptr, P.mag_r, nullptr, invM, dynA);
             if (MODE == MODE_MIXED && prA != MF_P32) XA.force_pr = prA;
             if (P.lean_f16) XA.lean_pr = MF_P16;
-            spmv_range<MODE, false>(P, c.sbeg, c.send, c.i, c.hmask, XA, cnt, [&](int R, double y) {
+            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask, XA, cnt, [&](int R, double y) {
                 const int row = R * MF_BS + c.i;
                 if (row < n) {
                     const double pn = P.r[row] + beta2 * P.p[row];
@@ -1071,9 +1204,9 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                     P.q[row] = qn;
                     ppq += pn * qn;
                 }
-            });
+            }, sh.whole);
             if (has_empty) {
-                for (int R = c.rbeg; R < c.rend; R++) {
+                for (int R = c.rbeg; LEN == 0 && R < c.rend; R++) {
                     if (P.seg_ptr[R] != P.seg_ptr[R + 1]) continue;
                     const int row = R * MF_BS + c.i;
                     if (row < n) {
@@ -1155,7 +1288,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                 rmax = 0.0f;
                 rmin = 3.0e38f;
                 rsm = 0.0f;
-                spmv_range<MODE, true>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr,
+                spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr,
                                        [&](int R, double y) {
                                            const int row = R * MF_BS + c.i;
                                            const bool valid = row < n;
@@ -1170,7 +1303,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                                                              rthr, &rsm);
                                        });
                 if (has_empty) {
-                    for (int R = c.rbeg; R < c.rend; R++) {
+                    for (int R = c.rbeg; LEN == 0 && R < c.rend; R++) {
                         if (P.seg_ptr[R] != P.seg_ptr[R + 1]) continue;
                         const int row = R * MF_BS + c.i;
                         const bool valid = row < n;
@@ -1209,7 +1342,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
         if (!bicg) {
             // ---- A: q = A p, p.q ----
             double ppq = 0.0;
-            spmv_range<MODE, false>(P, c.sbeg, c.send, c.i, c.hmask,
+            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask,
                              make_x(P.p, P.p32, P.p16, P.p8, P.mag_p, P.lab_p, invM), cnt,
                              [&](int R, double y) {
                                  const int row = R * MF_BS + c.i;
@@ -1257,7 +1390,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             double prv = 0.0;
             const int useA = (kFb && coolA > 0) ? 0 : dynA;
             const unsigned d0A = demoted();
-            spmv_range<MODE, false>(P, c.sbeg, c.send, c.i, c.hmask,
+            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask,
                              lean_base(make_x(P.p, P.p32, P.p16, P.p8, P.mag_p, P.lab_p, invM, useA)), cnt,
                              [&](int R, double y) {
                                  const int row = R * MF_BS + c.i;
@@ -1265,7 +1398,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                                      P.q[row] = y;
                                      prv += P.rh[row] * y;
                                  }
-                             });
+                             }, sh.whole);
             nspmv++;
             clk.lap(PH_SPMV);
             block_partial(P, sh, 1, prv, (double)(demoted() - d0A), 0, 0, kNvFb, 0u);
@@ -1302,7 +1435,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             double pts = 0.0, ptt = 0.0;
             const int useS = (kFb && coolS > 0) ? 0 : dynS;
             const unsigned d0S = demoted();
-            spmv_range<MODE, false>(P, c.sbeg, c.send, c.i, c.hmask,
+            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask,
                              lean_base(make_x(P.s, P.s32, P.s16, P.s8, P.mag_s, P.lab_s, invMs, useS)), cnt,
                              [&](int R, double y) {
                                  const int row = R * MF_BS + c.i;
@@ -1311,7 +1444,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                                      pts += y * P.s[row];
                                      ptt += y * y;
                                  }
-                             });
+                             }, sh.whole);
             nspmv++;
             clk.lap(PH_SPMV);
             block_partial(P, sh, 3, pts, ptt, (double)(demoted() - d0S), 0, kNvFb + 1, 0u);
@@ -1360,7 +1493,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             }
             // ---- FP64 true residual: r = b - A x ----
             double prt = 0.0, prth = 0.0;
-            spmv_range<MODE, true>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
+            spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
                 const int row = R * MF_BS + c.i;
                 if (row < n) {
                     const double rv = P.b[row] - y;
@@ -1370,7 +1503,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                 }
             });
             // rows of tile-rows without tiles (A row = 0): r = b there
-            for (int R = c.rbeg; R < c.rend; R++) {
+            for (int R = c.rbeg; LEN == 0 && R < c.rend; R++) {
                 if (P.seg_ptr[R] != P.seg_ptr[R + 1]) continue;
                 const int row = R * MF_BS + c.i;
                 if (row < n) {
@@ -1449,14 +1582,14 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     // ---- final FP64 true residual when the last one was not already formed ----
     if (!last_true) {
         double prt = 0.0;
-        spmv_range<MODE, true>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
+        spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
             const int row = R * MF_BS + c.i;
             if (row < n) {
                 const double d = P.b[row] - y;
                 prt += d * d;
             }
         });
-        for (int R = c.rbeg; R < c.rend; R++) {
+        for (int R = c.rbeg; LEN == 0 && R < c.rend; R++) {
             if (P.seg_ptr[R] != P.seg_ptr[R + 1]) continue;
             const int row = R * MF_BS + c.i;
             if (row < n) prt += P.b[row] * P.b[row];
@@ -1470,6 +1603,13 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     // tile-use counters
     __syncwarp();
     if (cnt && c.i < 10 && cnt[c.i]) atomicAdd(&P.counts[c.i], (unsigned long long)cnt[c.i]);
+    if (cnt && blockIdx.x == 0 && threadIdx.x == 0) {
+        for (int pr = 0; pr < 4; pr++) {
+            if (!sh.whole[pr]) continue;
+            atomicAdd(&P.counts[pr], (unsigned long long)sh.whole[pr] * (unsigned long long)P.ntiles);
+            atomicAdd(&P.counts[5 + pr], (unsigned long long)sh.whole[pr] * (unsigned long long)P.nnz);
+        }
+    }
     if (clk.on() && P.phase_ns)
         for (int j = 0; j < 5; j++) P.phase_ns[j] = sh.clk_acc[j];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1485,6 +1625,15 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
 }
 
 // ------------------------------------------------------------ workspace
+// What a solve leaves for the host.
+struct Readback {
+    int err, pad[31];
+    double out[16];
+    unsigned long long counts[16];
+    unsigned long long phase_ns[8];
+};
+constexpr size_t kCtlBytes = 128 + sizeof(Readback);
+
 struct Workspace {
     int G;                 // grid blocks of the persistent kernel
     int lb;                // register-budget variant (blocks per SM it was built for)
@@ -1501,6 +1650,9 @@ struct Workspace {
     int8_t *p8, *s8;
     signed char *lab_p, *lab_s;
     double *red;
+    // one block zeroed before a solve and read back after it: the barrier counter
+    // (a 128-byte line of its own), then Readback
+    char *ctl;
     unsigned int *bar;
     int *err;
     double *out;
@@ -1595,6 +1747,7 @@ void fill_params(SolverParams &P, mf_matrix_s *A, Workspace *w)
     P.ntiles = A->tilenum;
     P.chk_xlen = A->vec_len;
     P.n_payload = A->slice_entries;
+    P.nnz = A->nnz;
     if (w) {
         P.hw_begin = w->hw_begin;
         P.x = w->x; P.r = w->r; P.p = w->p; P.q = w->q; P.rh = w->rh; P.s = w->s; P.t = w->t;

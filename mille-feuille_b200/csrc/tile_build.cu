@@ -423,8 +423,9 @@ __global__ void k_seg_shape(const int *__restrict__ tile_ptr, const int *__restr
                             const unsigned char *__restrict__ tptr, int tilem, int rowA,
                             int *__restrict__ seg_tile0, int *__restrict__ seg_kp,
                             uint16_t *__restrict__ seg_rowlen, int *__restrict__ seg_entries,
-                            long long *__restrict__ row_cost)
+                            long long *__restrict__ row_cost, int *__restrict__ shape)
 {
+    int longest = 0;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -456,9 +457,14 @@ __global__ void k_seg_shape(const int *__restrict__ tile_ptr, const int *__restr
                 seg_entries[s] = kp * MF_BS;
             }
             cost += kp + 6;
+            longest = max(longest, K);
         }
         if (lane == 0) row_cost[R] = cost;
+        // not one slice of one chunk (kp + 6 = 14 past the base cost of 4)
+        if (lane == 0 && cost != 18) shape[1] = 1;
     }
+    // shape[0]: the longest row; shape[1]: some tile-row is not one chunk
+    if (lane == 0 && longest > 0) atomicMax(&shape[0], longest);
 }
 
 __global__ void k_seg_fill(const int *__restrict__ tile_ptr, const int *__restrict__ seg_ptr,
@@ -752,11 +758,14 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     MF_TRY(tmp.get(&d_seg_entries, nseg + 1));
     MF_TRY(dalloc(&A->d_seg_off, nseg + 1, s));
     MF_TRY(tmp.get(&d_cost, tilem + 1));
+    int *d_shape = nullptr;
+    MF_TRY(tmp.get(&d_shape, 2));
+    MF_CUDA_TRY(cudaMemsetAsync(d_shape, 0, 2 * sizeof(int), s));
     MF_TRY(dalloc(&A->d_row_cost, tilem + 1, s));
     if (tilem > 0) {
         k_seg_shape<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_seg_ptr, A->d_csr_offset, A->d_csrptr_offset,
                                                A->d_tptr, tilem, rowA, A->d_seg_tile0, A->d_seg_kp,
-                                               A->d_seg_rowlen, d_seg_entries, d_cost);
+                                               A->d_seg_rowlen, d_seg_entries, d_cost, d_shape);
         MF_CUDA_TRY(cudaGetLastError());
     }
     MF_TRY(mf_scan_i32_to_i64(d_seg_entries, A->d_seg_off, nseg, s));
@@ -774,9 +783,13 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
         MF_CUDA_TRY(cudaGetLastError());
     }
     long long ent = 0;
+    int h_shape[2] = {0, 0};
     MF_CUDA_TRY(cudaMemcpyAsync(&ent, A->d_seg_off + nseg, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    MF_CUDA_TRY(cudaMemcpyAsync(h_shape, d_shape, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     MF_CUDA_TRY(cudaStreamSynchronize(s));
     A->slice_entries = ent;
+    A->max_row = h_shape[0];
+    A->one_chunk = tilem > 0 && h_shape[1] == 0 ? 1 : 0;
     if ((ent >> 7) >= (1LL << 31)) return MF_ERR_UNSUPPORTED;
     MF_TRY(dalloc(&A->d_meta, ent, s));
     MF_TRY(dalloc(&A->d_v64, ent, s));
