@@ -37,7 +37,8 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
            "-ccbin", "g++", "-I", INCLUDE]
-SOURCES = ["pool.cu", "scan.cu", "tile_build.cu", "solver.cu", "solve_rows.cu", "multi.cu", "api.cu", "adjoint.cu", "mmio.cpp"]
+SOURCES = ["pool.cu", "scan.cu", "tile_build.cu", "solver.cu", "solve_rows.cu", "solve_small.cu",
+           "multi.cu", "api.cu", "adjoint.cu", "mmio.cpp"]
 HEADERS = ["mf_internal.cuh", "solver_dev.cuh"]
 
 
@@ -84,7 +85,7 @@ def build(verbose: bool = False, check: bool = False) -> str:
     jobs.append(("api.cu", api_fp64, ("MF_CG_INC_FP64",)))
     swap = {}
     if check:
-        for src in ("solver.cu", "solve_rows.cu", "multi.cu", "api.cu"):
+        for src in ("solver.cu", "solve_rows.cu", "solve_small.cu", "multi.cu", "api.cu"):
             obj = os.path.join(BUILD, src.replace(".cu", "_check.cu.o"))
             swap[src + ".o"] = obj
             jobs.append((src, obj, ("MF_CHECK",)))

@@ -203,6 +203,11 @@ int mf_ws_get(mf_matrix_s *A, int blocks_per_sm, void **out, cudaStream_t s);
 // longest row), and that file's bounds-check report
 const void *mf_solve_rows_kernel(int mode, int method, int max_row);
 int mf_rows_chk_take();
+// solve_small.cu: the same for systems with no more tile-rows than half-warps, and for
+// one cluster (max_row 0: not a one-chunk matrix; rows_per_hw: tile-rows per half-warp)
+const void *mf_solve_resident_kernel(int mode, int lb, int max_row);
+const void *mf_solve_cluster_kernel(int mode, int method, int max_row, int rows_per_hw);
+int mf_small_chk_take();
 
 // ------------------------------------------------------- device utilities
 #ifdef __CUDACC__

@@ -9,9 +9,9 @@
 // kernels.
 //
 // What the pool holds beyond live allocations is bounded: at most kKeepBytes
-// (the release threshold; more goes back at the next synchronisation), and once
-// nothing is live, at most what was live since it was last empty
-// (mf_pool_settle).  A failed allocation gives the rest back and tries again.
+// (the release threshold follows what is live, see follow(); more goes back at
+// the next synchronisation), and once nothing is live, at most what was live
+// since it was last empty (mf_pool_settle).  A failed allocation gives the rest back and tries again.
 // The pool is stream-ordered and safe with any number of threads.
 #include "mf_internal.cuh"
 
@@ -37,7 +37,7 @@ int pool_of(int dev, cudaMemPool_t *out)
         cudaMemPool_t p = nullptr;
         MF_CUDA_TRY(cudaMemPoolCreate(&p, &pr));
         unsigned long long keep = kKeepBytes;
-        const cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        const cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);   // nothing live yet
         if (e != cudaSuccess) {
             cudaMemPoolDestroy(p);
             MF_CUDA_TRY(e);
@@ -47,6 +47,22 @@ int pool_of(int dev, cudaMemPool_t *out)
     *out = g_pool[dev];
     return MF_SUCCESS;
 }
+
+// The driver compares the release threshold with all the memory a pool holds,
+// live allocations included.  With a fixed one, handles above it (three 128^3
+// systems) had every freed array unmapped at the next synchronisation and mapped
+// again for the next solve (first solve of a handle 4.9 -> 8.5 ms).
+void follow(cudaMemPool_t pool)
+{
+    unsigned long long used = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
+        used += kKeepBytes;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &used);
+    }
+    cudaGetLastError();
+}
+
+constexpr size_t kFollowBytes = 4u << 20;    // allocations that move the threshold
 
 }  // namespace
 
@@ -69,6 +85,7 @@ int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s)
         cudaGetLastError();
     }
     MF_CUDA_TRY(e);
+    if (bytes >= kFollowBytes) follow(pool);
     return MF_SUCCESS;
 }
 
@@ -81,7 +98,9 @@ void mf_pool_settle(int dev)
 {
     cudaMemPool_t pool = nullptr;
     unsigned long long used = 0, high = 0, held = 0, zero = 0;
-    if (pool_of(dev, &pool) != MF_SUCCESS || cudaStreamSynchronize(0) != cudaSuccess ||
+    if (pool_of(dev, &pool) != MF_SUCCESS) return;
+    follow(pool);
+    if (cudaStreamSynchronize(0) != cudaSuccess ||
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > 0 ||
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &high) != cudaSuccess ||
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) {

@@ -9,10 +9,10 @@ template <int LEN>
 const void *rows_kernel(int mode, int method)
 {
     if (method == MF_METHOD_BICGSTAB)
-        return mode == MODE_FP64 ? (const void *)k_solve<MODE_FP64, 2, MF_METHOD_BICGSTAB, LEN>
-                                 : (const void *)k_solve<MODE_MIXED, 2, MF_METHOD_BICGSTAB, LEN>;
-    return mode == MODE_FP64 ? (const void *)k_solve<MODE_FP64, 2, MF_METHOD_CG, LEN>
-                             : (const void *)k_solve<MODE_MIXED, 2, MF_METHOD_CG, LEN>;
+        return mode == MODE_FP64 ? (const void *)k_solve<MODE_FP64, 2, MF_METHOD_BICGSTAB, LEN, kVarGrid>
+                                 : (const void *)k_solve<MODE_MIXED, 2, MF_METHOD_BICGSTAB, LEN, kVarGrid>;
+    return mode == MODE_FP64 ? (const void *)k_solve<MODE_FP64, 2, MF_METHOD_CG, LEN, kVarGrid>
+                             : (const void *)k_solve<MODE_MIXED, 2, MF_METHOD_CG, LEN, kVarGrid>;
 }
 
 }  // namespace

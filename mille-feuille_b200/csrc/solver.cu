@@ -51,13 +51,13 @@ template <int METH>
 const void *solve_kernel_m(int mode, int lb)
 {
     if (lb == 2) {
-        if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 2, METH, 0>;
-        if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 2, METH, 0>;
-        return (const void *)k_solve<MODE_PARITY, 2, METH, 0>;
+        if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 2, METH, 0, kVarGrid>;
+        if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 2, METH, 0, kVarGrid>;
+        return (const void *)k_solve<MODE_PARITY, 2, METH, 0, kVarGrid>;
     }
-    if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 1, METH, 0>;
-    if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 1, METH, 0>;
-    return (const void *)k_solve<MODE_PARITY, 1, METH, 0>;
+    if (mode == MODE_FP64) return (const void *)k_solve<MODE_FP64, 1, METH, 0, kVarGrid>;
+    if (mode == MODE_MIXED) return (const void *)k_solve<MODE_MIXED, 1, METH, 0, kVarGrid>;
+    return (const void *)k_solve<MODE_PARITY, 1, METH, 0, kVarGrid>;
 }
 
 const void *solve_kernel(int mode, int lb, int method)
@@ -107,6 +107,7 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
     memset(w, 0, sizeof(*w));
     w->G = G;
     w->lb = lb;
+    w->nsm = nsm;
     const long long L = A->vec_len;
     const long long S = std::max(A->tilem, A->tilen) + 1;
     {
@@ -147,6 +148,38 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
     MF_CUDA_TRY(cudaMemsetAsync(w->mag_p, 0, (size_t)S * sizeof(float), s));
     MF_CUDA_TRY(cudaMemsetAsync(w->mag_s, 0, (size_t)S * sizeof(float), s));
     MF_TRY(exact_tiles(A, w->counts, s));    // counts: scratch before the first solve zeroes it
+    // Small systems run as one cluster of up to 16 blocks, where the device can place
+    // it.  One-chunk matrices up to two tile-rows per half-warp (1,024): us per
+    // iteration, one cluster against the grid, 8,281 / 16,384 rows of the 2D
+    // Laplacian 3.2 / 3.4 against 6.2 / 6.1 (CG, FP64), 9,261 rows in 3D 4.2 against
+    // 7.0 (CG), 12.9 against 18.6 (BiCGSTAB); 32,768 rows 8.0 against 6.9.  Others
+    // have more to stream through 16 SMs: 27-point 9,261 rows 9.0 against 11.2,
+    // 32,768 rows 18.9 against 12.5; irregular 16,000 rows 11.3 against 11.5.
+    if (A->tilem <= (A->one_chunk ? 2 * kMaxCluster * kWarps * 2 : 768)) {
+        const void *fn = mf_solve_cluster_kernel(MODE_FP64, MF_METHOD_CG, 0, 1);
+        const int C = std::min(G, kMaxCluster);
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(C);
+        cfg.blockDim = dim3(kThreads);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = C;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess)
+            cudaGetLastError();
+        if (fit > 0) {
+            const int nhw = C * kWarps * 2;
+            w->cluster = C;
+            MF_TRY(mf_pool_array(&w->hw_begin_cl, nhw + 1, s));
+            k_partition<<<(nhw + 256) / 256, 256, 0, s>>>(A->d_row_cost, A->tilem, nhw, w->hw_begin_cl);
+            MF_CUDA_TRY(cudaGetLastError());
+        }
+    }
     w->nhw = G * kWarps * 2;
     MF_TRY(mf_pool_array(&w->hw_begin, w->nhw + 1, s));
     MF_CUDA_TRY(cudaEventCreate(&w->e0));
@@ -253,7 +286,7 @@ void mf_solver_free_ws(mf_matrix_s *A)
 {
     Workspace *w = (Workspace *)A->ws;
     if (!w) return;
-    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
+    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->hw_begin_cl, w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
     for (void *p : ptrs) mf_pool_free(p, 0);
     for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
     delete[] w->m_ev;
@@ -340,10 +373,41 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     // One-chunk matrices (the 5- and 7-point stencils) have kernels of their own
     // in the default two-blocks-per-SM budget; everything else, parity mode and
     // the one-block variant take the general walks.
+    // Systems with no more tile-rows than half-warps have kernels of theirs too.
+    // (They stay out of the stalled-barrier test, which needs the grid counter.)
     const bool rows = A->one_chunk && mode != MODE_PARITY && w->lb == 2;
-    const void *kfn = rows ? mf_solve_rows_kernel(mode, opt->method, A->max_row)
-                           : solve_kernel(mode, w->lb, opt->method);
-    cudaError_t lerr = cudaLaunchCooperativeKernel(kfn, dim3(w->G), dim3(kThreads), args, 0, s);
+    const bool small = mode != MODE_PARITY && w->lb == 2 && !opt->test_stall_barrier;
+    const bool cluster = small && w->cluster;
+    const void *kfn = cluster ? mf_solve_cluster_kernel(mode, opt->method, A->one_chunk ? A->max_row : 0,
+                                                          (A->tilem + w->cluster * kWarps * 2 - 1) /
+                                                              (w->cluster * kWarps * 2))
+                      : small && rows && opt->method == MF_METHOD_CG && A->tilem <= w->G * kWarps * 2
+                          ? mf_solve_resident_kernel(mode, w->G <= w->nsm ? 1 : 2, A->max_row)
+                      : rows ? mf_solve_rows_kernel(mode, opt->method, A->max_row)
+                             : solve_kernel(mode, w->lb, opt->method);
+    cudaError_t lerr;
+    if (cluster) {
+        // One cluster: its barrier and shared memory take the grid barrier's place
+        // (P.cluster).  An all-reduce with the barrier takes 0.9 us on 2 - 8 blocks and
+        // 1.05 on 16, through the grid counter 2.2 - 2.3 us.
+        P.cluster = w->cluster;
+        P.hw_begin = w->hw_begin_cl;
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(w->cluster);
+        cfg.blockDim = dim3(kThreads);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = w->cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        lerr = w->cluster > 8 ? cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
+        if (lerr == cudaSuccess) lerr = cudaLaunchKernelExC(&cfg, kfn, args);
+    } else {
+        lerr = cudaLaunchCooperativeKernel(kfn, dim3(w->G), dim3(kThreads), args, 0, s);
+    }
     if (lerr != cudaSuccess) {
         win.reset(s);
         MF_CUDA_TRY(lerr);
@@ -359,6 +423,7 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     int err = rb.err;
     int chk = chk_take();
     if (!chk) chk = mf_rows_chk_take();
+    if (!chk) chk = mf_small_chk_take();
     if (chk) err = chk;
     const auto t_done = std::chrono::steady_clock::now();
     float ms = 0.f;
@@ -375,7 +440,7 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
         rep->replacements = (int)out[5];
         rep->status = err ? err : (int)out[6];
         rep->time_ms = ms;
-        rep->grid_blocks = w->G;
+        rep->grid_blocks = cluster ? w->cluster : w->G;
         rep->threads_per_block = kThreads;
         for (int j = 0; j < 4; j++) rep->tile_uses[j] = (long long)counts[j];
         rep->tiles_skipped = (long long)counts[4];

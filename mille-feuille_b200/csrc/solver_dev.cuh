@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 namespace {
 
@@ -122,9 +123,16 @@ struct SolverParams {
     int nseg, ntiles, chk_xlen;
     long long n_payload;
     long long nnz;
+    int cluster;               // > 0: the launch is one cluster of this many blocks
 };
 
-struct Shared {
+constexpr int kMaxCluster = 16;
+
+// CL: a launch of one cluster (SolverParams::cluster blocks)
+template <bool CL>
+struct SharedT {
+    static constexpr bool kCluster = CL;
+    double part[CL ? kRedKinds : 1][kRedWidth][kMaxCluster];   // every block's partials
     double wred[kWarps][kRedWidth];
     double bcast[kRedWidth];
     int flag;
@@ -134,13 +142,32 @@ struct Shared {
 };
 
 // ------------------------------------------------------------ grid barrier
+// One-cluster solves: the hardware's cluster barrier, with release / acquire of
+// everything the blocks wrote.  It waits for the threads of the cluster that
+// have not exited, and all of them run through the same barriers, so it needs no
+// limit of its own.
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A double into another block's copy of `p` (shared memory of the cluster's block `rank`).
+__device__ __forceinline__ void cluster_store(double *p, int rank, double v)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    unsigned ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(ra), "d"(v) : "memory");
+}
+
 template <class SH>
 __device__ bool grid_barrier(const SolverParams &P, unsigned &epoch, SH &sh)
 {
     __syncthreads();
     epoch += 1;
     if (threadIdx.x == 0) {
-        const unsigned long long tw0 = mf_globaltimer();
+        const bool timed = blockIdx.x == 0 && P.phase_ns;
+        const unsigned long long tw0 = timed ? mf_globaltimer() : 0ull;
         const unsigned target = epoch * gridDim.x + ((P.stall_first_barrier && epoch == 1) ? 1u : 0u);
         // fence-release pattern: the block's writes (ordered before by bar.sync) are
         // visible at gpu scope before the arrival; polls are relaxed loads and one
@@ -162,15 +189,28 @@ __device__ bool grid_barrier(const SolverParams &P, unsigned &epoch, SH &sh)
         }
         mf_fence_acq_rel_gpu();
         sh.flag = ok ? 1 : 0;
-        if (blockIdx.x == 0 && P.phase_ns) P.phase_ns[5] += mf_globaltimer() - tw0;   // block 0 spin time
+        if (timed) P.phase_ns[5] += mf_globaltimer() - tw0;   // block 0 spin time
     }
     __syncthreads();
     return sh.flag != 0;
 }
 
+// The barrier of a solve: the cluster's or the grid's.
+template <bool CL>
+__device__ __forceinline__ bool solve_barrier(const SolverParams &P, unsigned &epoch, SharedT<CL> &sh)
+{
+    if constexpr (CL) {
+        cluster_barrier();
+        return true;
+    } else {
+        return grid_barrier(P, epoch, sh);
+    }
+}
+
 // Block partial of up to 4 sums (mask bit k set -> max instead of sum) written
 // to red[kind][k][block] (value-major, so a collect reads consecutive blocks).
-__device__ void block_partial(const SolverParams &P, Shared &sh, int kind, double v0, double v1, double v2,
+template <bool CL>
+__device__ void block_partial(const SolverParams &P, SharedT<CL> &sh, int kind, double v0, double v1, double v2,
                               double v3, int nv, unsigned maxmask)
 {
     double v[kRedWidth] = {v0, v1, v2, v3};
@@ -188,17 +228,18 @@ __device__ void block_partial(const SolverParams &P, Shared &sh, int kind, doubl
         if (lane == 0) sh.wred[wib][k] = a;
     }
     __syncthreads();
-    if (wib == 0) {
-        for (int k = 0; k < nv; k++) {
-            const bool mx = (maxmask >> k) & 1u;
-            double a = (lane < kWarps) ? sh.wred[lane][k] : (mx ? -1.0e300 : 0.0);
+    if (wib < nv) {                       // warp k reduces value k
+        const int k = wib;
+        const bool mx = (maxmask >> k) & 1u;
+        double a = (lane < kWarps) ? sh.wred[lane][k] : (mx ? -1.0e300 : 0.0);
 #pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                double b = __shfl_xor_sync(0xffffffffu, a, o);
-                a = mx ? fmax(a, b) : a + b;
-            }
-            if (lane == 0) P.red[((long long)kind * kRedWidth + k) * gridDim.x + blockIdx.x] = a;
+        for (int o = 16; o; o >>= 1) {
+            double b = __shfl_xor_sync(0xffffffffu, a, o);
+            a = mx ? fmax(a, b) : a + b;
         }
+        if (CL) {
+            if (lane < P.cluster) cluster_store(&sh.part[CL ? kind : 0][k][blockIdx.x], lane, a);
+        } else if (lane == 0) P.red[((long long)kind * kRedWidth + k) * gridDim.x + blockIdx.x] = a;
     }
 }
 
@@ -209,9 +250,25 @@ __device__ void block_partial(const SolverParams &P, Shared &sh, int kind, doubl
 // trip instead of one per partial.  No trailing barrier: the next writer of
 // sh.bcast is the next collect, which every thread reaches only through the
 // barriers of block_partial and grid_barrier, after it has read bcast here.
-__device__ void grid_collect(const SolverParams &P, Shared &sh, int kind, int nv, unsigned maxmask,
+template <bool CL>
+__device__ void grid_collect(const SolverParams &P, SharedT<CL> &sh, int kind, int nv, unsigned maxmask,
                              double *outv)
 {
+    if constexpr (CL) {
+        // every block holds all partials: each thread sums them in the same order
+#pragma unroll
+        for (int k = 0; k < kRedWidth; k++) {
+            if (k >= nv) break;
+            const bool mx = (maxmask >> k) & 1u;
+            double a = sh.part[kind][k][0];
+            for (int c = 1; c < P.cluster; c++) {
+                const double b = sh.part[kind][k][c];
+                a = mx ? fmax(a, b) : a + b;
+            }
+            outv[k] = a;
+        }
+        return;
+    }
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (wib < nv) {
         const bool mx = (maxmask >> wib) & 1u;
@@ -238,7 +295,9 @@ __device__ void grid_collect(const SolverParams &P, Shared &sh, int kind, int nv
         if (lane == 0) sh.bcast[wib] = a;
     }
     __syncthreads();
-    for (int k = 0; k < nv; k++) outv[k] = sh.bcast[k];
+#pragma unroll
+    for (int k = 0; k < kRedWidth; k++)
+        if (k < nv) outv[k] = sh.bcast[k];
 }
 
 // ------------------------------------------------------------ tile SpMV
@@ -981,10 +1040,11 @@ __device__ __forceinline__ XVec fp64_x(const double *x64)
 // 1 -> up to 128 registers (no spills, 16 warps / SM), 2 -> 64 registers (32 warps / SM).
 // Block 0 / thread 0 splits its wall time into phases (%globaltimer deltas);
 // the state lives in shared memory so the other threads spend no registers on it.
+template <class SH>
 struct PhaseClock {
-    Shared *sh;
+    SH *sh;
     __device__ bool on() const { return blockIdx.x == 0 && threadIdx.x == 0; }
-    __device__ void start(Shared *s)
+    __device__ void start(SH *s)
     {
         sh = s;
         if (on()) {
@@ -1041,12 +1101,21 @@ __device__ __forceinline__ int relaxed_precision(const SolverParams &P, double r
 // each gets its own register allocation: the kernel sits at the 64-register
 // limit of two 512-thread blocks per SM, and code in one method's branch
 // moves spills into the other's hot loop.
+enum { kVarGrid = 0, kVarResident = 1, kVarCluster = 2, kVarCluster2 = 3 };
 // LEN > 0: for one-chunk matrices with rows of up to LEN entries (spmv_rows); these
 // instantiations hold none of the general walks.
-template <int MODE, int LB, int METH, int LEN>
+// VAR: kVarGrid the whole chip; kVarResident a grid with no more tile-rows than
+// half-warps (CG iterations stay in registers); kVarCluster and kVarCluster2 one
+// cluster with up to one and two tile-rows per half-warp in registers (four did
+// not fit 128 registers: 32,768 rows took 8.0 us an iteration against 6.9 on the
+// grid).  Instantiations of their own: the resident loop and the cluster's
+// reduction inside the large kernels raised their spills from 0 - 68 to 250 - 300
+// bytes.
+template <int MODE, int LB, int METH, int LEN, int VAR>
 __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
 {
-    __shared__ Shared sh;
+    constexpr bool CL = VAR >= kVarCluster;
+    __shared__ SharedT<CL> sh;
     const Ctx c = make_ctx(P);
     unsigned epoch = 0;
     // tile-use counters: FP64 mode needs none (every tile of every SpMV is FP64;
@@ -1056,7 +1125,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     if (threadIdx.x < 4) sh.whole[threadIdx.x] = 0u;
     int nspmv = 0;
     __syncwarp();
-    PhaseClock clk;
+    PhaseClock<SharedT<CL>> clk;
     clk.start(&sh);
     const int n = P.n;
     constexpr bool bicg = (METH == MF_METHOD_BICGSTAB);
@@ -1073,7 +1142,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             if (row < n) pbb += P.b[row] * P.b[row];
         }
         block_partial(P, sh, 8, pbb, 0, 0, 0, 1, 0u);
-        if (!grid_barrier(P, epoch, sh)) return;
+        if (!solve_barrier(P, epoch, sh)) return;
         double vb[4] = {0.0, 0.0, 0.0, 0.0};
         grid_collect(P, sh, 8, 1, 0u, vb);
         bb0 = vb[0];
@@ -1115,11 +1184,12 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     }
     // the smallest segment magnitude (carried as -min) matters only to the mixed
     // mode's SpMV; FP64 and parity reduce (sum, max) as before
-    // (sum, max, -min, small segments) in mixed mode; FP64 and parity reduce (sum, max)
-    constexpr int kNvSeg = (MODE == MODE_MIXED) ? 4 : 2;
-    constexpr int kNvSegB = (MODE == MODE_MIXED) ? 3 : 1;      // (max, -min, small) without a sum
+    // (sum, max, -min, small segments) in mixed mode, (sum, max) in parity mode; FP64
+    // reads no magnitudes and reduces the sum alone
+    constexpr int kNvSeg = (MODE == MODE_MIXED) ? 4 : (MODE == MODE_PARITY) ? 2 : 1;
+    constexpr int kNvSegB = (MODE == MODE_MIXED) ? 3 : (MODE == MODE_PARITY) ? 1 : 0;   // without a sum
     block_partial(P, sh, 0, pb, (double)bmax, -(double)bmin, (double)nsm, kNvSeg, 0x6u);
-    if (!grid_barrier(P, epoch, sh)) return;
+    if (!solve_barrier(P, epoch, sh)) return;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     grid_collect(P, sh, 0, kNvSeg, 0x6u, v);
     // mixed: can any tile of the next SpMV leave FP32 at all?  Not when the
@@ -1182,8 +1252,148 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     // mixed CG: uniform reduced precision of the next SpMV (relaxed_precision)
     int prA = (MODE == MODE_MIXED) ? relaxed_precision(P, rr, bb) : MF_P32;
 
+    // ---- resident iterations (CG, one-chunk matrices, up to kKR tile-rows per half-warp) ----
+    // With no more tile-rows than that (kKR = 1 on the grid: 151,552 rows on 148 SMs)
+    // everything a lane needs of its rows stays in registers from one iteration to
+    // the next: values, gather positions, p, q, x and r.  An iteration is then the
+    // gather of r from L2, two reductions and one store of r.  Without it an
+    // iteration of the 256^2 Laplacian spent 2.2 us (FP64) on loads that depend on
+    // one another (tile word and values, gathered r, then p and q; x, p, r, q in the
+    // update).
+    // The loop leaves for the general iteration's tail (`tail`) when a residual
+    // replacement or a convergence check is due, at the end, and in mixed mode when
+    // enough segments are small that narrower tiles may be chosen; x, p and q
+    // are written back then, and a barrier makes them visible.
+    constexpr bool kRes = VAR != kVarGrid && MODE != MODE_PARITY && !bicg && LEN > 0;
+    constexpr int kKR = VAR == kVarCluster2 ? 2 : 1;
+    constexpr int kLen = LEN > 0 ? LEN : 1;
+    const int resR = (int)(blockIdx.x * kWarps * 2 + (threadIdx.x >> 4)), resS = (int)gridDim.x * kWarps * 2;
+    const bool resident = kRes && P.tilem <= kKR * resS && P.relax_eta <= 0.0f;
+
     while (!conv && k < P.max_iter) {
+        bool tail = false;
+        double rr_tail = 0.0;
+        float rthr = invM > 0.0f ? P.demote16 / invM : -1.0f;
+        if constexpr (kRes) {
+            if (resident && !dynA && (MODE == MODE_FP64 || !magB)) {
+                typename std::conditional<MODE == MODE_FP64, double, float>::type val[kKR][kLen];
+                int at[kKR][kLen];
+                double xr[kKR], pr[kKR], qr[kKR], rv[kKR];
+                bool own[kKR], valid[kKR];
+#pragma unroll
+                for (int u = 0; u < kKR; u++) {
+                    const int R = resR + u * resS, row = R * MF_BS + c.i;
+                    own[u] = R < P.tilem;                       // uniform over the half-warp
+                    valid[u] = own[u] && row < n;
+#pragma unroll
+                    for (int j = 0; j < kLen; j++) {
+                        val[u][j] = 0;
+                        at[u][j] = 0;
+                    }
+                    const long long cb = (long long)R * 128;
+                    if (own[u] && chk_in(CHK_PAYLOAD, cb + 127, P.n_payload)) {
+                        const int xb = (load_tw(P, R, c.i) >> 8) * MF_BS;
+                        const unsigned long long m8 = *((const unsigned long long *)(P.meta + cb) + c.i);
+#pragma unroll
+                        for (int j = 0; j < LEN; j++) {
+                            const unsigned mm = (unsigned)(m8 >> (8 * j)) & 0xFFu;
+                            const int xi = __shfl_sync(c.hmask, xb, (int)(mm >> 4), 16) + (int)(mm & 15u);
+                            if (!chk_in(CHK_X, xi, P.chk_xlen)) continue;
+                            at[u][j] = xi;
+                            if (MODE == MODE_FP64) val[u][j] = P.v64[mf_slot<8>(cb, j, c.i)];
+                            else val[u][j] = P.lean_f16 ? __half2float(P.v16[mf_slot<2>(cb, j, c.i)])
+                                                        : P.v32[mf_slot<4>(cb, j, c.i)];
+                        }
+                    }
+                    xr[u] = valid[u] ? P.x[row] : 0.0;
+                    pr[u] = valid[u] ? P.p[row] : 0.0;
+                    qr[u] = valid[u] ? P.q[row] : 0.0;
+                    rv[u] = valid[u] ? P.r[row] : 0.0;
+                }
+                unsigned done = 0;
+                for (;;) {
+                    double ppq = 0.0;
+                    {
+                        double xv[kKR][kLen];
+#pragma unroll
+                        for (int u = 0; u < kKR; u++)
+                            if (own[u]) {
+#pragma unroll
+                                for (int j = 0; j < LEN; j++) xv[u][j] = P.r[at[u][j]];
+                            }
+#pragma unroll
+                        for (int u = 0; u < kKR; u++) {
+                            double w = 0.0;
+                            if (own[u]) {
+#pragma unroll
+                                for (int j = 0; j < LEN; j++) w = fma((double)val[u][j], xv[u][j], w);
+                            }
+                            pr[u] = rv[u] + beta2 * pr[u];
+                            qr[u] = w + beta2 * qr[u];
+                            if (valid[u]) ppq += pr[u] * qr[u];
+                        }
+                    }
+                    done++;
+                    clk.lap(PH_SPMV);
+                    block_partial(P, sh, 1, ppq, 0, 0, 0, 1, 0u);
+                    if (!solve_barrier(P, epoch, sh)) return;
+                    grid_collect(P, sh, 1, 1, 0u, v);
+                    clk.lap(PH_BAR);
+                    const double alpha2 = rr / v[0];
+                    if (!isfinite(alpha2)) { status = MF_ERR_BREAKDOWN; break; }
+                    rthr = invM > 0.0f ? P.demote16 / invM : -1.0f;
+                    const bool voteB = (k & 3) == 0;
+                    double prr = 0.0;
+                    float rmax = 0.0f, rsm = 0.0f;
+#pragma unroll
+                    for (int u = 0; u < kKR; u++) {
+                        xr[u] += alpha2 * pr[u];
+                        rv[u] = valid[u] ? rv[u] - alpha2 * qr[u] : 0.0;
+                        if (valid[u]) P.r[(resR + u * resS) * MF_BS + c.i] = rv[u];
+                        prr += rv[u] * rv[u];
+                        const float m = (float)fabs(rv[u]);
+                        rmax = fmaxf(rmax, m);
+                        if (MODE == MODE_MIXED && voteB && own[u] && __all_sync(c.hmask, m <= rthr) && c.i == 0)
+                            rsm += 1.0f;
+                    }
+                    clk.lap(PH_VECB);
+                    // (without counted segments only r's norm and maximum are read)
+                    const int nvB = (MODE == MODE_MIXED && !voteB) ? 2 : kNvSeg;
+                    block_partial(P, sh, 2, prr, (double)rmax, -(double)3.0e38f, (double)rsm, nvB, 0x6u);
+                    if (!solve_barrier(P, epoch, sh)) return;
+                    grid_collect(P, sh, 2, nvB, 0x6u, v);
+                    clk.lap(PH_BAR);
+                    invM = v[1] > 0.0 ? (float)(1.0 / v[1]) : 0.0f;
+                    if (MODE == MODE_MIXED && voteB) magB = (P.lossless_any || v[3] >= (double)half_small) ? 1 : 0;
+                    if ((!P.fixed_iters && v[0] <= thr2) || (P.replace_every > 0 && (k + 1) % P.replace_every == 0) ||
+                        k + 1 >= P.max_iter || (MODE == MODE_MIXED && magB))
+                        break;
+                    beta2 = v[0] / rr;
+                    rr = v[0];
+                    k++;
+                    last_true = 0;
+                }
+                rr_tail = v[0];
+                tail = true;
+                nspmv += (int)done;
+                if (MODE == MODE_MIXED && blockIdx.x == 0 && threadIdx.x == 0)
+                    sh.whole[P.lean_f16 ? MF_P16 : MF_P32] += done;
+#pragma unroll
+                for (int u = 0; u < kKR; u++)
+                    if (valid[u]) {
+                        const int row = (resR + u * resS) * MF_BS + c.i;
+                        P.x[row] = xr[u];
+                        P.p[row] = pr[u];
+                        P.q[row] = qr[u];
+                    }
+                if (!solve_barrier(P, epoch, sh)) return;
+                if (status) break;
+            }
+        }
         if (MODE != MODE_PARITY && !bicg) {
+            double rr_new = rr_tail;
+            float rmax = 0.0f, rmin = 3.0e38f, rsm = 0.0f;
+            if (!tail) {
             // CG with two grid syncs per iteration.  The SpMV is applied to r:
             // w = A r, then p = r + beta p and q = A p = w + beta q, so p never
             // needs a halo of its own; alpha = r.r / p.q and beta = r'.r' / r.r
@@ -1221,15 +1431,13 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             nspmv++;
             clk.lap(PH_SPMV);
             block_partial(P, sh, 1, ppq, 0, 0, 0, 1, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 1, 1, 0u, v);
             clk.lap(PH_BAR);
             const double alpha2 = rr / v[0];
             if (!isfinite(alpha2)) { status = MF_ERR_BREAKDOWN; break; }
             // ---- B: x += alpha p; r -= alpha q; r.r; r's shadow ----
             double prr = 0.0;
-            float rmax = 0.0f, rmin = 3.0e38f, rsm = 0.0f;
-            const float rthr = invM > 0.0f ? P.demote16 / invM : -1.0f;
             const bool voteB = magB || (k & 3) == 0;     // this update counts small segments
             // kVB tile-rows per step: all loads first, so kVB round trips overlap
             for (int R0 = c.rbeg; R0 < c.rend; R0 += kVB) {
@@ -1267,16 +1475,17 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             }
             clk.lap(PH_VECB);
             block_partial(P, sh, 2, prr, (double)rmax, -(double)rmin, (double)rsm, kNvSeg, 0x6u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 2, kNvSeg, 0x6u, v);
             clk.lap(PH_BAR);
-            double rr_new = v[0];
-            const double rr_rec = rr_new;       // recursive r.r of this iteration
+            rr_new = v[0];
             invM = v[1] > 0.0 ? (float)(1.0 / v[1]) : 0.0f;
             if (MODE == MODE_MIXED) {
                 dynA = magB ? dyn_of(v[1], v[2], v[3]) : 0;
                 if (voteB) magB = (P.lossless_any || v[3] >= (double)half_small) ? 1 : 0;
             }
+            }
+            const double rr_rec = rr_new;       // recursive r.r of this iteration
             k++;
             last_true = 0;
             const bool want_check = !P.fixed_iters && rr_new <= thr2;
@@ -1318,7 +1527,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                 }
                 clk.lap(PH_REPL);
                 block_partial(P, sh, 5, prt, (double)rmax, -(double)rmin, (double)rsm, kNvSeg, 0x6u);
-                if (!grid_barrier(P, epoch, sh)) return;
+                if (!solve_barrier(P, epoch, sh)) return;
                 grid_collect(P, sh, 5, kNvSeg, 0x6u, v);
                 clk.lap(PH_BAR);
                 rr_new = v[0];
@@ -1354,7 +1563,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             nspmv++;
             clk.lap(PH_SPMV);
             block_partial(P, sh, 1, ppq, 0, 0, 0, 1, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 1, 1, 0u, v);
             clk.lap(PH_BAR);
             alpha = rr / v[0];
@@ -1382,7 +1591,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             }
             clk.lap(PH_VECB);
             block_partial(P, sh, 2, prr, 0, 0, 0, 1, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 2, 1, 0u, v);
             clk.lap(PH_BAR);
         } else {
@@ -1402,7 +1611,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             nspmv++;
             clk.lap(PH_SPMV);
             block_partial(P, sh, 1, prv, (double)(demoted() - d0A), 0, 0, kNvFb, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 1, kNvFb, 0u, v);
             clk.lap(PH_BAR);
             if (kFb) coolA = next_cool(coolA, useA != 0, v[1]);
@@ -1426,7 +1635,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             clk.lap(PH_VECB);
             // (max, -min) of s's segment magnitudes; only the mixed mode uses the minimum
             block_partial(P, sh, 2, (double)smax, -(double)smin, (double)ssm, 0, kNvSegB, 0x3u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 2, kNvSegB, 0x3u, v);
             clk.lap(PH_BAR);
             invMs = v[0] > 0.0 ? (float)(1.0 / v[0]) : 0.0f;
@@ -1448,7 +1657,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             nspmv++;
             clk.lap(PH_SPMV);
             block_partial(P, sh, 3, pts, ptt, (double)(demoted() - d0S), 0, kNvFb + 1, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 3, kNvFb + 1, 0u, v);
             clk.lap(PH_BAR);
             if (kFb) coolS = next_cool(coolS, useS != 0, v[2]);
@@ -1469,7 +1678,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             }
             clk.lap(PH_VECB);
             block_partial(P, sh, 4, prr, prh, 0, 0, 2, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 4, 2, 0u, v);
             clk.lap(PH_BAR);
         }
@@ -1489,7 +1698,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                     if (row < n) P.x[row] += alpha * P.p[row];
                 }
                 x_done = true;
-                if (!grid_barrier(P, epoch, sh)) return;
+                if (!solve_barrier(P, epoch, sh)) return;
             }
             // ---- FP64 true residual: r = b - A x ----
             double prt = 0.0, prth = 0.0;
@@ -1515,7 +1724,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             }
             clk.lap(PH_REPL);
             block_partial(P, sh, 5, prt, prth, 0, 0, 2, 0u);
-            if (!grid_barrier(P, epoch, sh)) return;
+            if (!solve_barrier(P, epoch, sh)) return;
             grid_collect(P, sh, 5, 2, 0u, v);
             clk.lap(PH_BAR);
             rr_new = v[0];
@@ -1573,7 +1782,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
         }
         clk.lap(PH_VECC);
         block_partial(P, sh, 6, (double)bmax, -(double)pmin, (double)psm, 0, kNvSegB, 0x3u);
-        if (!grid_barrier(P, epoch, sh)) return;
+        if (!solve_barrier(P, epoch, sh)) return;
         grid_collect(P, sh, 6, kNvSegB, 0x3u, v);
             clk.lap(PH_BAR);
         invM = v[0] > 0.0 ? (float)(1.0 / v[0]) : 0.0f;
@@ -1595,7 +1804,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             if (row < n) prt += P.b[row] * P.b[row];
         }
         block_partial(P, sh, 7, prt, 0, 0, 0, 1, 0u);
-        if (!grid_barrier(P, epoch, sh)) return;
+        if (!solve_barrier(P, epoch, sh)) return;
         grid_collect(P, sh, 7, 1, 0u, v);
             clk.lap(PH_BAR);
         rr_true = v[0];
@@ -1637,6 +1846,9 @@ constexpr size_t kCtlBytes = 128 + sizeof(Readback);
 struct Workspace {
     int G;                 // grid blocks of the persistent kernel
     int lb;                // register-budget variant (blocks per SM it was built for)
+    int cluster;           // blocks of a one-cluster launch (0: none), and its partition
+    int *hw_begin_cl;
+    int nsm;
     // every solver vector lives in one block, ordered so that one L2
     // access-policy window can cover any number of the vectors a solve reuses
     // most (vec_window):

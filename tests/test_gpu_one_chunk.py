@@ -1,7 +1,8 @@
 """Matrices whose every tile-row is one chunk (rows of up to 8 entries in up to 15
 tiles) have walks and solve kernels of their own, by their longest row (5, 7, 8).
-Row counts at the edges of a tile-row (16), of a block's turn (32 tile-rows) and
-of two blocks; longest rows on both sides of each kernel's limit; a matrix with
+Row counts at the edges of a tile-row (16), of a block's turn (32 tile-rows), of
+one cluster (512 tile-rows), of one and two blocks per SM (where CG iterations
+stop being kept in registers); longest rows on both sides of each kernel's limit; a matrix with
 one empty tile-row (which takes the general kernels) beside each.
 
 Bounds: a product's row is a sum of k <= 9 terms in FP64, within k eps of
@@ -72,7 +73,8 @@ def _bicgstab(A, b, k):
 
 
 @pytest.mark.parametrize("longest", [1, 5, 6, 7, 8])
-@pytest.mark.parametrize("n", [1, 16, 17, 511, 512, 513, 1025, 148 * 2 * 512 + 33])
+@pytest.mark.parametrize("n", [1, 16, 17, 511, 512, 513, 1025, 8192, 8193, 148 * 512 + 1, 148 * 2 * 512,
+                               148 * 2 * 512 + 33])
 @pytest.mark.parametrize("empty_tile_row", [False, True])
 def test_one_chunk_products_and_solves(mf, cuda, n, longest, empty_tile_row):
     import torch
