@@ -19,7 +19,7 @@ constexpr int kRedWidthM = kMaxNR + 2;    // NR dot products + segment max / -mi
 struct SharedM {
     double wred[kWarps][kRedWidthM];
     double bcast[kRedWidthM];
-    double alpha[kMaxNR], beta[kMaxNR], rr[kMaxNR], thr2[kMaxNR], bb[kMaxNR];
+    double alpha[kMaxNR], beta[kMaxNR], rr[kMaxNR], thr2[kMaxNR], bb[kMaxNR], rt[kMaxNR];
     int active[kMaxNR], pending[kMaxNR], iters[kMaxNR], conv[kMaxNR];
     int brk;                  // some column broke down (a scalar became non-finite)
     int flag;                 // grid_barrier's result
@@ -29,7 +29,7 @@ struct MultiParams {
     const double *B;          // [vec_len * NR] interleaved right-hand sides (zero columns past nr)
     double *X, *R, *Pv, *Q;   // interleaved
     float *mag;               // per tile-row: max over its rows and columns of |R|
-    double *red;              // [kinds][G][kRedWidthM]
+    double *red;              // [kinds][kRedWidthM][blocks]: a collect reads consecutive blocks
     double *out;              // per column: iterations, converged, true rel. residual, recursive; then k, status
     int nr;                   // columns in use
 };
@@ -62,20 +62,22 @@ __device__ void block_partial_m(const MultiParams &M, SharedM &sh, int kind, con
             const double b = __shfl_xor_sync(0xffffffffu, a, o);
             a = mx ? fmax(a, b) : a + b;
         }
-        if (lane == 0) M.red[((long long)kind * nblk + bidx) * kRedWidthM + wib] = a;
+        if (lane == 0) M.red[((long long)kind * kRedWidthM + wib) * nblk + bidx] = a;
     }
 }
 
 // After the sync: every block of the group sums the nblk partials of `kind` in
-// the same order.
+// the same order, into sh.bcast.  It stays there until the next collect, which
+// every thread reaches only through the barriers of block_partial_m and of the
+// sync, so there is no trailing barrier.
 template <int NV>
-__device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsigned maxmask, double (&out)[NV],
-                               int nblk)
+__device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsigned maxmask, int nblk)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (wib < NV) {
         const bool mx = (maxmask >> wib) & 1u;
         const double id = mx ? -1.0e300 : 0.0;
+        const double *src = M.red + ((long long)kind * kRedWidthM + wib) * nblk;
         double a = id;
         // lane c takes blocks c, c + 32, ...; a pass issues all its loads first
         constexpr int kU = 5;               // 160 blocks per pass (one block per SM on 148 SMs)
@@ -84,7 +86,7 @@ __device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsi
 #pragma unroll
             for (int j = 0; j < kU; j++) {
                 const int cb = c0 + lane + 32 * j;
-                t[j] = cb < nblk ? M.red[((long long)kind * nblk + cb) * kRedWidthM + wib] : id;
+                t[j] = cb < nblk ? src[cb] : id;
             }
 #pragma unroll
             for (int j = 0; j < kU; j++) a = mx ? fmax(a, t[j]) : a + t[j];
@@ -96,9 +98,6 @@ __device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsi
         }
         if (lane == 0) sh.bcast[wib] = a;
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; k++) out[k] = sh.bcast[k];
     __syncthreads();
 }
 
@@ -257,7 +256,10 @@ __device__ __forceinline__ void store_row(double *v, int row, const double (&in)
 }
 
 // The CG iterations on NR columns, generic in how the threads that share a
-// system synchronise: the whole grid (k_solve_multi) or one block (k_batch).
+// system synchronise: the whole grid (k_solve_multi), a team or one block
+// (k_batch).  sy.reduce leaves its results in sh.bcast; thread j keeps column j's
+// scalars (one thread for all of them spent 8 divisions in a row on every
+// block's critical path, twice an iteration).
 template <int MODE, int NR, class Sync>
 __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const Ctx &c, SharedM &sh, Sync &sy)
 {
@@ -269,7 +271,7 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
     // ---- init: X = 0, R = B, P = Q = 0; |b_k|^2; R's segment magnitudes ----
     // With an initial guess (x0_given): |b_k|^2 reduced first (it scales the
     // convergence test), then R = B - A X in FP64.
-    double pb[NR + 2], bb0[NR];
+    double pb[NR + 2];
 #pragma unroll
     for (int k = 0; k < NR + 2; k++) pb[k] = 0.0;
     SegMM st = {0.0f, 3.0e38f};
@@ -286,7 +288,8 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
                 for (int k = 0; k < NR; k++) pbb[k] += bv[k] * bv[k];
             }
         }
-        if (!sy.template reduce<NR>(8, pbb, 0u, bb0)) return;
+        if (!sy.template reduce<NR>(8, pbb, 0u)) return;
+        if (threadIdx.x < NR) sh.bb[threadIdx.x] = sh.bcast[threadIdx.x];
         auto init_r = [&](int R, const double (&y)[NR]) {
             const int row = R * MF_BS + c.i;
             const bool valid = row < n;
@@ -334,33 +337,31 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
     }
     pb[NR] = st.mx;
     pb[NR + 1] = -st.mn;
-    double v[NR + 2];
-    if (!sy.template reduce<NR + 2>(0, pb, mm2, v)) return;
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NR; k++) {
-            sh.bb[k] = P.x0_given ? bb0[k] : v[k];
-            sh.rr[k] = v[k];
-            sh.thr2[k] = P.tol * P.tol * sh.bb[k];
-            sh.beta[k] = 0.0;
-            sh.pending[k] = 0;
-            sh.iters[k] = 0;
-            sh.conv[k] = (k < M.nr && !P.fixed_iters && v[k] <= sh.thr2[k]) ? 1 : 0;
-            sh.active[k] = (k < M.nr && !sh.conv[k]) ? 1 : 0;
-        }
-        sh.brk = 0;
+    if (!sy.template reduce<NR + 2>(0, pb, mm2)) return;
+    if (threadIdx.x < NR) {
+        const int k = threadIdx.x;
+        const double rr0 = sh.bcast[k];
+        if (!P.x0_given) sh.bb[k] = rr0;
+        sh.rr[k] = rr0;
+        sh.rt[k] = rr0;
+        sh.thr2[k] = P.tol * P.tol * sh.bb[k];
+        sh.beta[k] = 0.0;
+        sh.pending[k] = 0;
+        sh.iters[k] = 0;
+        sh.conv[k] = (k < M.nr && !P.fixed_iters && rr0 <= sh.thr2[k]) ? 1 : 0;
+        sh.active[k] = (k < M.nr && !sh.conv[k]) ? 1 : 0;
     }
+    if (threadIdx.x == 0) sh.brk = 0;
+    float invM = sh.bcast[NR] > 0.0 ? (float)(1.0 / sh.bcast[NR]) : 0.0f;
+    const double neg_mn0 = sh.bcast[NR + 1], mx0 = sh.bcast[NR];
     __syncthreads();
-    float invM = v[NR] > 0.0 ? (float)(1.0 / v[NR]) : 0.0f;
     // mixed: some tile may leave FP32 only if the smallest segment is below
     // demote_fp16 of the largest or lossless classes apply (see dyn in XVec)
     auto dyn_of = [&](double mx, double neg_mn) -> int {
         return (P.lossless_any || mx <= 0.0 || -neg_mn <= (double)P.demote16 * mx) ? 1 : 0;
     };
-    int dyn = dyn_of(v[NR], v[NR + 1]);
+    int dyn = dyn_of(mx0, neg_mn0);
     int k = 0, status = 0, repl = 0, last_true = 0;
-    double rt[NR];
-#pragma unroll
-    for (int j = 0; j < NR; j++) rt[j] = v[j];
 
     for (;;) {
         int any = 0;
@@ -396,18 +397,16 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
             for (int R = c.rbeg; R < c.rend; R++)
                 if (P.seg_ptr[R] == P.seg_ptr[R + 1]) upd_a(R, zw);
         }
-        double pq[NR];
-        if (!sy.template reduce<NR>(1, ppq, 0u, pq)) return;
-        if (threadIdx.x == 0) {
-            for (int j = 0; j < NR; j++) {
-                double a = sh.active[j] ? sh.rr[j] / pq[j] : 0.0;
-                if (!isfinite(a)) {      // breakdown of this column: it stops where it is
-                    a = 0.0;
-                    sh.active[j] = 0;
-                    sh.brk = 1;
-                }
-                sh.alpha[j] = a;
+        if (!sy.template reduce<NR>(1, ppq, 0u)) return;
+        if (threadIdx.x < NR) {
+            const int j = threadIdx.x;
+            double a = sh.active[j] ? sh.rr[j] / sh.bcast[j] : 0.0;
+            if (!isfinite(a)) {          // breakdown of this column: it stops where it is
+                a = 0.0;
+                sh.active[j] = 0;
+                sh.brk = 1;
             }
+            sh.alpha[j] = a;
         }
         __syncthreads();
         if (sh.brk) status = MF_ERR_BREAKDOWN;
@@ -441,18 +440,18 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
         }
         prr[NR] = st.mx;
         prr[NR + 1] = -st.mn;
-        if (!sy.template reduce<NR + 2>(2, prr, mm2, v)) return;
-        invM = v[NR] > 0.0 ? (float)(1.0 / v[NR]) : 0.0f;
-        dyn = dyn_of(v[NR], v[NR + 1]);
+        if (!sy.template reduce<NR + 2>(2, prr, mm2)) return;
+        invM = sh.bcast[NR] > 0.0 ? (float)(1.0 / sh.bcast[NR]) : 0.0f;
+        dyn = dyn_of(sh.bcast[NR], sh.bcast[NR + 1]);
         k++;
         last_true = 0;
         bool want_repl = P.replace_every > 0 && (k % P.replace_every) == 0;
 #pragma unroll
         for (int j = 0; j < NR; j++)
-            if (sh.active[j] && !P.fixed_iters && v[j] <= sh.thr2[j]) want_repl = true;
-        double rnew[NR], rrec[NR];
-#pragma unroll
-        for (int j = 0; j < NR; j++) rnew[j] = rrec[j] = v[j];
+            if (sh.active[j] && !P.fixed_iters && sh.bcast[j] <= sh.thr2[j]) want_repl = true;
+        // thread j: column j's recursive r.r, and its true one when that is formed
+        const double rrec = threadIdx.x < NR ? sh.bcast[threadIdx.x] : 0.0;
+        double rnew = rrec;
         if (want_repl) {
             // ---- FP64 R = B - A X, R's shadow, true residual norms ----
             double prt[NR + 2];
@@ -486,29 +485,29 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
             }
             prt[NR] = st.mx;
             prt[NR + 1] = -st.mn;
-            if (!sy.template reduce<NR + 2>(5, prt, mm2, v)) return;
-            invM = v[NR] > 0.0 ? (float)(1.0 / v[NR]) : 0.0f;
-            dyn = dyn_of(v[NR], v[NR + 1]);
+            if (!sy.template reduce<NR + 2>(5, prt, mm2)) return;
+            invM = sh.bcast[NR] > 0.0 ? (float)(1.0 / sh.bcast[NR]) : 0.0f;
+            dyn = dyn_of(sh.bcast[NR], sh.bcast[NR + 1]);
             repl++;
             last_true = 1;
-#pragma unroll
-            for (int j = 0; j < NR; j++) {
-                rt[j] = v[j];
-                rnew[j] = v[j];
+            if (threadIdx.x < NR) {
+                rnew = sh.bcast[threadIdx.x];
+                sh.rt[threadIdx.x] = rnew;
             }
+        } else {
+            __syncthreads();              // every thread has read `active` before column threads change it
         }
-        if (threadIdx.x == 0) {
-            for (int j = 0; j < NR; j++) {
-                if (sh.active[j] && last_true && !P.fixed_iters && rnew[j] <= sh.thr2[j]) {
-                    sh.active[j] = 0;            // converged on the FP64 true residual
-                    sh.conv[j] = 1;
-                    sh.iters[j] = k;
-                }
-                const bool restart = last_true &&
-                                     restart_after_replacement(!P.fixed_iters && rrec[j] <= sh.thr2[j], rnew[j], rrec[j]);
-                sh.beta[j] = (sh.active[j] && !restart) ? rnew[j] / sh.rr[j] : 0.0;
-                if (sh.active[j] || !sh.conv[j]) sh.rr[j] = rnew[j];
+        if (threadIdx.x < NR) {
+            const int j = threadIdx.x;
+            if (sh.active[j] && last_true && !P.fixed_iters && rnew <= sh.thr2[j]) {
+                sh.active[j] = 0;            // converged on the FP64 true residual
+                sh.conv[j] = 1;
+                sh.iters[j] = k;
             }
+            const bool restart = last_true &&
+                                 restart_after_replacement(!P.fixed_iters && rrec <= sh.thr2[j], rnew, rrec);
+            sh.beta[j] = (sh.active[j] && !restart) ? rnew / sh.rr[j] : 0.0;
+            if (sh.active[j] || !sh.conv[j]) sh.rr[j] = rnew;
         }
         __syncthreads();
     }
@@ -534,17 +533,16 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
             for (int R = c.rbeg; R < c.rend; R++)
                 if (P.seg_ptr[R] == P.seg_ptr[R + 1]) acc_r(R, zy);
         }
-        double w[NR];
-        if (!sy.template reduce<NR>(7, prt, 0u, w)) return;
-#pragma unroll
-        for (int j = 0; j < NR; j++) rt[j] = w[j];
+        if (!sy.template reduce<NR>(7, prt, 0u)) return;
+        if (threadIdx.x < NR) sh.rt[threadIdx.x] = sh.bcast[threadIdx.x];
+        __syncthreads();
     }
     if (sy.writer()) {
         for (int j = 0; j < NR; j++) {
             const double bb = sh.bb[j];
             M.out[4 * j + 0] = (double)(sh.conv[j] ? sh.iters[j] : k);
             M.out[4 * j + 1] = (double)sh.conv[j];
-            M.out[4 * j + 2] = bb > 0 ? sqrt(rt[j] / bb) : 0.0;
+            M.out[4 * j + 2] = bb > 0 ? sqrt(sh.rt[j] / bb) : 0.0;
             M.out[4 * j + 3] = bb > 0 ? sqrt(sh.rr[j] / bb) : 0.0;
         }
         M.out[4 * NR + 0] = (double)k;
@@ -560,11 +558,11 @@ struct GridSync {
     SharedM &sh;
     unsigned epoch;
     template <int NV>
-    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask, double (&out)[NV])
+    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask)
     {
         block_partial_m<NV>(M, sh, kind, v, maxmask, (int)gridDim.x, (int)blockIdx.x);
         if (!grid_barrier(P, epoch, sh)) return false;
-        grid_collect_m<NV>(M, sh, kind, maxmask, out, (int)gridDim.x);
+        grid_collect_m<NV>(M, sh, kind, maxmask, (int)gridDim.x);
         return true;
     }
     __device__ bool writer() const { return blockIdx.x == 0 && threadIdx.x == 0; }
@@ -623,6 +621,7 @@ struct BatchItem {
     int n, tilem, nr;             // nr: interleave width (1, 2, 4 or 8)
     int tilenum;
     int team;                     // blocks solving the item (1: queue item)
+    int nrhs, group;              // the system's right-hand sides, and which group of nr the item holds
     int nseg, vec_len;            // extents for the bounds-checked build
     long long n_payload;
 };
@@ -648,7 +647,7 @@ struct BatchParams {
 struct BlockSync {
     SharedM &sh;
     template <int NV>
-    __device__ bool reduce(int, const double (&v)[NV], unsigned maxmask, double (&out)[NV])
+    __device__ bool reduce(int, const double (&v)[NV], unsigned maxmask)
     {
         const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
 #pragma unroll
@@ -674,9 +673,6 @@ struct BlockSync {
             if (lane == 0) sh.bcast[wib] = a;
         }
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < NV; k++) out[k] = sh.bcast[k];
-        __syncthreads();
         return true;
     }
     __device__ bool writer() const { return threadIdx.x == 0; }
@@ -687,11 +683,12 @@ struct BlockSync {
 // by `limit_ns`; a timeout, or an error set elsewhere, returns false and the
 // first error is kept in *err.
 __device__ bool team_barrier(unsigned *ctr, unsigned k, unsigned &epoch, int *err, unsigned long long limit_ns,
-                             SharedM &sh, int stall = 0)
+                             unsigned long long first_limit_ns, SharedM &sh, int stall)
 {
     __syncthreads();
-    epoch += 1;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) {                // epoch: in shared memory, thread 0's alone
+        if (epoch == 0) limit_ns = first_limit_ns;
+        epoch += 1;
         const unsigned target = epoch * k + ((stall && epoch == 1) ? 1u : 0u);
         __threadfence();
         mf_red_relaxed_add_u32(ctr, 1u);
@@ -734,18 +731,14 @@ struct TeamSync {
     SharedM &sh;
     TeamShared &ts;
     template <int NV>
-    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask, double (&out)[NV])
+    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask)
     {
         MultiParams R;
         R.red = ts.red;
         block_partial_m<NV>(R, sh, kind, v, maxmask, ts.k, ts.r);
-        unsigned ep = ts.epoch;
-        const bool ok =
-            team_barrier(ts.ctr, (unsigned)ts.k, ep, ts.err, ep == 0 ? ts.arrive_ns : ts.limit_ns, sh, ts.stall);
-        if (!ok) return false;
-        grid_collect_m<NV>(R, sh, kind, maxmask, out, ts.k);
-        if (threadIdx.x == 0) ts.epoch = ep;
-        __syncthreads();
+        if (!team_barrier(ts.ctr, (unsigned)ts.k, ts.epoch, ts.err, ts.limit_ns, ts.arrive_ns, sh, ts.stall))
+            return false;
+        grid_collect_m<NV>(R, sh, kind, maxmask, ts.k);
         return true;
     }
     __device__ bool writer() const { return ts.r == 0 && threadIdx.x == 0; }
@@ -1078,7 +1071,6 @@ struct BatchImpl {
     size_t ctl_bytes = 0;
     char *d_pool = nullptr;
     size_t pool_bytes = 0;
-    std::vector<size_t> out_off;       // offset of each item's report words in the pool
     cudaStream_t own = nullptr;        // used when the caller passes the default stream
     cudaGraphExec_t graph = nullptr;
     std::vector<const void *> graph_key;
@@ -1206,18 +1198,15 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
         bptr.assign(B.grid + 1, 0);
     }
     B.nqueue = (int)queue.size();
-    // per item: B | X | R | P | Q (doubles), segment magnitudes,
-    // report words, team partials
+    // per item: B | X | R | P | Q (doubles), segment magnitudes, team partials
     std::vector<size_t> off(B.nitems), red_off(B.nitems, 0);
-    size_t total = 0;
-    B.out_off.assign(B.nitems, 0);
+    // the report words of all items first, so one copy reads them back
+    size_t total = align256((size_t)B.nitems * kOutWords * sizeof(double));
     for (int t = 0; t < B.nitems; t++) {
         const mf_matrix_s *A = B.sys[B.it_sys[t]];
         const size_t L = (size_t)A->vec_len, nr = (size_t)B.it_nr[t];
         off[t] = total;
         total += align256(5 * L * nr * sizeof(double)) + align256((size_t)(A->tilem + 1) * sizeof(float));
-        B.out_off[t] = total;
-        total += align256(kOutWords * sizeof(double));
         if (B.it_team[t] > 1) {
             red_off[t] = total;
             total += align256((size_t)kRedKinds * B.it_team[t] * kRedWidthM * sizeof(double));
@@ -1242,6 +1231,7 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
         it.seg_rowlen = A->d_seg_rowlen; it.meta = A->d_meta; it.v64 = A->d_v64; it.v32 = A->d_v32;
         it.v16 = A->d_v16; it.v8 = A->d_v8; it.i8_scale = A->d_i8_scale; it.row_cost = A->d_row_cost;
         it.n = A->n_rows; it.tilem = A->tilem; it.nr = (int)nr; it.team = B.it_team[t];
+        it.nrhs = B.nrhs[B.it_sys[t]]; it.group = B.it_col0[t] / it.nr;
         it.n_exact = A->n_exact; it.tilenum = A->tilenum;
         it.nseg = A->nseg; it.vec_len = A->vec_len; it.n_payload = A->slice_entries;
         char *base = B.d_pool + off[t];
@@ -1249,7 +1239,7 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
         it.M.B = v; it.M.X = v + L * nr; it.M.R = v + 2 * L * nr; it.M.Pv = v + 3 * L * nr; it.M.Q = v + 4 * L * nr;
         it.M.mag = (float *)(base + align256(5 * L * nr * sizeof(double)));
         it.M.red = it.team > 1 ? (double *)(B.d_pool + red_off[t]) : nullptr;
-        it.M.out = (double *)(B.d_pool + B.out_off[t]);
+        it.M.out = (double *)B.d_pool + (size_t)t * kOutWords;
         it.M.nr = B.it_ncol[t];
         it.ctr = it.team > 1 ? B.d_ctl + 2 + ctr_of[t] : nullptr;
     }
@@ -1269,22 +1259,56 @@ int batch_build_items(BatchImpl &B, int cap, int lb, cudaStream_t s)
     return MF_SUCCESS;
 }
 
+// Every item's columns between the caller's arrays (one column after another)
+// and the interleaved vectors: up to kMoveItems items per launch (blockIdx.y),
+// their arrays passed as arguments.  (A launch per item and direction, and a
+// read-back per item, took 1.5 of the 7.9 ms of a 40-system solve.)
+constexpr int kMoveItems = 64;
+enum { kMoveB = 0, kMoveX0 = 1, kMoveX = 2 };       // B in, X in, X out
+struct MoveArgs {
+    double *p[kMoveItems];
+    int first, what;
+};
+
+__global__ void k_batch_move(const BatchItem *items, MoveArgs a)
+{
+    const BatchItem &it = items[a.first + blockIdx.y];
+    double *flat = a.p[blockIdx.y];
+    const int NR = it.nr, sh = __ffs(NR) - 1, n = it.n;
+    double *mix = a.what == kMoveB ? const_cast<double *>(it.M.B) : it.M.X;
+    const long long end = (long long)(a.what == kMoveX ? n : it.vec_len) * NR;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < end;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int row = (int)(t >> sh), col = it.group * NR + (int)(t & (NR - 1));
+        const bool real = row < n && col < it.nrhs;
+        if (a.what != kMoveX) mix[t] = real ? flat[(long long)col * n + row] : 0.0;
+        else if (real) flat[(long long)col * n + row] = mix[t];
+    }
+}
+
+int batch_move(BatchImpl &B, const double *const *arrays, int what, cudaStream_t s)
+{
+    for (int t0 = 0; t0 < B.nitems; t0 += kMoveItems) {
+        MoveArgs a;
+        memset(&a, 0, sizeof(a));
+        a.first = t0;
+        a.what = what;
+        const int count = std::min(kMoveItems, B.nitems - t0);
+        for (int k = 0; k < count; k++) a.p[k] = const_cast<double *>(arrays[B.it_sys[t0 + k]]);
+        k_batch_move<<<dim3(64, count), 256, 0, s>>>(B.d_items, a);
+        MF_CUDA_TRY(cudaGetLastError());
+    }
+    return MF_SUCCESS;
+}
+
 // Enqueue one batched solve on s: interleave every item's columns, reset the
 // queue head, error word and team counters, the cooperative persistent launch,
 // de-interleave.  No host synchronisation.
 int batch_enqueue(BatchImpl &B, const double *const *Bd, double *const *Xd, const BatchParams &bp0, int mode,
                   cudaStream_t s)
 {
-    for (int t = 0; t < B.nitems; t++) {
-        const mf_matrix_s *A = B.sys[B.it_sys[t]];
-        const int nr = B.it_nr[t], g = B.it_col0[t] / nr;
-        k_interleave<<<148, 256, 0, s>>>(Bd[B.it_sys[t]], A->n_rows, A->vec_len, B.nrhs[B.it_sys[t]], g, nr,
-                                          (double *)B.h_items[t].M.B);
-        if (bp0.x0_given)          // the initial guesses: R = B - A X is formed in the launch
-            k_interleave<<<148, 256, 0, s>>>(Xd[B.it_sys[t]], A->n_rows, A->vec_len, B.nrhs[B.it_sys[t]], g, nr,
-                                              B.h_items[t].M.X);
-    }
-    MF_CUDA_TRY(cudaGetLastError());
+    MF_TRY(batch_move(B, Bd, kMoveB, s));
+    if (bp0.x0_given) MF_TRY(batch_move(B, Xd, kMoveX0, s));     // the initial guesses: R = B - A X is formed in the launch
     MF_CUDA_TRY(cudaMemsetAsync(B.d_ctl, 0, B.ctl_bytes, s));
     BatchParams bp = bp0;
     bp.items = B.d_items;
@@ -1312,13 +1336,7 @@ int batch_enqueue(BatchImpl &B, const double *const *Bd, double *const *Xd, cons
         if (mode == MODE_FP64) MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_batch<MODE_FP64, 1>, bp));
         else MF_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_batch<MODE_MIXED, 1>, bp));
     }
-    for (int t = 0; t < B.nitems; t++) {
-        const mf_matrix_s *A = B.sys[B.it_sys[t]];
-        const int nr = B.it_nr[t], g = B.it_col0[t] / nr;
-        k_deinterleave<<<148, 256, 0, s>>>(B.h_items[t].M.X, A->n_rows, B.nrhs[B.it_sys[t]], g, nr,
-                                            Xd[B.it_sys[t]]);
-    }
-    MF_CUDA_TRY(cudaGetLastError());
+    MF_TRY(batch_move(B, Xd, kMoveX, s));
     return MF_SUCCESS;
 }
 
@@ -1484,9 +1502,7 @@ int mf_batch_solve_impl(mf_batch_s *b, const double *const *Bd, double *const *X
         MF_CUDA_TRY(cudaEventRecord(B.e1, run));
     }
     std::vector<double> outs((size_t)B.nitems * kOutWords);
-    for (int t = 0; t < B.nitems; t++)
-        MF_CUDA_TRY(cudaMemcpyAsync(outs.data() + (size_t)t * kOutWords, B.d_pool + B.out_off[t],
-                                    kOutWords * sizeof(double), cudaMemcpyDeviceToHost, run));
+    MF_CUDA_TRY(cudaMemcpyAsync(outs.data(), B.d_pool, outs.size() * sizeof(double), cudaMemcpyDeviceToHost, run));
     int team_err = 0;
     MF_CUDA_TRY(cudaMemcpyAsync(&team_err, B.d_ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, run));
     MF_CUDA_TRY(cudaStreamSynchronize(run));
