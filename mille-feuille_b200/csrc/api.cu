@@ -93,14 +93,6 @@ void mf_free_host(void *p) { free(p); }
 // ------------------------------------------------------------------ matrices
 namespace {
 
-__global__ void k_check_rowptr(const int *rowptr, int n, long long nnz, int *err)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int a = rowptr[i], b = rowptr[i + 1];
-        if (a < 0 || b < a || (long long)b > nnz) atomicExch(err, MF_ERR_INVALID);
-    }
-}
-
 // Work on any stream may still use the handle's arrays, so the device is
 // synchronised first (as cudaFree does); the frees themselves are then
 // stream-ordered on an idle device.
@@ -186,17 +178,7 @@ extern "C" int mf_matrix_create(mf_matrix *out, int n_rows, int n_cols, long lon
         (val_low && nnz > 0 &&
          cudaMemcpyAsync(A->d_val_low, val_low, (size_t)nnz * sizeof(float), kind, s) != cudaSuccess))
         return fail(MF_ERR_CUDA);
-    int *d_err = nullptr;
-    if ((rc = mf_pool_array(&d_err, 1, s)) != MF_SUCCESS) return fail(rc);
-    cudaMemsetAsync(d_err, 0, sizeof(int), s);
-    if (n_rows > 0) k_check_rowptr<<<(n_rows + 255) / 256, 256, 0, s>>>(A->d_rowptr, n_rows, nnz, d_err);
-    int h_err = 0;
-    cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    const cudaError_t se = cudaStreamSynchronize(s);
-    mf_pool_free(d_err, s);
-    if (se != cudaSuccess) return fail(MF_ERR_CUDA);
-    if (h_err) return fail(h_err);
-    rc = mf_build_tiles(A, s);
+    rc = mf_build_tiles(A, nnz, s);
     if (rc != MF_SUCCESS) return fail(rc);
     *out = A;
     return MF_SUCCESS;

@@ -154,9 +154,12 @@ struct MfDeviceGuard {
 int mf_scan_i32_to_i32(const int *d_in, int *d_out, long long n, cudaStream_t s);   // out[0..n]
 int mf_scan_i32_to_i64(const int *d_in, long long *d_out, long long n, cudaStream_t s);
 int mf_scan_i64_to_i64(const long long *d_in, long long *d_out, long long n, cudaStream_t s);
+// tiles per tile-row -> tile_ptr, row-block offsets and seg_ptr in one pass
+int mf_scan_tile_counts(const int *d_ntiles, int *d_tile_ptr, int *d_rb_ptr, int *d_seg_ptr, long long n,
+                        cudaStream_t s);
 
-// tile build (tile_build.cu)
-int mf_build_tiles(mf_matrix_s *A, cudaStream_t s);
+// tile build (tile_build.cu); nnz: entries of the caller's arrays
+int mf_build_tiles(mf_matrix_s *A, long long nnz, cudaStream_t s);
 
 // solver (solver.cu)
 int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_options *opt,

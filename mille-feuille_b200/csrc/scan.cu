@@ -1,10 +1,11 @@
 // scan.cu -- device exclusive prefix sums used by the GPU tiler.
 // out[0..n] with out[0] = 0 and out[n] = total (the form of the reference's
-// exclusive_scan over length n+1, utils.h:34-49).  Three passes: per-block
-// scan with block totals, recursive scan of the totals, add-back.
+// exclusive_scan over length n+1, utils.h:34-49).  Two kernels: totals per block
+// of 4,096 elements, then every block adds up the totals before its own and scans
+// its elements (n = 16.8 M makes 4,096 totals, 8 loads a thread).  The tiler's
+// scans are short, so launches count: three levels with an add-back were 4 or 5
+// kernels and two allocations each, some 30 of the 75 launches of a build.
 #include "mf_internal.cuh"
-
-#include <vector>
 
 namespace {
 
@@ -12,117 +13,154 @@ constexpr int kThreads = 512;
 constexpr int kItems = 8;
 constexpr int kTile = kThreads * kItems;
 
-template <typename TI, typename TO>
-__global__ void k_block_scan(const TI *__restrict__ in, TO *__restrict__ out, TO *__restrict__ block_sums,
-                             long long n)
+// what one tile-row adds to the tile, row-block and slice counts
+struct Tile3 {
+    int tiles, blocks, slices;
+};
+__device__ __forceinline__ Tile3 operator+(Tile3 x, Tile3 y)
 {
-    __shared__ TO warp_tot[kThreads / 32];
-    const long long base = (long long)blockIdx.x * kTile + (long long)threadIdx.x * kItems;
-    TO v[kItems];
-    TO run = 0;
-#pragma unroll
-    for (int j = 0; j < kItems; j++) {
-        long long i = base + j;
-        TO x = (i < n) ? (TO)in[i] : (TO)0;
-        v[j] = run;
-        run += x;
+    return {x.tiles + y.tiles, x.blocks + y.blocks, x.slices + y.slices};
+}
+
+__device__ __forceinline__ int shfl_up(int v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ long long shfl_up(long long v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ Tile3 shfl_up(Tile3 v, int o)
+{
+    return {shfl_up(v.tiles, o), shfl_up(v.blocks, o), shfl_up(v.slices, o)};
+}
+
+template <typename TI, typename TO>
+struct PlainScan {
+    using Value = TO;
+    const TI *in;
+    TO *out;
+    __device__ Value load(long long i) const { return (TO)in[i]; }
+    __device__ void store(long long i, Value v) const { out[i] = v; }
+};
+
+// Row-block split of blockspmv_cpu (blockspmv_cpu.h:35-83, PREFETCH_SMEM_TH = 4)
+// and slices of up to MF_SEG_TILES tiles, from the tiles of a tile-row.
+struct TileScan {
+    using Value = Tile3;
+    const int *ntiles;
+    int *tile_ptr, *rb_ptr, *seg_ptr;
+    __device__ Value load(long long i) const
+    {
+        const int nt = ntiles[i];
+        return {nt, nt <= 4 ? 1 : (nt + 3) / 4, (nt + MF_SEG_TILES - 1) / MF_SEG_TILES};
     }
-    // exclusive scan of per-thread totals across the block
+    __device__ void store(long long i, Value v) const
+    {
+        tile_ptr[i] = v.tiles;
+        rb_ptr[i] = v.blocks;
+        seg_ptr[i] = v.slices;
+    }
+};
+
+// Exclusive scan of one value per thread over the block; *total: the block's sum.
+template <typename T>
+__device__ T block_scan(T mine, T *total)
+{
+    __shared__ T warp_tot[kThreads / 32], all;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    TO incl = run;
+    T incl = mine;
+    const T zero = T();
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        TO t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+        const T t = shfl_up(incl, o);
+        if (lane >= o) incl = incl + t;
     }
     if (lane == 31) warp_tot[wid] = incl;
+    T before = shfl_up(incl, 1);
+    if (lane == 0) before = zero;
     __syncthreads();
     if (wid == 0) {
-        TO w = (lane < kThreads / 32) ? warp_tot[lane] : (TO)0;
-        TO wi = w;
+        T wi = lane < kThreads / 32 ? warp_tot[lane] : zero;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            TO t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += t;
+            const T t = shfl_up(wi, o);
+            if (lane >= o) wi = wi + t;
         }
-        if (lane < kThreads / 32) warp_tot[lane] = wi - w;   // exclusive warp offsets
-        if (lane == kThreads / 32 - 1 && block_sums) block_sums[blockIdx.x] = wi;
+        T ex = shfl_up(wi, 1);
+        if (lane == 0) ex = zero;
+        if (lane < kThreads / 32) warp_tot[lane] = ex;
+        if (lane == kThreads / 32 - 1) all = wi;
     }
     __syncthreads();
-    TO off = warp_tot[wid] + incl - run;
+    *total = all;
+    const T r = warp_tot[wid] + before;
+    __syncthreads();
+    return r;
+}
+
+template <typename S>
+__global__ void k_block_sums(S s, typename S::Value *sums, long long n)
+{
+    using T = typename S::Value;
+    const long long base = (long long)blockIdx.x * kTile + (long long)threadIdx.x * kItems;
+    T run = T();
+#pragma unroll
+    for (int j = 0; j < kItems; j++)
+        if (base + j < n) run = run + s.load(base + j);
+    T total;
+    block_scan(run, &total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+template <typename S>
+__global__ void k_scan_out(S s, const typename S::Value *sums, long long n)
+{
+    using T = typename S::Value;
+    T part = T(), offset = T();
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += kThreads) part = part + sums[b];
+    if (blockIdx.x > 0) block_scan(part, &offset);
+    const long long base = (long long)blockIdx.x * kTile + (long long)threadIdx.x * kItems;
+    T v[kItems], run = T(), total;
 #pragma unroll
     for (int j = 0; j < kItems; j++) {
-        long long i = base + j;
-        if (i < n) out[i] = v[j] + off;
+        v[j] = run;
+        if (base + j < n) run = run + s.load(base + j);
     }
+    const T off = offset + block_scan(run, &total);
+#pragma unroll
+    for (int j = 0; j < kItems; j++)
+        if (base + j < n) s.store(base + j, off + v[j]);
+    if (blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) s.store(n, offset + total);
 }
 
-template <typename TO>
-__global__ void k_add_offsets(TO *out, const TO *block_off, long long n)
+template <typename S>
+int scan_impl(S sc, long long n, cudaStream_t s)
 {
-    const long long base = (long long)blockIdx.x * kTile;
-    const TO o = block_off[blockIdx.x];
-    for (int j = threadIdx.x; j < kTile; j += kThreads) {
-        long long i = base + j;
-        if (i < n) out[i] += o;
+    using T = typename S::Value;
+    const long long nb = n > 0 ? (n + kTile - 1) / kTile : 1;
+    T *sums = nullptr;
+    if (nb > 1) {
+        const int rc = mf_pool_array(&sums, nb, s);
+        if (rc != MF_SUCCESS) return rc;
+        k_block_sums<<<(unsigned)nb, kThreads, 0, s>>>(sc, sums, n);
     }
-}
-
-template <typename TO>
-__global__ void k_set_total(TO *out, long long n, const TO *block_sums_scanned, long long nb)
-{
-    // out[n] = total = scanned block offsets [nb]
-    out[n] = block_sums_scanned[nb];
-}
-
-template <typename TI, typename TO>
-int scan_impl(const TI *d_in, TO *d_out, long long n, cudaStream_t s)
-{
-    if (n <= 0) {
-        MF_CUDA_TRY(cudaMemsetAsync(d_out, 0, sizeof(TO), s));
-        return MF_SUCCESS;
-    }
-    long long nb = (n + kTile - 1) / kTile;
-    TO *sums = nullptr, *sums_scanned = nullptr;
-    int rc = mf_pool_array(&sums, nb + 1, s);
-    if (rc == MF_SUCCESS) rc = mf_pool_array(&sums_scanned, nb + 1, s);
-    if (rc != MF_SUCCESS) {
-        mf_pool_free(sums, s);
-        return rc;
-    }
-    k_block_scan<TI, TO><<<(unsigned)nb, kThreads, 0, s>>>(d_in, d_out, sums, n);
-    MF_CUDA_TRY(cudaGetLastError());
-    if (nb == 1) {
-        MF_CUDA_TRY(cudaMemsetAsync(sums_scanned, 0, sizeof(TO), s));
-        MF_CUDA_TRY(cudaMemcpyAsync(sums_scanned + 1, sums, sizeof(TO), cudaMemcpyDeviceToDevice, s));
-        rc = MF_SUCCESS;
-    } else {
-        rc = scan_impl<TO, TO>(sums, sums_scanned, nb, s);
-    }
-    if (rc == MF_SUCCESS) {
-        if (nb > 1) {
-            k_add_offsets<TO><<<(unsigned)nb, kThreads, 0, s>>>(d_out, sums_scanned, n);
-            MF_CUDA_TRY(cudaGetLastError());
-        }
-        k_set_total<TO><<<1, 1, 0, s>>>(d_out, n, sums_scanned, nb);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
+    k_scan_out<<<(unsigned)nb, kThreads, 0, s>>>(sc, sums, n);
     mf_pool_free(sums, s);
-    mf_pool_free(sums_scanned, s);
-    return rc;
+    MF_CUDA_TRY(cudaGetLastError());
+    return MF_SUCCESS;
 }
 
 }  // namespace
 
 int mf_scan_i32_to_i32(const int *d_in, int *d_out, long long n, cudaStream_t s)
 {
-    return scan_impl<int, int>(d_in, d_out, n, s);
+    return scan_impl(PlainScan<int, int>{d_in, d_out}, n, s);
 }
 int mf_scan_i32_to_i64(const int *d_in, long long *d_out, long long n, cudaStream_t s)
 {
-    return scan_impl<int, long long>(d_in, d_out, n, s);
+    return scan_impl(PlainScan<int, long long>{d_in, d_out}, n, s);
 }
 int mf_scan_i64_to_i64(const long long *d_in, long long *d_out, long long n, cudaStream_t s)
 {
-    return scan_impl<long long, long long>(d_in, d_out, n, s);
+    return scan_impl(PlainScan<long long, long long>{d_in, d_out}, n, s);
+}
+int mf_scan_tile_counts(const int *d_ntiles, int *d_tile_ptr, int *d_rb_ptr, int *d_seg_ptr, long long n,
+                        cudaStream_t s)
+{
+    return scan_impl(TileScan{d_ntiles, d_tile_ptr, d_rb_ptr, d_seg_ptr}, n, s);
 }

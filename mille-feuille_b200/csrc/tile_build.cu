@@ -11,6 +11,11 @@
 // so the tile order is ascending as in convert_step2 (csr2block.h:89-102).
 // Entries are then ranked inside their tile in CSR order with __match_any_sync
 // (the order convert_step4 appends them in, csr2block.h:204-219).
+//
+// The host waits four times: for the tile-rows' spans (which also check the row
+// pointers), for the tile counts, for the sizes that depend on the filled tiles,
+// and at the end.  With ten waits, a copy per number and up to five kernels a
+// scan, a 65,280-row build took 0.44 ms for 0.15 ms of kernels.
 #include "mf_internal.cuh"
 
 #include <algorithm>
@@ -28,107 +33,102 @@ __device__ __forceinline__ int tile_row_end(int R, int tilem, int rowA)
 }
 
 // ---- K0: column-tile span per tile-row, and the maxima the host needs ----
+// Also the check of the row pointers (in [0, nnz], not decreasing) and of the
+// columns: a tile-row's entries are read only when its row pointers are in order.
 __global__ void k_span(const int *__restrict__ rowptr, const int *__restrict__ colidx, int tilem, int rowA,
-                       int colA, int *__restrict__ span_base, int *__restrict__ maxes, int *__restrict__ err)
+                       int colA, long long nnz, int2 *__restrict__ spans, int *__restrict__ max_words,
+                       int *__restrict__ err)
 {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int R = warp; R < tilem; R += nwarps) {
-        const int a = rowptr[R * MF_BS], b = rowptr[tile_row_end(R, tilem, rowA)];
+        const int rows = tile_row_end(R, tilem, rowA) - R * MF_BS;
+        const int rp = lane <= rows ? rowptr[R * MF_BS + lane] : 0;
+        const int next = __shfl_down_sync(0xffffffffu, rp, 1);
+        bool bad = lane < rows && (rp < 0 || next < rp || (long long)next > nnz);
         int jmin = INT_MAX, jmax = -1;
-        bool bad = (b < a);
-        for (int j = a + lane; j < b; j += 32) {
-            int c = colidx[j];
-            if (c < 0 || c >= colA) { bad = true; continue; }
-            int jc = c >> 4;
-            jmin = min(jmin, jc);
-            jmax = max(jmax, jc);
+        if (!__any_sync(0xffffffffu, bad)) {
+            const int a = __shfl_sync(0xffffffffu, rp, 0), b = __shfl_sync(0xffffffffu, rp, rows);
+            for (int j = a + lane; j < b; j += 32) {
+                int c = colidx[j];
+                if (c < 0 || c >= colA) { bad = true; continue; }
+                int jc = c >> 4;
+                jmin = min(jmin, jc);
+                jmax = max(jmax, jc);
+            }
         }
-        for (int o = 16; o; o >>= 1) {
-            jmin = min(jmin, __shfl_xor_sync(0xffffffffu, jmin, o));
-            jmax = max(jmax, __shfl_xor_sync(0xffffffffu, jmax, o));
-        }
+        jmin = __reduce_min_sync(0xffffffffu, jmin);
+        jmax = __reduce_max_sync(0xffffffffu, jmax);
         bad = __any_sync(0xffffffffu, bad);
         if (lane == 0) {
             if (bad) atomicExch(err, MF_ERR_INVALID);
-            int words = (jmax < 0) ? 0 : (jmax >> 5) - (jmin >> 5) + 1;
-            span_base[R] = (jmax < 0) ? 0 : (jmin >> 5);
-            atomicMax(&maxes[0], words);
-            atomicMax(&maxes[1], b - a);
+            const int words = (jmax < 0) ? 0 : (jmax >> 5) - (jmin >> 5) + 1;
+            spans[R] = make_int2((jmax < 0) ? 0 : (jmin >> 5), words);     // first word, words
+            if (words > *(volatile int *)max_words) atomicMax(max_words, words);
         }
     }
 }
 
-// scratch layout per warp (32-bit words): bitmap[span], prefix[span], cnt[max_tiles]
-struct Scratch {
-    unsigned int *bm;
-    int *pre;
-    int *cnt;
-};
-
-__device__ __forceinline__ Scratch warp_scratch(unsigned int *smem, unsigned int *gscratch, int words_per_warp,
-                                                int span, int global_mode)
+// A warp's scratch, in shared memory or (wide spans, many tiles) in global memory.
+__device__ __forceinline__ unsigned int *warp_scratch(unsigned int *smem, unsigned int *gscratch, int words_per_warp,
+                                                      int global_mode)
 {
     const int wib = threadIdx.x >> 5;
     const long long gw = (long long)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    unsigned int *base = global_mode ? gscratch + gw * (long long)words_per_warp : smem + (long long)wib * words_per_warp;
-    Scratch s;
-    s.bm = base;
-    s.pre = (int *)(base + span);
-    s.cnt = (int *)(base + 2 * span);
-    return s;
+    return global_mode ? gscratch + gw * (long long)words_per_warp : smem + (long long)wib * words_per_warp;
 }
 
 // Build the tile-row bitmap; returns the number of distinct tiles.
-__device__ int build_bitmap(const Scratch &S, const int *__restrict__ colidx, int a, int b, int base_word,
+__device__ int build_bitmap(unsigned int *bm, const int *__restrict__ colidx, int a, int b, int base_word,
                             int words, int lane)
 {
-    for (int w = lane; w < words; w += 32) S.bm[w] = 0u;
+    for (int w = lane; w < words; w += 32) bm[w] = 0u;
     __syncwarp();
     for (int j = a + lane; j < b; j += 32) {
         int jc = colidx[j] >> 4;
-        atomicOr(&S.bm[(jc >> 5) - base_word], 1u << (jc & 31));
+        atomicOr(&bm[(jc >> 5) - base_word], 1u << (jc & 31));
     }
     __syncwarp();
     int cnt = 0;
-    for (int w = lane; w < words; w += 32) cnt += __popc(S.bm[w]);
+    for (int w = lane; w < words; w += 32) cnt += __popc(bm[w]);
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     return cnt;
 }
 
-// ---- K1: distinct tiles per tile-row ----
+// ---- K1: distinct tiles per tile-row, and the most of any ----
 __global__ void k_count_tiles(const int *__restrict__ rowptr, const int *__restrict__ colidx, int tilem, int rowA,
-                              const int *__restrict__ span_base, int span, int words_per_warp, int global_mode,
-                              unsigned int *gscratch, int *__restrict__ ntiles)
+                              const int2 *__restrict__ spans, int words_per_warp, int global_mode,
+                              unsigned int *gscratch, int *__restrict__ ntiles, int *__restrict__ max_tiles)
 {
     extern __shared__ unsigned int smem[];
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    Scratch S = warp_scratch(smem, gscratch, words_per_warp, span, global_mode);
+    unsigned int *bm = warp_scratch(smem, gscratch, words_per_warp, global_mode);
     for (int R = warp; R < tilem; R += nwarps) {
         const int a = rowptr[R * MF_BS], b = rowptr[tile_row_end(R, tilem, rowA)];
-        const int base_word = span_base[R];
-        int words = 0;
-        if (b > a) {
-            int jmax_word = base_word;   // recompute the span of this tile-row
-            int jm = -1;
-            for (int j = a + lane; j < b; j += 32) jm = max(jm, colidx[j] >> 4);
-            for (int o = 16; o; o >>= 1) jm = max(jm, __shfl_xor_sync(0xffffffffu, jm, o));
-            jmax_word = jm >> 5;
-            words = jmax_word - base_word + 1;
+        const int2 sp = spans[R];
+        const int c = (sp.y > 0) ? build_bitmap(bm, colidx, a, b, sp.x, sp.y, lane) : 0;
+        if (lane == 0) {
+            ntiles[R] = c;
+            if (c > *(volatile int *)max_tiles) atomicMax(max_tiles, c);
         }
-        int c = (words > 0) ? build_bitmap(S, colidx, a, b, base_word, words, lane) : 0;
-        if (lane == 0) ntiles[R] = c;
         __syncwarp();
     }
 }
 
 // ---- K2: tile columns, payload offsets, scatter, uint8 row starts ----
+// Scratch per warp: bitmap[span], prefix[span], next payload position[max_tiles],
+// entries per (tile, row)[16 max_tiles].  Entries are taken 32 at a time across
+// the rows of the tile-row (CSR order is row by row already): 7-point tile-rows
+// are 4 steps a pass, where going row by row made 16 with two warp barriers each
+// (128^3: 0.84 ms of 2 ms of kernels).  The row starts come from the (tile, row)
+// counts.  max_tiles is counted, not bounded by the span: irregular matrices with
+// wide spans stay in shared memory.
 __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restrict__ colidx,
                              const double *__restrict__ val, const float *__restrict__ val_low, int tilem,
-                             int rowA, const int *__restrict__ span_base, int span, int words_per_warp,
+                             int rowA, const int2 *__restrict__ spans, int span, int max_tiles, int words_per_warp,
                              int global_mode, unsigned int *gscratch, const int *__restrict__ tile_ptr,
                              int *__restrict__ tile_columnidx, int *__restrict__ csr_offset,
                              int *__restrict__ csrptr_offset, double *__restrict__ tval,
@@ -140,12 +140,14 @@ __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restri
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
-    Scratch S = warp_scratch(smem, gscratch, words_per_warp, span, global_mode);
+    unsigned int *bm = warp_scratch(smem, gscratch, words_per_warp, global_mode);
+    int *pre = (int *)bm + span, *next = pre + span, *hist = next + max_tiles;
     const int nz0 = rowptr[0];
     for (int R = warp; R < tilem; R += nwarps) {
         const int rs = R * MF_BS, re = tile_row_end(R, tilem, rowA);
         const int rowlen = re - rs;
-        const int a = rowptr[rs], b = rowptr[re];
+        const int rp = lane <= rowlen ? rowptr[rs + lane] : INT_MAX;
+        const int a = __shfl_sync(0xffffffffu, rp, 0), b = __shfl_sync(0xffffffffu, rp, rowlen);
         const int t0 = tile_ptr[R], nt = tile_ptr[R + 1] - t0;
         // csrptr_offset: exclusive scan of tile-row heights over tiles (csr2block.h:146,347)
         for (int s = lane; s < nt; s += 32) csrptr_offset[t0 + s] = t0 * MF_BS + s * rowlen;
@@ -154,30 +156,27 @@ __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restri
             if (R == tilem - 1 && lane == 0) csr_offset[t0] = b - nz0;
             continue;
         }
-        const int base_word = span_base[R];
-        int jm = -1;
-        for (int j = a + lane; j < b; j += 32) jm = max(jm, colidx[j] >> 4);
-        for (int o = 16; o; o >>= 1) jm = max(jm, __shfl_xor_sync(0xffffffffu, jm, o));
-        const int words = (jm >> 5) - base_word + 1;
-        build_bitmap(S, colidx, a, b, base_word, words, lane);
+        const int base_word = spans[R].x, words = spans[R].y;
+        for (int h = lane; h < nt * MF_BS; h += 32) hist[h] = 0;
+        build_bitmap(bm, colidx, a, b, base_word, words, lane);
         // exclusive popcount prefix over the bitmap words
         int carry = 0;
         for (int w0 = 0; w0 < words; w0 += 32) {
             int w = w0 + lane;
-            int c = (w < words) ? __popc(S.bm[w]) : 0;
+            int c = (w < words) ? __popc(bm[w]) : 0;
             int incl = c;
             for (int o = 1; o < 32; o <<= 1) {
                 int t = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += t;
             }
-            if (w < words) S.pre[w] = carry + incl - c;
+            if (w < words) pre[w] = carry + incl - c;
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
         __syncwarp();
         // tile_columnidx, ascending
         for (int w = lane; w < words; w += 32) {
-            unsigned int m = S.bm[w];
-            int r = S.pre[w];
+            unsigned int m = bm[w];
+            int r = pre[w];
             while (m) {
                 int bit = __ffs(m) - 1;
                 m &= m - 1u;
@@ -185,21 +184,30 @@ __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restri
                 r++;
             }
         }
-        // pass 1: entries per tile
-        for (int s = lane; s < nt; s += 32) S.cnt[s] = 0;
-        __syncwarp();
-        for (int j = a + lane; j < b; j += 32) {
-            int jc = colidx[j] >> 4;
-            int w = (jc >> 5) - base_word, bit = jc & 31;
-            int slot = S.pre[w] + __popc(S.bm[w] & ((1u << bit) - 1u));
-            atomicAdd(&S.cnt[slot], 1);
+        auto slot_of = [&](int c) -> int {
+            const int jc = c >> 4, w = (jc >> 5) - base_word;
+            return pre[w] + __popc(bm[w] & ((1u << (jc & 31)) - 1u));
+        };
+        // pass 1: entries per tile and row
+        for (int j0 = a; j0 < b; j0 += 32) {
+            const int j = j0 + lane;
+            int ri = 0;
+            for (int q = 1; q < rowlen; q++) ri += (j >= __shfl_sync(0xffffffffu, rp, q)) ? 1 : 0;
+            if (j < b) atomicAdd(&hist[slot_of(colidx[j]) * MF_BS + ri], 1);
         }
         __syncwarp();
-        // payload offsets: tile-row payload starts at rowptr[rs] (csr_offset scan)
+        // row starts and payload offsets: tile-row payload starts at rowptr[rs] (csr_offset scan)
         int run = a - nz0;
         for (int s0 = 0; s0 < nt; s0 += 32) {
-            int s = s0 + lane;
-            int c = (s < nt) ? S.cnt[s] : 0;
+            const int s = s0 + lane;
+            int c = 0;
+            if (s < nt)
+                for (int ri = 0; ri < rowlen; ri++) {
+                    if (c > 255) atomicExch(err, MF_ERR_UNSUPPORTED);
+                    // csrptr_offset[t0 + s] = t0 * 16 + s * rowlen (only the last tile-row is short)
+                    tptr[(long long)t0 * MF_BS + (long long)s * rowlen + ri] = (unsigned char)c;
+                    c += hist[s * MF_BS + ri];
+                }
             int incl = c;
             for (int o = 1; o < 32; o <<= 1) {
                 int t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -207,48 +215,33 @@ __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restri
             }
             if (s < nt) {
                 csr_offset[t0 + s] = run + incl - c;
+                next[s] = run + incl - c;
                 if (c > 256) atomicExch(err, MF_ERR_UNSUPPORTED);   // duplicate columns overflow a tile
             }
             run += __shfl_sync(0xffffffffu, incl, 31);
         }
         if (R == tilem - 1 && lane == 0) csr_offset[t0 + nt] = run;
         __syncwarp();
-        for (int s = lane; s < nt; s += 32) S.cnt[s] = 0;
-        __syncwarp();
-        // pass 2: row by row in CSR order
-        for (int ri = 0; ri < rowlen; ri++) {
-            for (int s = lane; s < nt; s += 32) {
-                int c = S.cnt[s];
-                if (c > 255) atomicExch(err, MF_ERR_UNSUPPORTED);
-                // csrptr_offset[t0 + s] = t0 * 16 + s * rowlen (only the last tile-row is short)
-                tptr[(long long)t0 * MF_BS + (long long)s * rowlen + ri] = (unsigned char)c;
+        // pass 2: the payload, in CSR order within a tile
+        for (int j0 = a; j0 < b; j0 += 32) {
+            const int j = j0 + lane;
+            const bool act = j < b;
+            int slot = -1, c = 0;
+            if (act) {
+                c = colidx[j];
+                slot = slot_of(c);
             }
+            const unsigned grp = __match_any_sync(0xffffffffu, slot);
+            const int rank = __popc(grp & lt_mask);
+            const int o = act ? next[slot] + rank : 0;
             __syncwarp();
-            const int ja = rowptr[rs + ri], jb = rowptr[rs + ri + 1];
-            for (int j0 = ja; j0 < jb; j0 += 32) {
-                int j = j0 + lane;
-                bool act = j < jb;
-                unsigned amask = __ballot_sync(0xffffffffu, act);
-                int slot = 0, c = 0;
-                if (act) {
-                    c = colidx[j];
-                    int jc = c >> 4;
-                    int w = (jc >> 5) - base_word, bit = jc & 31;
-                    slot = S.pre[w] + __popc(S.bm[w] & ((1u << bit) - 1u));
-                }
-                unsigned grp = __match_any_sync(0xffffffffu, act ? slot : -1);
-                if (act) {
-                    int rank = __popc(grp & lt_mask);
-                    int pos = S.cnt[slot] + rank;
-                    int o = csr_offset[t0 + slot] + pos;
-                    tval[o] = val[j];
-                    tval_low[o] = val_low ? val_low[j] : (float)val[j];
-                    tcol[o] = (unsigned char)(c & 15);
-                }
-                __syncwarp();
-                if (act && (grp & lt_mask) == 0) S.cnt[slot] += __popc(grp);
-                __syncwarp();
-                (void)amask;
+            if (act && rank == 0) next[slot] += __popc(grp);
+            __syncwarp();
+            if (act) {
+                const double v = val[j];
+                tval[o] = v;
+                tval_low[o] = val_low ? val_low[j] : (float)v;
+                tcol[o] = (unsigned char)(c & 15);
             }
         }
         __syncwarp();
@@ -322,14 +315,6 @@ __global__ void k_rowlist_fill(const int *__restrict__ tile_ptr, const int *__re
 }
 
 // ---- row-block split of blockspmv_cpu (blockspmv_cpu.h:35-83), PREFETCH_SMEM_TH = 4 ----
-__global__ void k_rowblk_count(const int *__restrict__ tile_ptr, int tilem, int *__restrict__ cnt)
-{
-    int R = blockIdx.x * blockDim.x + threadIdx.x;
-    if (R >= tilem) return;
-    int nb = tile_ptr[R + 1] - tile_ptr[R];
-    cnt[R] = (nb <= 4) ? 1 : (nb + 3) / 4;
-}
-
 __global__ void k_rowblk_fill(const int *__restrict__ tile_ptr, int tilem, const int *__restrict__ off,
                               unsigned int *__restrict__ idx, int *__restrict__ cs, int *__restrict__ ce)
 {
@@ -409,14 +394,6 @@ __global__ void k_encode_tiles(const int *__restrict__ csr_offset, int tilenum, 
 }
 
 // ---- solver slices ----
-__global__ void k_seg_count(const int *__restrict__ tile_ptr, int tilem, int *__restrict__ nseg)
-{
-    int R = blockIdx.x * blockDim.x + threadIdx.x;
-    if (R >= tilem) return;
-    int nt = tile_ptr[R + 1] - tile_ptr[R];
-    nseg[R] = (nt + MF_SEG_TILES - 1) / MF_SEG_TILES;
-}
-
 // lane-per-row statistics of every segment: row lengths and padded width
 __global__ void k_seg_shape(const int *__restrict__ tile_ptr, const int *__restrict__ seg_ptr,
                             const int *__restrict__ csr_offset, const int *__restrict__ csrptr_offset,
@@ -583,7 +560,45 @@ struct Temps {
         if (_rc != MF_SUCCESS) return _rc;  \
     } while (0)
 
-int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
+namespace {
+
+// The numbers the host waits for, gathered on the device and read in one copy.
+struct Counts {
+    int err, span, max_tiles;                       // written by the kernels as they go
+    int longest, not_one_chunk;                     // k_seg_shape
+    int tilenum, last_tile0, rowblocks, nseg, nz_lo, nz_hi;
+    int nonempty;
+    long long entries;
+};
+
+__global__ void k_counts_tiles(Counts *c, const int *tile_ptr, const int *rb_ptr, const int *seg_ptr,
+                               const int *rowptr, int tilem, int rowA)
+{
+    c->tilenum = tile_ptr[tilem];
+    c->last_tile0 = tilem > 0 ? tile_ptr[tilem - 1] : 0;
+    c->rowblocks = rb_ptr[tilem];
+    c->nseg = seg_ptr[tilem];
+    c->nz_lo = rowptr[0];
+    c->nz_hi = rowptr[rowA];
+}
+
+__global__ void k_counts_filled(Counts *c, const int *nonzero_row, int tilenum, const long long *seg_off, int nseg)
+{
+    c->nonempty = nonzero_row[tilenum];
+    c->entries = seg_off[nseg];
+}
+
+int read_counts(Counts *h, const Counts *d, cudaStream_t s)
+{
+    MF_CUDA_TRY(cudaGetLastError());
+    MF_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(*h), cudaMemcpyDeviceToHost, s));
+    MF_CUDA_TRY(cudaStreamSynchronize(s));
+    return h->err;
+}
+
+}  // namespace
+
+int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
 {
     auto t_start = std::chrono::steady_clock::now();
     const int rowA = A->n_rows, colA = A->n_cols;
@@ -593,141 +608,120 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
     A->tilen = tilen;
     A->vec_len = std::max(tilem, tilen) * MF_BS;
     Temps tmp{s, {}};
-    int *d_err = nullptr, *d_maxes = nullptr, *d_span_base = nullptr, *d_ntiles = nullptr;
-    MF_TRY(tmp.get(&d_err, 1));
-    MF_TRY(tmp.get(&d_maxes, 2));
-    MF_TRY(tmp.get(&d_span_base, tilem));
-    MF_TRY(tmp.get(&d_ntiles, tilem + 1));
-    MF_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
-    MF_CUDA_TRY(cudaMemsetAsync(d_maxes, 0, 2 * sizeof(int), s));
-    MF_CUDA_TRY(cudaMemsetAsync(d_ntiles, 0, (tilem + 1) * sizeof(int), s));
+    Counts *d_c = nullptr, c;
+    int2 *d_spans = nullptr;
+    int *d_ntiles = nullptr, *d_rbo = nullptr;
+    MF_TRY(tmp.get(&d_c, 1));
+    MF_TRY(tmp.get(&d_spans, tilem));
+    MF_TRY(tmp.get(&d_ntiles, tilem));
+    MF_TRY(tmp.get(&d_rbo, (long long)tilem + 1));
+    MF_TRY(dalloc(&A->d_tile_ptr, (long long)tilem + 1, s));
+    MF_TRY(dalloc(&A->d_seg_ptr, (long long)tilem + 1, s));
+    MF_CUDA_TRY(cudaMemsetAsync(d_c, 0, sizeof(Counts), s));
     const int wgrid = grid_for((long long)tilem * 32, kThreads);
-    if (tilem > 0) {
-        k_span<<<wgrid, kThreads, 0, s>>>(A->d_rowptr, A->d_colidx, tilem, rowA, colA, d_span_base, d_maxes, d_err);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    int h_maxes[2] = {0, 0}, h_err = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(h_maxes, d_maxes, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    if (h_err) return h_err;
-    const int span = std::max(h_maxes[0], 1);
-    // scratch per warp: bitmap + prefix (span words each) + tile counters (<= 32 * span)
-    long long words_per_warp = 2LL * span + 32LL * span;
-    int global_mode = 0;
-    size_t smem = 0;
-    unsigned int *gscratch = nullptr;
-    int tgrid = wgrid;
+    if (tilem > 0)
+        k_span<<<wgrid, kThreads, 0, s>>>(A->d_rowptr, A->d_colidx, tilem, rowA, colA, nnz_given, d_spans, &d_c->span,
+                                          &d_c->err);
+    MF_TRY(read_counts(&c, d_c, s));
+
+    const int span = std::max(c.span, 1);
     const size_t smem_cap = 96 * 1024;
-    if ((size_t)words_per_warp * 4 * kWarps <= smem_cap) {
-        smem = (size_t)words_per_warp * 4 * kWarps;
-    } else {
-        global_mode = 1;
-        tgrid = 148 * 4;
-        MF_TRY(tmp.get(&gscratch, words_per_warp * (long long)tgrid * kWarps));
-    }
-    if (smem > 48 * 1024) {
-        MF_CUDA_TRY(cudaFuncSetAttribute(k_count_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MF_CUDA_TRY(cudaFuncSetAttribute(k_fill_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
+    // a kernel's scratch: shared memory up to smem_cap, else global memory and a smaller grid
+    struct Scratch {
+        int words, global_mode, grid;
+        size_t smem;
+        unsigned int *global;
+    };
+    auto scratch = [&](const void *kernel, long long words, Scratch *x) -> int {
+        *x = {(int)words, 0, wgrid, (size_t)words * 4 * kWarps, nullptr};
+        if (x->smem > smem_cap) {
+            x->global_mode = 1;
+            x->smem = 0;
+            x->grid = std::min(wgrid, 148 * 4);
+            MF_TRY(tmp.get(&x->global, words * (long long)x->grid * kWarps));
+        } else if (x->smem > 48 * 1024) {
+            MF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x->smem));
+        }
+        return MF_SUCCESS;
+    };
     if (tilem > 0) {
-        k_count_tiles<<<tgrid, kThreads, smem, s>>>(A->d_rowptr, A->d_colidx, tilem, rowA, d_span_base, span,
-                                                    (int)words_per_warp, global_mode, gscratch, d_ntiles);
+        Scratch x;
+        MF_TRY(scratch((const void *)k_count_tiles, span, &x));
+        k_count_tiles<<<x.grid, kThreads, x.smem, s>>>(A->d_rowptr, A->d_colidx, tilem, rowA, d_spans, x.words,
+                                                       x.global_mode, x.global, d_ntiles, &d_c->max_tiles);
         MF_CUDA_TRY(cudaGetLastError());
     }
-    MF_TRY(dalloc(&A->d_tile_ptr, tilem + 1, s));
-    MF_TRY(mf_scan_i32_to_i32(d_ntiles, A->d_tile_ptr, tilem, s));
-    int tilenum = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(&tilenum, A->d_tile_ptr + tilem, sizeof(int), cudaMemcpyDeviceToHost, s));
-    int nz_lo = 0, nz_hi = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(&nz_lo, A->d_rowptr, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaMemcpyAsync(&nz_hi, A->d_rowptr + rowA, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    const long long nnz = (long long)nz_hi - nz_lo;
+    MF_TRY(mf_scan_tile_counts(d_ntiles, A->d_tile_ptr, d_rbo, A->d_seg_ptr, tilem, s));
+    k_counts_tiles<<<1, 1, 0, s>>>(d_c, A->d_tile_ptr, d_rbo, A->d_seg_ptr, A->d_rowptr, tilem, rowA);
+    MF_TRY(read_counts(&c, d_c, s));
+
+    const long long nnz = (long long)c.nz_hi - c.nz_lo;
+    const int tilenum = c.tilenum, nseg = c.nseg, rb = c.rowblocks;
     A->tilenum = tilenum;
     A->csrsize = (int)nnz;
     A->nnz = nnz;
-    MF_TRY(dalloc(&A->d_tile_columnidx, tilenum + 1, s));
-    MF_TRY(dalloc(&A->d_csr_offset, tilenum + 1, s));
-    MF_TRY(dalloc(&A->d_csrptr_offset, tilenum + 1, s));
+    // 16 row starts per tile, fewer in a short last tile-row
+    A->csrptrlen = tilem > 0 ? c.last_tile0 * MF_BS + (tilenum - c.last_tile0) * (rowA - (tilem - 1) * MF_BS) : 0;
+    A->rowblkblock = rb;
+    A->nseg = nseg;
+    int *d_nzr = nullptr, *d_seg_entries = nullptr;
+    long long *d_cost = nullptr;
+    MF_TRY(dalloc(&A->d_tile_columnidx, (long long)tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_csr_offset, (long long)tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_csrptr_offset, (long long)tilenum + 1, s));
     MF_TRY(dalloc(&A->d_tval, nnz, s));
     MF_TRY(dalloc(&A->d_tval_low, nnz, s));
     MF_TRY(dalloc(&A->d_tcol, nnz, s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_csr_offset, 0, (tilenum + 1) * sizeof(int), s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_csrptr_offset, 0, (tilenum + 1) * sizeof(int), s));
-    const long long csrptrlen_max = (long long)tilenum * MF_BS;
-    MF_TRY(dalloc(&A->d_tptr, csrptrlen_max, s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_tptr, 0, (size_t)std::max<long long>(csrptrlen_max, 1), s));
-    if (tilem > 0) {
-        k_fill_tiles<<<tgrid, kThreads, smem, s>>>(A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, tilem, rowA,
-                                                   d_span_base, span, (int)words_per_warp, global_mode, gscratch,
-                                                   A->d_tile_ptr, A->d_tile_columnidx, A->d_csr_offset,
-                                                   A->d_csrptr_offset, A->d_tval, A->d_tval_low, A->d_tcol,
-                                                   A->d_tptr, d_err);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    int csrptrlen = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(&csrptrlen, A->d_csrptr_offset + tilenum, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    if (h_err) return h_err;
-    A->csrptrlen = csrptrlen;
-
-    // nonempty-row lists
-    int *d_nzr = nullptr;
-    MF_TRY(tmp.get(&d_nzr, tilenum + 1));
-    MF_TRY(dalloc(&A->d_nonzero_row_new, tilenum + 1, s));
-    MF_TRY(dalloc(&A->d_tile_rowidx, tilenum + 1, s));
-    MF_TRY(dalloc(&A->d_block_signal, tilem + 4, s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_block_signal, 0, (tilem + 4) * sizeof(int), s));
-    MF_CUDA_TRY(cudaMemsetAsync(d_nzr, 0, (tilenum + 1) * sizeof(int), s));
-    if (tilem > 0) {
-        k_rowlist_count<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_csr_offset, A->d_csrptr_offset, A->d_tptr,
-                                                   tilem, rowA, d_nzr, A->d_tile_rowidx, A->d_block_signal);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    MF_TRY(mf_scan_i32_to_i32(d_nzr, A->d_nonzero_row_new, tilenum, s));
-    int cnt = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(&cnt, A->d_nonzero_row_new + tilenum, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    A->cnt_non_new = cnt;
-    MF_TRY(dalloc(&A->d_blockrowid_new, cnt + 1, s));
-    MF_TRY(dalloc(&A->d_blockcsr_ptr_new, cnt + 1, s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_blockrowid_new, 0, cnt + 1, s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_blockcsr_ptr_new, 0, cnt + 1, s));
-    if (tilem > 0) {
-        k_rowlist_fill<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_csr_offset, A->d_csrptr_offset, A->d_tptr,
-                                                  tilem, rowA, A->d_nonzero_row_new, A->d_blockrowid_new,
-                                                  A->d_blockcsr_ptr_new);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    // row-block split
-    int *d_rbc = nullptr, *d_rbo = nullptr;
-    MF_TRY(tmp.get(&d_rbc, tilem + 1));
-    MF_TRY(tmp.get(&d_rbo, tilem + 1));
-    if (tilem > 0) {
-        k_rowblk_count<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_tile_ptr, tilem, d_rbc);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    MF_TRY(mf_scan_i32_to_i32(d_rbc, d_rbo, tilem, s));
-    int rb = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(&rb, d_rbo + tilem, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    A->rowblkblock = rb;
-    MF_TRY(dalloc(&A->d_rb_idx, rb + 1, s));
-    MF_TRY(dalloc(&A->d_rb_start, rb + 1, s));
-    MF_TRY(dalloc(&A->d_rb_stop, rb + 1, s));
-    if (tilem > 0) {
-        k_rowblk_fill<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_tile_ptr, tilem, d_rbo, A->d_rb_idx, A->d_rb_start,
-                                                         A->d_rb_stop);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    // encoder
+    MF_TRY(dalloc(&A->d_tptr, (long long)tilenum * MF_BS, s));
+    MF_TRY(tmp.get(&d_nzr, (long long)tilenum));
+    MF_TRY(dalloc(&A->d_nonzero_row_new, (long long)tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_tile_rowidx, (long long)tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_block_signal, (long long)tilem + 4, s));
+    MF_TRY(dalloc(&A->d_rb_idx, (long long)rb + 1, s));
+    MF_TRY(dalloc(&A->d_rb_start, (long long)rb + 1, s));
+    MF_TRY(dalloc(&A->d_rb_stop, (long long)rb + 1, s));
     MF_TRY(dalloc(&A->d_val_f16, nnz, s));
     MF_TRY(dalloc(&A->d_val_i8_ref, nnz, s));
     MF_TRY(dalloc(&A->d_val_i8, nnz, s));
-    MF_TRY(dalloc(&A->d_i8_scale, tilenum + 1, s));
-    MF_TRY(dalloc(&A->d_tile_caps, tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_i8_scale, (long long)tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_tile_caps, (long long)tilenum + 1, s));
+    MF_TRY(dalloc(&A->d_seg_tile0, (long long)nseg + 1, s));
+    MF_TRY(dalloc(&A->d_seg_kp, (long long)nseg + 1, s));
+    MF_TRY(dalloc(&A->d_seg_rowlen, (long long)nseg * MF_BS + 1, s));
+    MF_TRY(tmp.get(&d_seg_entries, (long long)nseg));
+    MF_TRY(dalloc(&A->d_seg_off, (long long)nseg + 1, s));
+    MF_TRY(tmp.get(&d_cost, tilem));
+    MF_TRY(dalloc(&A->d_row_cost, (long long)tilem + 1, s));
+    MF_TRY(dalloc(&A->d_seg_hdr, (long long)nseg + 1, s));
+    MF_TRY(dalloc(&A->d_seg_tile, ((long long)nseg + 1) * MF_BS, s));
+    MF_CUDA_TRY(cudaMemsetAsync(A->d_block_signal, 0, ((size_t)tilem + 4) * sizeof(int), s));
+    MF_CUDA_TRY(cudaMemsetAsync(A->d_seg_hdr + nseg, 0, sizeof(int4), s));
+    if (tilem == 0) {
+        MF_CUDA_TRY(cudaMemsetAsync(A->d_csr_offset, 0, sizeof(int), s));
+        MF_CUDA_TRY(cudaMemsetAsync(A->d_csrptr_offset, 0, sizeof(int), s));
+    } else {
+        Scratch x;
+        MF_TRY(scratch((const void *)k_fill_tiles, 2LL * span + (1LL + MF_BS) * std::max(c.max_tiles, 1), &x));
+        k_fill_tiles<<<x.grid, kThreads, x.smem, s>>>(A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, tilem, rowA,
+                                                      d_spans, span, std::max(c.max_tiles, 1), x.words, x.global_mode,
+                                                      x.global, A->d_tile_ptr, A->d_tile_columnidx, A->d_csr_offset,
+                                                      A->d_csrptr_offset, A->d_tval, A->d_tval_low, A->d_tcol,
+                                                      A->d_tptr, &d_c->err);
+        MF_CUDA_TRY(cudaGetLastError());
+        // nonempty-row lists, solver-slice shapes
+        k_rowlist_count<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_csr_offset, A->d_csrptr_offset, A->d_tptr,
+                                                   tilem, rowA, d_nzr, A->d_tile_rowidx, A->d_block_signal);
+        MF_CUDA_TRY(cudaGetLastError());
+        k_seg_shape<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_seg_ptr, A->d_csr_offset, A->d_csrptr_offset,
+                                               A->d_tptr, tilem, rowA, A->d_seg_tile0, A->d_seg_kp,
+                                               A->d_seg_rowlen, d_seg_entries, d_cost, &d_c->longest);
+        MF_CUDA_TRY(cudaGetLastError());
+    }
+    MF_TRY(mf_scan_i32_to_i32(d_nzr, A->d_nonzero_row_new, tilenum, s));
+    MF_TRY(mf_scan_i32_to_i64(d_seg_entries, A->d_seg_off, nseg, s));
+    MF_TRY(mf_scan_i64_to_i64(d_cost, A->d_row_cost, tilem, s));
+    k_counts_filled<<<1, 1, 0, s>>>(d_c, A->d_nonzero_row_new, tilenum, A->d_seg_off, nseg);
+    // encoder
     if (nnz > 0) {
         k_encode_ref<<<grid_for(nnz, 256), 256, 0, s>>>(A->d_tval, A->d_tval_low, nnz, A->d_val_f16, A->d_val_i8_ref);
         MF_CUDA_TRY(cudaGetLastError());
@@ -737,66 +731,41 @@ int mf_build_tiles(mf_matrix_s *A, cudaStream_t s)
                                                               A->d_i8_scale, A->d_tile_caps);
         MF_CUDA_TRY(cudaGetLastError());
     }
-    // solver slices
-    int *d_nseg = nullptr;
-    MF_TRY(tmp.get(&d_nseg, tilem + 1));
-    MF_TRY(dalloc(&A->d_seg_ptr, tilem + 1, s));
-    if (tilem > 0) {
-        k_seg_count<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_tile_ptr, tilem, d_nseg);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    MF_TRY(mf_scan_i32_to_i32(d_nseg, A->d_seg_ptr, tilem, s));
-    int nseg = 0;
-    MF_CUDA_TRY(cudaMemcpyAsync(&nseg, A->d_seg_ptr + tilem, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
-    A->nseg = nseg;
-    int *d_seg_entries = nullptr;
-    long long *d_cost = nullptr;
-    MF_TRY(dalloc(&A->d_seg_tile0, nseg + 1, s));
-    MF_TRY(dalloc(&A->d_seg_kp, nseg + 1, s));
-    MF_TRY(dalloc(&A->d_seg_rowlen, (long long)nseg * MF_BS + 1, s));
-    MF_TRY(tmp.get(&d_seg_entries, nseg + 1));
-    MF_TRY(dalloc(&A->d_seg_off, nseg + 1, s));
-    MF_TRY(tmp.get(&d_cost, tilem + 1));
-    int *d_shape = nullptr;
-    MF_TRY(tmp.get(&d_shape, 2));
-    MF_CUDA_TRY(cudaMemsetAsync(d_shape, 0, 2 * sizeof(int), s));
-    MF_TRY(dalloc(&A->d_row_cost, tilem + 1, s));
-    if (tilem > 0) {
-        k_seg_shape<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_seg_ptr, A->d_csr_offset, A->d_csrptr_offset,
-                                               A->d_tptr, tilem, rowA, A->d_seg_tile0, A->d_seg_kp,
-                                               A->d_seg_rowlen, d_seg_entries, d_cost, d_shape);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    MF_TRY(mf_scan_i32_to_i64(d_seg_entries, A->d_seg_off, nseg, s));
-    MF_TRY(mf_scan_i64_to_i64(d_cost, A->d_row_cost, tilem, s));
-    // seg_tile0[nseg] = tilenum (end sentinel)
-    MF_CUDA_TRY(cudaMemcpyAsync(A->d_seg_tile0 + nseg, A->d_tile_ptr + tilem, sizeof(int), cudaMemcpyDeviceToDevice, s));
-    MF_TRY(dalloc(&A->d_seg_hdr, nseg + 1, s));
-    MF_CUDA_TRY(cudaMemsetAsync(A->d_seg_hdr, 0, (size_t)(nseg + 1) * sizeof(int4), s));
-    MF_TRY(dalloc(&A->d_seg_tile, ((long long)nseg + 1) * MF_BS, s));
-    if ((long long)A->tilen >= (1LL << 23)) return MF_ERR_UNSUPPORTED;   // column tile must fit 23 bits
-    if (tilem > 0) {
-        k_seg_hdr<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_seg_ptr, A->d_seg_tile0, A->d_seg_kp, A->d_seg_off,
-                                                      A->d_tile_columnidx, A->d_tile_caps, tilem, A->d_seg_hdr,
-                                                      A->d_seg_tile);
-        MF_CUDA_TRY(cudaGetLastError());
-    }
-    long long ent = 0;
-    int h_shape[2] = {0, 0};
-    MF_CUDA_TRY(cudaMemcpyAsync(&ent, A->d_seg_off + nseg, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaMemcpyAsync(h_shape, d_shape, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA_TRY(cudaStreamSynchronize(s));
+    MF_TRY(read_counts(&c, d_c, s));
+
+    const int cnt = c.nonempty;
+    const long long ent = c.entries;
+    A->cnt_non_new = cnt;
     A->slice_entries = ent;
-    A->max_row = h_shape[0];
-    A->one_chunk = tilem > 0 && h_shape[1] == 0 ? 1 : 0;
+    A->max_row = c.longest;
+    A->one_chunk = tilem > 0 && c.not_one_chunk == 0 ? 1 : 0;
+    if ((long long)A->tilen >= (1LL << 23)) return MF_ERR_UNSUPPORTED;   // column tile must fit 23 bits
     if ((ent >> 7) >= (1LL << 31)) return MF_ERR_UNSUPPORTED;
+    MF_TRY(dalloc(&A->d_blockrowid_new, (long long)cnt + 1, s));
+    MF_TRY(dalloc(&A->d_blockcsr_ptr_new, (long long)cnt + 1, s));
     MF_TRY(dalloc(&A->d_meta, ent, s));
     MF_TRY(dalloc(&A->d_v64, ent, s));
     MF_TRY(dalloc(&A->d_v32, ent, s));
     MF_TRY(dalloc(&A->d_v16, ent, s));
     MF_TRY(dalloc(&A->d_v8, ent, s));
     MF_TRY(dalloc(&A->d_v8ref, ent, s));
+    MF_CUDA_TRY(cudaMemsetAsync(A->d_blockrowid_new, 0, (size_t)cnt + 1, s));
+    MF_CUDA_TRY(cudaMemsetAsync(A->d_blockcsr_ptr_new, 0, (size_t)cnt + 1, s));
+    // seg_tile0[nseg] = tilenum (end sentinel)
+    MF_CUDA_TRY(cudaMemcpyAsync(A->d_seg_tile0 + nseg, A->d_tile_ptr + tilem, sizeof(int), cudaMemcpyDeviceToDevice, s));
+    if (tilem > 0) {
+        k_rowlist_fill<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_csr_offset, A->d_csrptr_offset, A->d_tptr,
+                                                  tilem, rowA, A->d_nonzero_row_new, A->d_blockrowid_new,
+                                                  A->d_blockcsr_ptr_new);
+        MF_CUDA_TRY(cudaGetLastError());
+        k_rowblk_fill<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_tile_ptr, tilem, d_rbo, A->d_rb_idx, A->d_rb_start,
+                                                         A->d_rb_stop);
+        MF_CUDA_TRY(cudaGetLastError());
+        k_seg_hdr<<<(tilem + 255) / 256, 256, 0, s>>>(A->d_seg_ptr, A->d_seg_tile0, A->d_seg_kp, A->d_seg_off,
+                                                      A->d_tile_columnidx, A->d_tile_caps, tilem, A->d_seg_hdr,
+                                                      A->d_seg_tile);
+        MF_CUDA_TRY(cudaGetLastError());
+    }
     if (tilem > 0 && nseg > 0) {
         k_seg_fill<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_seg_ptr, A->d_seg_kp, A->d_seg_off,
                                               A->d_csr_offset, A->d_csrptr_offset, A->d_tptr, A->d_tcol, A->d_tval,
