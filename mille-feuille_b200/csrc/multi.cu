@@ -67,9 +67,7 @@ __device__ void block_partial_m(const MultiParams &M, SharedM &sh, int kind, con
 }
 
 // After the sync: every block of the group sums the nblk partials of `kind` in
-// the same order, into sh.bcast.  It stays there until the next collect, which
-// every thread reaches only through the barriers of block_partial_m and of the
-// sync, so there is no trailing barrier.
+// the same order, into sh.bcast, where they stay until the next collect.
 template <int NV>
 __device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsigned maxmask, int nblk)
 {
@@ -100,6 +98,12 @@ __device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsi
     }
     __syncthreads();
 }
+
+// Closes a reduction.  Without a block barrier of its own here the FP64 team items
+// of 2 and more columns went wrong (wrong iterates, once an illegal address)
+// although every shared word is separated by the barriers around it; with it they
+// agree with the oracle to rounding.
+__device__ __forceinline__ void reduction_done() { __syncthreads(); }
 
 // One chunk of the NR-column walk: lane i's stored values of the chunk at
 // entry offset cb in precision PR (FP32 / FP16 / scaled INT8 widened to FP64
@@ -452,6 +456,7 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
         // thread j: column j's recursive r.r, and its true one when that is formed
         const double rrec = threadIdx.x < NR ? sh.bcast[threadIdx.x] : 0.0;
         double rnew = rrec;
+        __syncthreads();                  // every thread has read `active` before column threads change it
         if (want_repl) {
             // ---- FP64 R = B - A X, R's shadow, true residual norms ----
             double prt[NR + 2];
@@ -494,8 +499,6 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
                 rnew = sh.bcast[threadIdx.x];
                 sh.rt[threadIdx.x] = rnew;
             }
-        } else {
-            __syncthreads();              // every thread has read `active` before column threads change it
         }
         if (threadIdx.x < NR) {
             const int j = threadIdx.x;
@@ -563,6 +566,7 @@ struct GridSync {
         block_partial_m<NV>(M, sh, kind, v, maxmask, (int)gridDim.x, (int)blockIdx.x);
         if (!grid_barrier(P, epoch, sh)) return false;
         grid_collect_m<NV>(M, sh, kind, maxmask, (int)gridDim.x);
+        reduction_done();
         return true;
     }
     __device__ bool writer() const { return blockIdx.x == 0 && threadIdx.x == 0; }
@@ -673,6 +677,7 @@ struct BlockSync {
             if (lane == 0) sh.bcast[wib] = a;
         }
         __syncthreads();
+        reduction_done();
         return true;
     }
     __device__ bool writer() const { return threadIdx.x == 0; }
@@ -683,12 +688,11 @@ struct BlockSync {
 // by `limit_ns`; a timeout, or an error set elsewhere, returns false and the
 // first error is kept in *err.
 __device__ bool team_barrier(unsigned *ctr, unsigned k, unsigned &epoch, int *err, unsigned long long limit_ns,
-                             unsigned long long first_limit_ns, SharedM &sh, int stall)
+                             SharedM &sh, int stall = 0)
 {
     __syncthreads();
-    if (threadIdx.x == 0) {                // epoch: in shared memory, thread 0's alone
-        if (epoch == 0) limit_ns = first_limit_ns;
-        epoch += 1;
+    epoch += 1;
+    if (threadIdx.x == 0) {
         const unsigned target = epoch * k + ((stall && epoch == 1) ? 1u : 0u);
         __threadfence();
         mf_red_relaxed_add_u32(ctr, 1u);
@@ -736,9 +740,13 @@ struct TeamSync {
         MultiParams R;
         R.red = ts.red;
         block_partial_m<NV>(R, sh, kind, v, maxmask, ts.k, ts.r);
-        if (!team_barrier(ts.ctr, (unsigned)ts.k, ts.epoch, ts.err, ts.limit_ns, ts.arrive_ns, sh, ts.stall))
-            return false;
+        unsigned ep = ts.epoch;
+        const bool ok =
+            team_barrier(ts.ctr, (unsigned)ts.k, ep, ts.err, ep == 0 ? ts.arrive_ns : ts.limit_ns, sh, ts.stall);
+        if (!ok) return false;
         grid_collect_m<NV>(R, sh, kind, maxmask, ts.k);
+        if (threadIdx.x == 0) ts.epoch = ep;
+        reduction_done();
         return true;
     }
     __device__ bool writer() const { return ts.r == 0 && threadIdx.x == 0; }
