@@ -737,11 +737,12 @@ __device__ __forceinline__ void spmv_range_lean(const SolverParams &P, int sb, i
 // cost 5 % on 128^3: then the update phase touches a row from another SM than
 // the product did.
 //
-// These products move what L2 and DRAM can deliver (128^3 FP32: 11 TB/s through
-// L2 inside a solve; 2048^2 FP64: 6.1 TB/s of DRAM), so bytes and requests count:
-// a TMA ring with mbarriers, asynchronous copies of the epilogue's operands,
-// gathers one step ahead and 3 or 4 blocks per SM were all measured, and none was
-// faster than this walk with the next chunk in registers.
+// What bounds it: DRAM for vectors larger than L2 (2048^2 FP64: 485 MB in 79 us,
+// 6.1 TB/s, a copy's speed), the gathers' trips to L2 otherwise (128^3 mixed: L2
+// 34 % busy, long_scoreboard first among the stalls).  Keeping more in flight was
+// tried in whole iterations and did not help: a TMA ring with mbarriers, copies of
+// the epilogue's operands with cp.async, gathers one step ahead, 3 or 4 blocks per
+// SM; none was faster than this walk with the next chunk in registers.
 template <int PR, int LEN, typename Epi>
 __device__ __forceinline__ void spmv_rows(const SolverParams &P, int R, int end, int stride, int i, unsigned hmask,
                                           const double *x64, Epi &epi)
