@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_spmv(SolverParams P, int force
         re = min(P.tilem, rb + rows_per_hw);
         if (rb >= re) return;
     }
-    spmv_range<MODE, MODE == MODE_FP64, LEN>(P, P.seg_ptr[rb], P.seg_ptr[re], i, hmask, X, nullptr, store);
+    spmv_range<MODE, MODE == MODE_FP64, LEN, true>(P, P.seg_ptr[rb], P.seg_ptr[re], i, hmask, X, nullptr, store);
     for (int R = rb; R < re; R++)            // tile-rows without tiles: y = 0
         if (P.seg_ptr[R] == P.seg_ptr[R + 1]) store(R, 0.0);
 }
@@ -377,7 +377,9 @@ int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_optio
     // (They stay out of the stalled-barrier test, which needs the grid counter.)
     const bool rows = A->one_chunk && mode != MODE_PARITY && w->lb == 2;
     const bool small = mode != MODE_PARITY && w->lb == 2 && !opt->test_stall_barrier;
-    const bool cluster = small && w->cluster;
+    // (BiCGSTAB on more than 512 tile-rows would be summed over fewer blocks than the
+    // grid's: its rounding stays as it is there.)
+    const bool cluster = small && w->cluster && (opt->method == MF_METHOD_CG || w->cluster == w->G);
     const void *kfn = cluster ? mf_solve_cluster_kernel(mode, opt->method, A->one_chunk ? A->max_row : 0,
                                                           (A->tilem + w->cluster * kWarps * 2 - 1) /
                                                               (w->cluster * kWarps * 2))

@@ -255,17 +255,22 @@ __device__ void grid_collect(const SolverParams &P, SharedT<CL> &sh, int kind, i
                              double *outv)
 {
     if constexpr (CL) {
-        // every block holds all partials: each thread sums them in the same order
+        // every block holds all partials: each thread sums them as the grid's shuffle
+        // tree does (blocks 8 apart first, then 4, 2, 1)
 #pragma unroll
         for (int k = 0; k < kRedWidth; k++) {
             if (k >= nv) break;
             const bool mx = (maxmask >> k) & 1u;
-            double a = sh.part[kind][k][0];
-            for (int c = 1; c < P.cluster; c++) {
-                const double b = sh.part[kind][k][c];
-                a = mx ? fmax(a, b) : a + b;
-            }
-            outv[k] = a;
+            double t[kMaxCluster];
+#pragma unroll
+            for (int c = 0; c < kMaxCluster; c++)
+                t[c] = c < P.cluster ? sh.part[CL ? kind : 0][k][c] : (mx ? -1.0e300 : 0.0);
+#pragma unroll
+            for (int o = kMaxCluster / 2; o; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < kMaxCluster / 2; c++)
+                    if (c < o) t[c] = mx ? fmax(t[c], t[c + o]) : t[c] + t[c + o];
+            outv[k] = t[0];
         }
         return;
     }
@@ -835,16 +840,21 @@ __device__ __forceinline__ void spmv_rows_dyn(const SolverParams &P, int R, int 
 // LEN > 0: a one-chunk matrix with rows of up to LEN entries (spmv_rows; the
 // range is then the block's own tile-rows in a solve, all of them in turn in the
 // standalone product, and sb, se are not used).
-template <int MODE, bool F64, int LEN, typename Epi>
+// TURN: the half-warps take the block's tile-rows in turn; without it each walks
+// its own range, so dot products are summed as by the general walk.  BiCGSTAB
+// does: its recurrences amplify the rounding of their order (two orders of the sums
+// were 1.9e-9 apart after 20 iterations on a 48^3 upwind system, with FP64's own
+// error at 3.7e-9), and turns gave it 3 %.
+template <int MODE, bool F64, int LEN, bool TURN, typename Epi>
 __device__ __forceinline__ void spmv_range(const SolverParams &P, int sb, int se, int i, unsigned hmask,
                                            const XVec &X, unsigned *cnt, Epi epi, unsigned *whole = nullptr)
 {
     if constexpr (LEN > 0) {
         const int h = (int)(threadIdx.x >> 4);
         const int *hb = P.hw_begin ? P.hw_begin + blockIdx.x * kWarps * 2 : nullptr;
-        const int R = hb ? hb[0] + h : (int)blockIdx.x * kWarps * 2 + h;
-        const int end = hb ? hb[kWarps * 2] : P.tilem;
-        const int stride = hb ? kWarps * 2 : (int)gridDim.x * kWarps * 2;
+        const int R = !hb ? (int)blockIdx.x * kWarps * 2 + h : TURN ? hb[0] + h : hb[h];
+        const int end = !hb ? P.tilem : TURN ? hb[kWarps * 2] : hb[h + 1];
+        const int stride = !hb ? (int)gridDim.x * kWarps * 2 : TURN ? kWarps * 2 : 1;
         if constexpr (MODE == MODE_FP64 || F64) {
             spmv_rows<MF_P64, LEN>(P, R, end, stride, i, hmask, X.x64, epi);
         } else {
@@ -1161,7 +1171,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                               &bmin);
             pb += rv * rv;
         };
-        spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, init_row);
+        spmv_range<MODE, true, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, init_row);
         for (int R = c.rbeg; LEN == 0 && R < c.rend; R++)
             if (P.seg_ptr[R] == P.seg_ptr[R + 1]) init_row(R, 0.0);
         nspmv++;
@@ -1406,7 +1416,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             XVec XA = make_x(P.r, nullptr, nullptr, nullptr, P.mag_r, nullptr, invM, dynA);
             if (MODE == MODE_MIXED && prA != MF_P32) XA.force_pr = prA;
             if (P.lean_f16) XA.lean_pr = MF_P16;
-            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask, XA, cnt, [&](int R, double y) {
+            spmv_range<MODE, false, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask, XA, cnt, [&](int R, double y) {
                 const int row = R * MF_BS + c.i;
                 if (row < n) {
                     const double pn = P.r[row] + beta2 * P.p[row];
@@ -1498,7 +1508,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
                 rmax = 0.0f;
                 rmin = 3.0e38f;
                 rsm = 0.0f;
-                spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr,
+                spmv_range<MODE, true, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr,
                                        [&](int R, double y) {
                                            const int row = R * MF_BS + c.i;
                                            const bool valid = row < n;
@@ -1552,7 +1562,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
         if (!bicg) {
             // ---- A: q = A p, p.q ----
             double ppq = 0.0;
-            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask,
+            spmv_range<MODE, false, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask,
                              make_x(P.p, P.p32, P.p16, P.p8, P.mag_p, P.lab_p, invM), cnt,
                              [&](int R, double y) {
                                  const int row = R * MF_BS + c.i;
@@ -1600,7 +1610,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             double prv = 0.0;
             const int useA = (kFb && coolA > 0) ? 0 : dynA;
             const unsigned d0A = demoted();
-            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask,
+            spmv_range<MODE, false, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask,
                              lean_base(make_x(P.p, P.p32, P.p16, P.p8, P.mag_p, P.lab_p, invM, useA)), cnt,
                              [&](int R, double y) {
                                  const int row = R * MF_BS + c.i;
@@ -1645,7 +1655,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             double pts = 0.0, ptt = 0.0;
             const int useS = (kFb && coolS > 0) ? 0 : dynS;
             const unsigned d0S = demoted();
-            spmv_range<MODE, false, LEN>(P, c.sbeg, c.send, c.i, c.hmask,
+            spmv_range<MODE, false, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask,
                              lean_base(make_x(P.s, P.s32, P.s16, P.s8, P.mag_s, P.lab_s, invMs, useS)), cnt,
                              [&](int R, double y) {
                                  const int row = R * MF_BS + c.i;
@@ -1703,7 +1713,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
             }
             // ---- FP64 true residual: r = b - A x ----
             double prt = 0.0, prth = 0.0;
-            spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
+            spmv_range<MODE, true, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
                 const int row = R * MF_BS + c.i;
                 if (row < n) {
                     const double rv = P.b[row] - y;
@@ -1792,7 +1802,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
     // ---- final FP64 true residual when the last one was not already formed ----
     if (!last_true) {
         double prt = 0.0;
-        spmv_range<MODE, true, LEN>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
+        spmv_range<MODE, true, LEN, !bicg>(P, c.sbeg, c.send, c.i, c.hmask, fp64_x(P.x), nullptr, [&](int R, double y) {
             const int row = R * MF_BS + c.i;
             if (row < n) {
                 const double d = P.b[row] - y;
