@@ -152,6 +152,11 @@ __device__ __forceinline__ void cluster_barrier()
 }
 
 // A double into another block's copy of `p` (shared memory of the cluster's block `rank`).
+// Another block's shared memory may be accessed only between that block's start and
+// its exit.  Start: k_solve passes a cluster_barrier before its first reduction, and
+// no block leaves that barrier before all have arrived.  Exit: every store here is
+// followed by a cluster_barrier that the target passes too (solve_barrier, before the
+// partials are read), and a block returns only after its last one.
 __device__ __forceinline__ void cluster_store(double *p, int rank, double v)
 {
     const unsigned a = (unsigned)__cvta_generic_to_shared(p);
@@ -1127,6 +1132,7 @@ __global__ void __launch_bounds__(kThreads, LB) k_solve(SolverParams P)
 {
     constexpr bool CL = VAR >= kVarCluster;
     __shared__ SharedT<CL> sh;
+    if constexpr (CL) cluster_barrier();       // every block has started: see cluster_store
     const Ctx c = make_ctx(P);
     unsigned epoch = 0;
     // tile-use counters: FP64 mode needs none (every tile of every SpMV is FP64;
