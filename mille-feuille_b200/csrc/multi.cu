@@ -19,7 +19,7 @@ constexpr int kRedWidthM = kMaxNR + 2;    // NR dot products + segment max / -mi
 struct SharedM {
     double wred[kWarps][kRedWidthM];
     double bcast[kRedWidthM];
-    double alpha[kMaxNR], beta[kMaxNR], rr[kMaxNR], thr2[kMaxNR], bb[kMaxNR], rt[kMaxNR];
+    double alpha[kMaxNR], beta[kMaxNR], rr[kMaxNR], thr2[kMaxNR], bb[kMaxNR];
     int active[kMaxNR], pending[kMaxNR], iters[kMaxNR], conv[kMaxNR];
     int brk;                  // some column broke down (a scalar became non-finite)
     int flag;                 // grid_barrier's result
@@ -35,12 +35,15 @@ struct MultiParams {
 };
 
 // Block partial of NV values (maxmask bit k: max instead of sum) into
-// red[kind][bidx][*] of an nblk-block group (the grid, or a batched item's team).
+// red[kind][*][bidx] of an nblk-block group (the grid, or a batched item's team).
+// The half-warps of a warp come from loops over tile-row ranges of different
+// lengths: they meet here before the shuffles and the barriers.
 template <int NV>
 __device__ void block_partial_m(const MultiParams &M, SharedM &sh, int kind, const double (&v)[NV], unsigned maxmask,
                                 int nblk, int bidx)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < NV; k++) {
         double a = v[k];
@@ -69,7 +72,8 @@ __device__ void block_partial_m(const MultiParams &M, SharedM &sh, int kind, con
 // After the sync: every block of the group sums the nblk partials of `kind` in
 // the same order, into sh.bcast, where they stay until the next collect.
 template <int NV>
-__device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsigned maxmask, int nblk)
+__device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsigned maxmask, double (&out)[NV],
+                               int nblk)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (wib < NV) {
@@ -97,13 +101,10 @@ __device__ void grid_collect_m(const MultiParams &M, SharedM &sh, int kind, unsi
         if (lane == 0) sh.bcast[wib] = a;
     }
     __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; k++) out[k] = sh.bcast[k];
+    __syncthreads();
 }
-
-// Closes a reduction.  Without a block barrier of its own here the FP64 team items
-// of 2 and more columns went wrong (wrong iterates, once an illegal address)
-// although every shared word is separated by the barriers around it; with it they
-// agree with the oracle to rounding.
-__device__ __forceinline__ void reduction_done() { __syncthreads(); }
 
 // One chunk of the NR-column walk: lane i's stored values of the chunk at
 // entry offset cb in precision PR (FP32 / FP16 / scaled INT8 widened to FP64
@@ -260,10 +261,7 @@ __device__ __forceinline__ void store_row(double *v, int row, const double (&in)
 }
 
 // The CG iterations on NR columns, generic in how the threads that share a
-// system synchronise: the whole grid (k_solve_multi), a team or one block
-// (k_batch).  sy.reduce leaves its results in sh.bcast; thread j keeps column j's
-// scalars (one thread for all of them spent 8 divisions in a row on every
-// block's critical path, twice an iteration).
+// system synchronise: the whole grid (k_solve_multi) or one block (k_batch).
 template <int MODE, int NR, class Sync>
 __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const Ctx &c, SharedM &sh, Sync &sy)
 {
@@ -275,7 +273,7 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
     // ---- init: X = 0, R = B, P = Q = 0; |b_k|^2; R's segment magnitudes ----
     // With an initial guess (x0_given): |b_k|^2 reduced first (it scales the
     // convergence test), then R = B - A X in FP64.
-    double pb[NR + 2];
+    double pb[NR + 2], bb0[NR];
 #pragma unroll
     for (int k = 0; k < NR + 2; k++) pb[k] = 0.0;
     SegMM st = {0.0f, 3.0e38f};
@@ -292,8 +290,7 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
                 for (int k = 0; k < NR; k++) pbb[k] += bv[k] * bv[k];
             }
         }
-        if (!sy.template reduce<NR>(8, pbb, 0u)) return;
-        if (threadIdx.x < NR) sh.bb[threadIdx.x] = sh.bcast[threadIdx.x];
+        if (!sy.template reduce<NR>(8, pbb, 0u, bb0)) return;
         auto init_r = [&](int R, const double (&y)[NR]) {
             const int row = R * MF_BS + c.i;
             const bool valid = row < n;
@@ -341,31 +338,33 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
     }
     pb[NR] = st.mx;
     pb[NR + 1] = -st.mn;
-    if (!sy.template reduce<NR + 2>(0, pb, mm2)) return;
-    if (threadIdx.x < NR) {
-        const int k = threadIdx.x;
-        const double rr0 = sh.bcast[k];
-        if (!P.x0_given) sh.bb[k] = rr0;
-        sh.rr[k] = rr0;
-        sh.rt[k] = rr0;
-        sh.thr2[k] = P.tol * P.tol * sh.bb[k];
-        sh.beta[k] = 0.0;
-        sh.pending[k] = 0;
-        sh.iters[k] = 0;
-        sh.conv[k] = (k < M.nr && !P.fixed_iters && rr0 <= sh.thr2[k]) ? 1 : 0;
-        sh.active[k] = (k < M.nr && !sh.conv[k]) ? 1 : 0;
+    double v[NR + 2];
+    if (!sy.template reduce<NR + 2>(0, pb, mm2, v)) return;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < NR; k++) {
+            sh.bb[k] = P.x0_given ? bb0[k] : v[k];
+            sh.rr[k] = v[k];
+            sh.thr2[k] = P.tol * P.tol * sh.bb[k];
+            sh.beta[k] = 0.0;
+            sh.pending[k] = 0;
+            sh.iters[k] = 0;
+            sh.conv[k] = (k < M.nr && !P.fixed_iters && v[k] <= sh.thr2[k]) ? 1 : 0;
+            sh.active[k] = (k < M.nr && !sh.conv[k]) ? 1 : 0;
+        }
+        sh.brk = 0;
     }
-    if (threadIdx.x == 0) sh.brk = 0;
-    float invM = sh.bcast[NR] > 0.0 ? (float)(1.0 / sh.bcast[NR]) : 0.0f;
-    const double neg_mn0 = sh.bcast[NR + 1], mx0 = sh.bcast[NR];
     __syncthreads();
+    float invM = v[NR] > 0.0 ? (float)(1.0 / v[NR]) : 0.0f;
     // mixed: some tile may leave FP32 only if the smallest segment is below
     // demote_fp16 of the largest or lossless classes apply (see dyn in XVec)
     auto dyn_of = [&](double mx, double neg_mn) -> int {
         return (P.lossless_any || mx <= 0.0 || -neg_mn <= (double)P.demote16 * mx) ? 1 : 0;
     };
-    int dyn = dyn_of(mx0, neg_mn0);
+    int dyn = dyn_of(v[NR], v[NR + 1]);
     int k = 0, status = 0, repl = 0, last_true = 0;
+    double rt[NR];
+#pragma unroll
+    for (int j = 0; j < NR; j++) rt[j] = v[j];
 
     for (;;) {
         int any = 0;
@@ -401,16 +400,18 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
             for (int R = c.rbeg; R < c.rend; R++)
                 if (P.seg_ptr[R] == P.seg_ptr[R + 1]) upd_a(R, zw);
         }
-        if (!sy.template reduce<NR>(1, ppq, 0u)) return;
-        if (threadIdx.x < NR) {
-            const int j = threadIdx.x;
-            double a = sh.active[j] ? sh.rr[j] / sh.bcast[j] : 0.0;
-            if (!isfinite(a)) {          // breakdown of this column: it stops where it is
-                a = 0.0;
-                sh.active[j] = 0;
-                sh.brk = 1;
+        double pq[NR];
+        if (!sy.template reduce<NR>(1, ppq, 0u, pq)) return;
+        if (threadIdx.x == 0) {
+            for (int j = 0; j < NR; j++) {
+                double a = sh.active[j] ? sh.rr[j] / pq[j] : 0.0;
+                if (!isfinite(a)) {      // breakdown of this column: it stops where it is
+                    a = 0.0;
+                    sh.active[j] = 0;
+                    sh.brk = 1;
+                }
+                sh.alpha[j] = a;
             }
-            sh.alpha[j] = a;
         }
         __syncthreads();
         if (sh.brk) status = MF_ERR_BREAKDOWN;
@@ -444,19 +445,18 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
         }
         prr[NR] = st.mx;
         prr[NR + 1] = -st.mn;
-        if (!sy.template reduce<NR + 2>(2, prr, mm2)) return;
-        invM = sh.bcast[NR] > 0.0 ? (float)(1.0 / sh.bcast[NR]) : 0.0f;
-        dyn = dyn_of(sh.bcast[NR], sh.bcast[NR + 1]);
+        if (!sy.template reduce<NR + 2>(2, prr, mm2, v)) return;
+        invM = v[NR] > 0.0 ? (float)(1.0 / v[NR]) : 0.0f;
+        dyn = dyn_of(v[NR], v[NR + 1]);
         k++;
         last_true = 0;
         bool want_repl = P.replace_every > 0 && (k % P.replace_every) == 0;
 #pragma unroll
         for (int j = 0; j < NR; j++)
-            if (sh.active[j] && !P.fixed_iters && sh.bcast[j] <= sh.thr2[j]) want_repl = true;
-        // thread j: column j's recursive r.r, and its true one when that is formed
-        const double rrec = threadIdx.x < NR ? sh.bcast[threadIdx.x] : 0.0;
-        double rnew = rrec;
-        __syncthreads();                  // every thread has read `active` before column threads change it
+            if (sh.active[j] && !P.fixed_iters && v[j] <= sh.thr2[j]) want_repl = true;
+        double rnew[NR], rrec[NR];
+#pragma unroll
+        for (int j = 0; j < NR; j++) rnew[j] = rrec[j] = v[j];
         if (want_repl) {
             // ---- FP64 R = B - A X, R's shadow, true residual norms ----
             double prt[NR + 2];
@@ -490,27 +490,29 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
             }
             prt[NR] = st.mx;
             prt[NR + 1] = -st.mn;
-            if (!sy.template reduce<NR + 2>(5, prt, mm2)) return;
-            invM = sh.bcast[NR] > 0.0 ? (float)(1.0 / sh.bcast[NR]) : 0.0f;
-            dyn = dyn_of(sh.bcast[NR], sh.bcast[NR + 1]);
+            if (!sy.template reduce<NR + 2>(5, prt, mm2, v)) return;
+            invM = v[NR] > 0.0 ? (float)(1.0 / v[NR]) : 0.0f;
+            dyn = dyn_of(v[NR], v[NR + 1]);
             repl++;
             last_true = 1;
-            if (threadIdx.x < NR) {
-                rnew = sh.bcast[threadIdx.x];
-                sh.rt[threadIdx.x] = rnew;
+#pragma unroll
+            for (int j = 0; j < NR; j++) {
+                rt[j] = v[j];
+                rnew[j] = v[j];
             }
         }
-        if (threadIdx.x < NR) {
-            const int j = threadIdx.x;
-            if (sh.active[j] && last_true && !P.fixed_iters && rnew <= sh.thr2[j]) {
-                sh.active[j] = 0;            // converged on the FP64 true residual
-                sh.conv[j] = 1;
-                sh.iters[j] = k;
+        if (threadIdx.x == 0) {
+            for (int j = 0; j < NR; j++) {
+                if (sh.active[j] && last_true && !P.fixed_iters && rnew[j] <= sh.thr2[j]) {
+                    sh.active[j] = 0;            // converged on the FP64 true residual
+                    sh.conv[j] = 1;
+                    sh.iters[j] = k;
+                }
+                const bool restart = last_true &&
+                                     restart_after_replacement(!P.fixed_iters && rrec[j] <= sh.thr2[j], rnew[j], rrec[j]);
+                sh.beta[j] = (sh.active[j] && !restart) ? rnew[j] / sh.rr[j] : 0.0;
+                if (sh.active[j] || !sh.conv[j]) sh.rr[j] = rnew[j];
             }
-            const bool restart = last_true &&
-                                 restart_after_replacement(!P.fixed_iters && rrec <= sh.thr2[j], rnew, rrec);
-            sh.beta[j] = (sh.active[j] && !restart) ? rnew / sh.rr[j] : 0.0;
-            if (sh.active[j] || !sh.conv[j]) sh.rr[j] = rnew;
         }
         __syncthreads();
     }
@@ -536,16 +538,17 @@ __device__ void cg_multi_body(const SolverParams &P, const MultiParams &M, const
             for (int R = c.rbeg; R < c.rend; R++)
                 if (P.seg_ptr[R] == P.seg_ptr[R + 1]) acc_r(R, zy);
         }
-        if (!sy.template reduce<NR>(7, prt, 0u)) return;
-        if (threadIdx.x < NR) sh.rt[threadIdx.x] = sh.bcast[threadIdx.x];
-        __syncthreads();
+        double w[NR];
+        if (!sy.template reduce<NR>(7, prt, 0u, w)) return;
+#pragma unroll
+        for (int j = 0; j < NR; j++) rt[j] = w[j];
     }
     if (sy.writer()) {
         for (int j = 0; j < NR; j++) {
             const double bb = sh.bb[j];
             M.out[4 * j + 0] = (double)(sh.conv[j] ? sh.iters[j] : k);
             M.out[4 * j + 1] = (double)sh.conv[j];
-            M.out[4 * j + 2] = bb > 0 ? sqrt(sh.rt[j] / bb) : 0.0;
+            M.out[4 * j + 2] = bb > 0 ? sqrt(rt[j] / bb) : 0.0;
             M.out[4 * j + 3] = bb > 0 ? sqrt(sh.rr[j] / bb) : 0.0;
         }
         M.out[4 * NR + 0] = (double)k;
@@ -561,12 +564,11 @@ struct GridSync {
     SharedM &sh;
     unsigned epoch;
     template <int NV>
-    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask)
+    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask, double (&out)[NV])
     {
         block_partial_m<NV>(M, sh, kind, v, maxmask, (int)gridDim.x, (int)blockIdx.x);
         if (!grid_barrier(P, epoch, sh)) return false;
-        grid_collect_m<NV>(M, sh, kind, maxmask, (int)gridDim.x);
-        reduction_done();
+        grid_collect_m<NV>(M, sh, kind, maxmask, out, (int)gridDim.x);
         return true;
     }
     __device__ bool writer() const { return blockIdx.x == 0 && threadIdx.x == 0; }
@@ -651,9 +653,10 @@ struct BatchParams {
 struct BlockSync {
     SharedM &sh;
     template <int NV>
-    __device__ bool reduce(int, const double (&v)[NV], unsigned maxmask)
+    __device__ bool reduce(int, const double (&v)[NV], unsigned maxmask, double (&out)[NV])
     {
         const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+        __syncwarp();                      // as in block_partial_m
 #pragma unroll
         for (int k = 0; k < NV; k++) {
             double a = v[k];
@@ -677,7 +680,9 @@ struct BlockSync {
             if (lane == 0) sh.bcast[wib] = a;
         }
         __syncthreads();
-        reduction_done();
+#pragma unroll
+        for (int k = 0; k < NV; k++) out[k] = sh.bcast[k];
+        __syncthreads();
         return true;
     }
     __device__ bool writer() const { return threadIdx.x == 0; }
@@ -719,37 +724,28 @@ __device__ bool team_barrier(unsigned *ctr, unsigned k, unsigned &epoch, int *er
 // The synchronisation of a team item: block partials into the team's slots,
 // the team barrier, then every member sums the k partials in the same order.
 // The first barrier (every member arriving at the item) may wait for members
-// still finishing earlier list entries, so it gets the longer limit.  The
-// team's parameters live in shared memory (no registers held across the body).
-struct TeamShared {
-    double *red;
-    unsigned *ctr;
-    int *err;
-    unsigned long long limit_ns, arrive_ns;
-    int k, r;
-    unsigned epoch;
-    int stall;
-};
-
+// still finishing earlier list entries, so it gets the longer limit.  The team's
+// words are read from the item, which nothing writes during the launch: a warp
+// that lags cannot see another item's.
 struct TeamSync {
+    const BatchParams &B;
+    const BatchItem &it;
     SharedM &sh;
-    TeamShared &ts;
+    int r;                        // this block's rank in the team
+    unsigned epoch;
     template <int NV>
-    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask)
+    __device__ bool reduce(int kind, const double (&v)[NV], unsigned maxmask, double (&out)[NV])
     {
         MultiParams R;
-        R.red = ts.red;
-        block_partial_m<NV>(R, sh, kind, v, maxmask, ts.k, ts.r);
-        unsigned ep = ts.epoch;
-        const bool ok =
-            team_barrier(ts.ctr, (unsigned)ts.k, ep, ts.err, ep == 0 ? ts.arrive_ns : ts.limit_ns, sh, ts.stall);
-        if (!ok) return false;
-        grid_collect_m<NV>(R, sh, kind, maxmask, ts.k);
-        if (threadIdx.x == 0) ts.epoch = ep;
-        reduction_done();
+        R.red = it.M.red;
+        const int k = it.team;
+        block_partial_m<NV>(R, sh, kind, v, maxmask, k, r);
+        const unsigned long long limit = epoch == 0 ? B.arrive_timeout_ns : B.timeout_ns;
+        if (!team_barrier(it.ctr, (unsigned)k, epoch, B.err, limit, sh, B.stall_first)) return false;
+        grid_collect_m<NV>(R, sh, kind, maxmask, out, k);
         return true;
     }
-    __device__ bool writer() const { return ts.r == 0 && threadIdx.x == 0; }
+    __device__ bool writer() const { return r == 0 && threadIdx.x == 0; }
 };
 
 // The half-warps of a team of k blocks (this block: rank r) split a system's
@@ -836,11 +832,10 @@ __device__ __forceinline__ void item_solve(const SolverParams &P, const MultiPar
 // thread, the widest items without spills; 2: 64 registers, twice the warps to
 // hide latency, for items of up to 4 columns).  The tuner picks.
 template <int MODE, int LB>
-__global__ void __launch_bounds__(kThreads, LB) k_batch(BatchParams B)
+__global__ void __launch_bounds__(kThreads, LB) k_batch(const __grid_constant__ BatchParams B)
 {
     __shared__ SharedM sh;
-    __shared__ TeamShared ts;
-    __shared__ int next;
+    __shared__ int next, stop;
     // this block's team entries, in the global schedule order
     for (int e = B.bptr[blockIdx.x]; e < B.bptr[blockIdx.x + 1]; e++) {
         const int2 ent = B.blist[e];
@@ -849,27 +844,16 @@ __global__ void __launch_bounds__(kThreads, LB) k_batch(BatchParams B)
         const SolverParams P = item_params(it, B);
         const Ctx c = team_ctx(it, ent.y, it.team);
         const MultiParams M = it.M;
-        if (threadIdx.x == 0) {
-            ts.red = M.red;
-            ts.ctr = it.ctr;
-            ts.err = B.err;
-            ts.limit_ns = B.timeout_ns;
-            ts.arrive_ns = B.arrive_timeout_ns;
-            ts.k = it.team;
-            ts.r = ent.y;
-            ts.epoch = 0u;
-            ts.stall = B.stall_first;
-        }
-        __syncthreads();
         const unsigned long long t0 = mf_globaltimer();
-        TeamSync sy{sh, ts};
+        TeamSync sy{B, it, sh, ent.y, 0u};
         item_solve<MODE, (LB == 1 ? 8 : 4)>(P, M, it.nr, c, sh, sy);
+        if (threadIdx.x == 0) stop = *(volatile int *)B.err;
         __syncthreads();
         if (ent.y == 0 && threadIdx.x == 0) {         // the item's start and end, for the report
             M.out[4 * it.nr + 3] = (double)t0;
             M.out[4 * it.nr + 4] = (double)mf_globaltimer();
         }
-        if (*(volatile int *)B.err) return;      // a team wait gave up: the launch reports it
+        if (stop) return;      // a team wait gave up: the launch reports it (one answer for the whole block)
     }
     for (;;) {
         if (threadIdx.x == 0) next = (int)atomicAdd(B.head, 1u);
