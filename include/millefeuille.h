@@ -401,6 +401,11 @@ int mf_debug_spmm(mf_matrix A, const double *X, double *Y, int tensor_cores, int
  * nseg <= max(tilem, tilen).  Undefined after solves in the other precisions. */
 int mf_debug_solver_labels(mf_matrix A, int *vis, int nseg);
 
+/* Test hook: bytes of the largest global-memory scratch a launch of A's tile
+ * build took (0: all of it in shared memory), or -1 for a null handle.
+ * No counterpart in the reference. */
+long long mf_debug_build_scratch(mf_matrix A);
+
 /* Test hook: the full report (mf_report) of the calling thread's last
  * drop-in solve (cg_solve_inc / _sync / _reduce, bicgstab / _sync / _inc), so a
  * caller of the reference's entry points can see which precision ran

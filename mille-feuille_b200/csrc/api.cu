@@ -529,6 +529,8 @@ extern "C" int mf_debug_spmm(mf_matrix A, const double *X, double *Y, int tensor
     return rc;
 }
 
+extern "C" long long mf_debug_build_scratch(mf_matrix A) { return A ? A->build_scratch : -1; }
+
 extern "C" int mf_debug_solver_labels(mf_matrix A, int *vis, int nseg)
 {
     if (!A || (nseg > 0 && !vis)) return MF_ERR_INVALID;

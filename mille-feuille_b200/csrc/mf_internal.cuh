@@ -93,6 +93,7 @@ struct mf_matrix_s {
     // tile-row ownership cost prefix for partitioning: [tilem+1]
     long long *d_row_cost;
     double build_ms;
+    long long build_scratch;   // largest global-memory scratch of a launch of the tile build, bytes
     // cached solver workspace
     void *ws;
     size_t ws_bytes;

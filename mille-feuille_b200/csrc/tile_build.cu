@@ -70,7 +70,28 @@ __global__ void k_span(const int *__restrict__ rowptr, const int *__restrict__ c
     }
 }
 
-// A warp's scratch, in shared memory or (wide spans, many tiles) in global memory.
+// ---- scratch of the per-tile-row kernels ----
+// k_count_tiles needs a bitmap over the tile-row's span, k_fill_tiles what
+// fill_words says.  One tile-row that touches every column tile (an arrow matrix,
+// a circuit's supply net) needs 17 words per tile: sized for it, the 4,736 warps
+// of a launch took 20 GB at 1 M columns.  So tile-rows are sorted by what they
+// need into three passes: up to kSharedWords in shared memory (the launch covers
+// all tile-rows and leaves out the others), up to kMidWords in global memory with
+// the full grid, and the rest with as many warps as kScratchBytes gives.
+constexpr int kSharedWords = 96 * 1024 / 4 / kWarps;
+constexpr int kGlobalGrid = 148 * 4;
+constexpr long long kScratchBytes = 256ll << 20;
+constexpr int kMidWords = (int)(kScratchBytes / 4 / kWarps / kGlobalGrid);
+
+// bitmap, prefix (a word per span word each), next position per tile, entries per (tile, row)
+__host__ __device__ constexpr int fill_words(int span, int tiles) { return 2 * span + (1 + MF_BS) * tiles; }
+
+// What k_count_tiles finds out about the passes; rows: the mid ones from the front, the large ones from the back.
+struct Passes {
+    int shared_words, mid_words, large_words, n_mid, n_large;
+};
+
+// A warp's scratch, in shared memory or in global memory.
 __device__ __forceinline__ unsigned int *warp_scratch(unsigned int *smem, unsigned int *gscratch, int words_per_warp,
                                                       int global_mode)
 {
@@ -96,10 +117,11 @@ __device__ int build_bitmap(unsigned int *bm, const int *__restrict__ colidx, in
     return cnt;
 }
 
-// ---- K1: distinct tiles per tile-row, and the most of any ----
+// ---- K1: distinct tiles per tile-row, and the pass that fills it ----
 __global__ void k_count_tiles(const int *__restrict__ rowptr, const int *__restrict__ colidx, int tilem, int rowA,
                               const int2 *__restrict__ spans, int words_per_warp, int global_mode,
-                              unsigned int *gscratch, int *__restrict__ ntiles, int *__restrict__ max_tiles)
+                              unsigned int *gscratch, int *__restrict__ ntiles, int *__restrict__ rows,
+                              Passes *__restrict__ passes)
 {
     extern __shared__ unsigned int smem[];
     const int lane = threadIdx.x & 31;
@@ -112,24 +134,32 @@ __global__ void k_count_tiles(const int *__restrict__ rowptr, const int *__restr
         const int c = (sp.y > 0) ? build_bitmap(bm, colidx, a, b, sp.x, sp.y, lane) : 0;
         if (lane == 0) {
             ntiles[R] = c;
-            if (c > *(volatile int *)max_tiles) atomicMax(max_tiles, c);
+            const int need = fill_words(sp.y, c);
+            if (need <= kSharedWords) {
+                if (need > *(volatile int *)&passes->shared_words) atomicMax(&passes->shared_words, need);
+            } else if (need <= kMidWords) {
+                rows[atomicAdd(&passes->n_mid, 1)] = R;
+                atomicMax(&passes->mid_words, need);
+            } else {
+                rows[tilem - 1 - atomicAdd(&passes->n_large, 1)] = R;
+                atomicMax(&passes->large_words, need);
+            }
         }
         __syncwarp();
     }
 }
 
 // ---- K2: tile columns, payload offsets, scatter, uint8 row starts ----
-// Scratch per warp: bitmap[span], prefix[span], next payload position[max_tiles],
-// entries per (tile, row)[16 max_tiles].  Entries are taken 32 at a time across
+// `rows` lists the `nrows` tile-rows of a launch; without it the launch takes all
+// whose scratch fits words_per_warp.  Entries are taken 32 at a time across
 // the rows of the tile-row (CSR order is row by row already): 7-point tile-rows
 // are 4 steps a pass, where going row by row made 16 with two warp barriers each
 // (128^3: 0.84 ms of 2 ms of kernels).  The row starts come from the (tile, row)
-// counts.  max_tiles is counted, not bounded by the span: irregular matrices with
-// wide spans stay in shared memory.
+// counts.
 __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restrict__ colidx,
                              const double *__restrict__ val, const float *__restrict__ val_low, int tilem,
-                             int rowA, const int2 *__restrict__ spans, int span, int max_tiles, int words_per_warp,
-                             int global_mode, unsigned int *gscratch, const int *__restrict__ tile_ptr,
+                             int rowA, const int2 *__restrict__ spans, const int *__restrict__ rows, int nrows,
+                             int words_per_warp, int global_mode, unsigned int *gscratch, const int *__restrict__ tile_ptr,
                              int *__restrict__ tile_columnidx, int *__restrict__ csr_offset,
                              int *__restrict__ csrptr_offset, double *__restrict__ tval,
                              float *__restrict__ tval_low, unsigned char *__restrict__ tcol,
@@ -141,14 +171,17 @@ __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restri
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
     unsigned int *bm = warp_scratch(smem, gscratch, words_per_warp, global_mode);
-    int *pre = (int *)bm + span, *next = pre + span, *hist = next + max_tiles;
     const int nz0 = rowptr[0];
-    for (int R = warp; R < tilem; R += nwarps) {
+    for (int q = warp; q < nrows; q += nwarps) {
+        const int R = rows ? rows[q] : q;
         const int rs = R * MF_BS, re = tile_row_end(R, tilem, rowA);
         const int rowlen = re - rs;
         const int rp = lane <= rowlen ? rowptr[rs + lane] : INT_MAX;
         const int a = __shfl_sync(0xffffffffu, rp, 0), b = __shfl_sync(0xffffffffu, rp, rowlen);
         const int t0 = tile_ptr[R], nt = tile_ptr[R + 1] - t0;
+        const int base_word = spans[R].x, words = spans[R].y;
+        if (fill_words(words, nt) > words_per_warp) continue;      // another pass fills it
+        int *pre = (int *)bm + words, *next = pre + words, *hist = next + nt;
         // csrptr_offset: exclusive scan of tile-row heights over tiles (csr2block.h:146,347)
         for (int s = lane; s < nt; s += 32) csrptr_offset[t0 + s] = t0 * MF_BS + s * rowlen;
         if (R == tilem - 1 && lane == 0) csrptr_offset[t0 + nt] = t0 * MF_BS + nt * rowlen;
@@ -156,7 +189,6 @@ __global__ void k_fill_tiles(const int *__restrict__ rowptr, const int *__restri
             if (R == tilem - 1 && lane == 0) csr_offset[t0] = b - nz0;
             continue;
         }
-        const int base_word = spans[R].x, words = spans[R].y;
         for (int h = lane; h < nt * MF_BS; h += 32) hist[h] = 0;
         build_bitmap(bm, colidx, a, b, base_word, words, lane);
         // exclusive popcount prefix over the bitmap words
@@ -577,7 +609,8 @@ namespace {
 
 // The numbers the host waits for, gathered on the device and read in one copy.
 struct Counts {
-    int err, span, max_tiles;                       // written by the kernels as they go
+    int err, span;                                  // written by the kernels as they go
+    Passes passes;
     int longest, not_one_chunk;                     // k_seg_shape
     int tilenum, last_tile0, rowblocks, nseg, nz_lo, nz_hi;
     int nonempty;
@@ -623,10 +656,11 @@ int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
     Temps tmp{s, {}};
     Counts *d_c = nullptr, c;
     int2 *d_spans = nullptr;
-    int *d_ntiles = nullptr, *d_rbo = nullptr;
+    int *d_ntiles = nullptr, *d_rbo = nullptr, *d_rows = nullptr;
     MF_TRY(tmp.get(&d_c, 1));
     MF_TRY(tmp.get(&d_spans, tilem));
     MF_TRY(tmp.get(&d_ntiles, tilem));
+    MF_TRY(tmp.get(&d_rows, tilem));
     MF_TRY(tmp.get(&d_rbo, (long long)tilem + 1));
     MF_TRY(dalloc(&A->d_tile_ptr, (long long)tilem + 1, s));
     MF_TRY(dalloc(&A->d_seg_ptr, (long long)tilem + 1, s));
@@ -637,21 +671,25 @@ int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
                                           &d_c->err);
     MF_TRY(read_counts(&c, d_c, s));
 
+    if ((long long)tilen >= (1LL << 23)) return MF_ERR_UNSUPPORTED;   // column tile must fit 23 bits
     const int span = std::max(c.span, 1);
-    const size_t smem_cap = 96 * 1024;
-    // a kernel's scratch: shared memory up to smem_cap, else global memory and a smaller grid
+    // a launch's scratch: shared memory up to kSharedWords a warp, else global memory within
+    // kScratchBytes (one block at least) for `rows` tile-rows, a warp each
     struct Scratch {
         int words, global_mode, grid;
         size_t smem;
         unsigned int *global;
     };
-    auto scratch = [&](const void *kernel, long long words, Scratch *x) -> int {
-        *x = {(int)words, 0, wgrid, (size_t)words * 4 * kWarps, nullptr};
-        if (x->smem > smem_cap) {
+    auto scratch = [&](const void *kernel, int words, long long rows, Scratch *x) -> int {
+        *x = {words, 0, grid_for(rows * 32, kThreads), (size_t)words * 4 * kWarps, nullptr};
+        if (words > kSharedWords) {
+            const long long fit = std::max(1LL, kScratchBytes / 4 / kWarps / words);
             x->global_mode = 1;
             x->smem = 0;
-            x->grid = std::min(wgrid, 148 * 4);
-            MF_TRY(tmp.get(&x->global, words * (long long)x->grid * kWarps));
+            x->grid = (int)std::min<long long>(std::min(x->grid, kGlobalGrid), fit);
+            const long long total = (long long)words * x->grid * kWarps;
+            MF_TRY(tmp.get(&x->global, total));
+            A->build_scratch = std::max(A->build_scratch, total * 4);
         } else if (x->smem > 48 * 1024) {
             MF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x->smem));
         }
@@ -659,9 +697,9 @@ int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
     };
     if (tilem > 0) {
         Scratch x;
-        MF_TRY(scratch((const void *)k_count_tiles, span, &x));
+        MF_TRY(scratch((const void *)k_count_tiles, span, tilem, &x));
         k_count_tiles<<<x.grid, kThreads, x.smem, s>>>(A->d_rowptr, A->d_colidx, tilem, rowA, d_spans, x.words,
-                                                       x.global_mode, x.global, d_ntiles, &d_c->max_tiles);
+                                                       x.global_mode, x.global, d_ntiles, d_rows, &d_c->passes);
         MF_CUDA_TRY(cudaGetLastError());
     }
     MF_TRY(mf_scan_tile_counts(d_ntiles, A->d_tile_ptr, d_rbo, A->d_seg_ptr, tilem, s));
@@ -713,14 +751,21 @@ int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
         MF_CUDA_TRY(cudaMemsetAsync(A->d_csr_offset, 0, sizeof(int), s));
         MF_CUDA_TRY(cudaMemsetAsync(A->d_csrptr_offset, 0, sizeof(int), s));
     } else {
-        Scratch x;
-        MF_TRY(scratch((const void *)k_fill_tiles, 2LL * span + (1LL + MF_BS) * std::max(c.max_tiles, 1), &x));
-        k_fill_tiles<<<x.grid, kThreads, x.smem, s>>>(A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, tilem, rowA,
-                                                      d_spans, span, std::max(c.max_tiles, 1), x.words, x.global_mode,
-                                                      x.global, A->d_tile_ptr, A->d_tile_columnidx, A->d_csr_offset,
-                                                      A->d_csrptr_offset, A->d_tval, A->d_tval_low, A->d_tcol,
-                                                      A->d_tptr, &d_c->err);
-        MF_CUDA_TRY(cudaGetLastError());
+        const Passes &ps = c.passes;
+        auto fill = [&](int words, const int *rows, int nrows) -> int {
+            Scratch x;
+            MF_TRY(scratch((const void *)k_fill_tiles, words, nrows, &x));
+            k_fill_tiles<<<x.grid, kThreads, x.smem, s>>>(A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, tilem,
+                                                          rowA, d_spans, rows, nrows, x.words, x.global_mode, x.global,
+                                                          A->d_tile_ptr, A->d_tile_columnidx, A->d_csr_offset,
+                                                          A->d_csrptr_offset, A->d_tval, A->d_tval_low, A->d_tcol,
+                                                          A->d_tptr, &d_c->err);
+            MF_CUDA_TRY(cudaGetLastError());
+            return MF_SUCCESS;
+        };
+        MF_TRY(fill(ps.shared_words, nullptr, tilem));
+        if (ps.n_mid > 0) MF_TRY(fill(ps.mid_words, d_rows, ps.n_mid));
+        if (ps.n_large > 0) MF_TRY(fill(ps.large_words, d_rows + tilem - ps.n_large, ps.n_large));
         // nonempty-row lists, solver-slice shapes
         k_rowlist_count<<<wgrid, kThreads, 0, s>>>(A->d_tile_ptr, A->d_csr_offset, A->d_csrptr_offset, A->d_tptr,
                                                    tilem, rowA, d_nzr, A->d_tile_rowidx, A->d_block_signal);
@@ -752,7 +797,6 @@ int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
     A->slice_entries = ent;
     A->max_row = c.longest;
     A->one_chunk = tilem > 0 && c.not_one_chunk == 0 ? 1 : 0;
-    if ((long long)A->tilen >= (1LL << 23)) return MF_ERR_UNSUPPORTED;   // column tile must fit 23 bits
     if ((ent >> 7) >= (1LL << 31)) return MF_ERR_UNSUPPORTED;
     MF_TRY(dalloc(&A->d_blockrowid_new, (long long)cnt + 1, s));
     MF_TRY(dalloc(&A->d_blockcsr_ptr_new, (long long)cnt + 1, s));

@@ -77,7 +77,7 @@ EXPORTED = [
     "mf_solve_multi", "mf_batch_create", "mf_batch_tune", "mf_batch_configure", "mf_batch_config",
     "mf_batch_solve", "mf_batch_destroy",
     "mf_batch_partition", "mf_batch_schedule", "mf_debug_spmv_tiles", "mf_debug_solver_labels",
-    "mf_dropin_last_report", "mf_debug_spmm",
+    "mf_dropin_last_report", "mf_debug_spmm", "mf_debug_build_scratch",
 ]
 
 _lib = None
@@ -118,6 +118,8 @@ def load() -> C.CDLL:
     L.mf_debug_ref_labels.argtypes = [vp, vp, C.c_int, vp, C.c_int]
     L.mf_debug_spmv_tiles.argtypes = [vp, vp, vp, C.c_int, C.c_int]
     L.mf_debug_solver_labels.argtypes = [vp, vp, C.c_int]
+    L.mf_debug_build_scratch.argtypes = [vp]
+    L.mf_debug_build_scratch.restype = C.c_longlong
     L.mf_dropin_last_report.argtypes = [C.POINTER(Report)]
     L.mf_debug_spmm.argtypes = [vp, vp, vp, C.c_int, C.c_int, dp]
     L.mf_read_matrix.argtypes = [C.c_char_p, ip, ip, ip, C.POINTER(ip), C.POINTER(ip), C.POINTER(dp), ip]

@@ -81,6 +81,36 @@ def test_gpu_tiles_wide_span_global_scratch(mf, oracle_mod, cuda):
     _check_against_oracle(mf, oracle_mod, n, ncols, rowptr, colidx, val)
 
 
+def _long_rows(n, rows, rng):
+    """The unit diagonal, and for each (row, k) of `rows` k columns spread over the matrix."""
+    cols = [np.array([i]) for i in range(n)]
+    for r, k in rows:
+        cols[r] = np.unique(np.concatenate([[r], np.linspace(0, n - 1, k).astype(np.int64)]))
+        rng.shuffle(cols[r])
+    rowptr = np.concatenate([[0], np.cumsum([c.size for c in cols])]).astype(np.int32)
+    colidx = np.concatenate(cols).astype(np.int32)
+    return rowptr, colidx, rng.standard_normal(colidx.size)
+
+
+@pytest.mark.parametrize("n,rows", [
+    (20000, [(7777, 20000)]),                                     # one full row: more than a launch of all warps gets
+    (20003, [(5, 400), (9000, 700), (9001, 3), (20001, 20003)]),  # three kinds, the short last tile-row among them
+    (3000, [(100, 3000)]),                                        # 188 tiles: just past shared memory
+    (2700, [(100, 2700)]),                                        # 169 tiles: just within it
+    (1000000, [(333333, 1000000)]),
+])
+def test_gpu_tiles_long_rows_have_bounded_scratch(mf, oracle_mod, cuda, n, rows):
+    """Tile-rows with many tiles are filled in passes of their own, in at most 256 MB
+    of scratch (one warp per tile-row of the grid sized for the longest took 20 GB at
+    a million columns)."""
+    from millefeuille import _lib
+    rowptr, colidx, val = _long_rows(n, rows, np.random.default_rng(n))
+    G, _, _ = _check_against_oracle(mf, oracle_mod, n, n, rowptr, colidx, val)
+    scratch = _lib.load().mf_debug_build_scratch(G._h)
+    assert scratch <= 256 << 20, scratch
+    assert (scratch == 0) == (n == 2700)
+
+
 def test_gpu_tiles_from_device_pointers(mf, oracle_mod, cuda):
     import torch
     from millefeuille import matrices as M
