@@ -8,6 +8,7 @@
 // No counterpart in the reference, which has no differentiation.
 #include "mf_internal.cuh"
 
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -88,6 +89,12 @@ constexpr int kTRounds = 16;                         // 32-entry rounds per warp
 constexpr int kTTile = kTThreads * kTRounds;         // entries per block: each warp takes a contiguous run
 constexpr int kDigits = 256;
 
+// A handle has up to 2^31 - 1 entries, so counts and midpoints near that stay in range.
+__host__ __device__ constexpr int sort_blocks(int n) { return (int)(((long long)n + kTTile - 1) / kTTile); }
+__host__ __device__ constexpr int midpoint(int lo, int hi) { return lo + ((hi - lo) >> 1); }
+static_assert(sort_blocks(2147483647) == 524288 && sort_blocks(0) == 0 && sort_blocks(kTTile + 1) == 2, "");
+static_assert(midpoint(2147483640, 2147483646) == 2147483643 && midpoint(0, 1) == 0, "");
+
 // rowptr -> the row of every entry (entries counted from row 0's first)
 __global__ void k_entry_rows(const int *__restrict__ rowptr, int n_rows, int *__restrict__ row)
 {
@@ -154,10 +161,11 @@ __global__ void k_digit_scatter(const int *__restrict__ key, const int *__restri
 // row pointers of A^T from the sorted columns: row j starts at the first entry of column >= j
 __global__ void k_sorted_rowptr(const int *__restrict__ key, int n, int n_cols, int *__restrict__ tp)
 {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= n_cols; j += gridDim.x * blockDim.x) {
+    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j <= n_cols;
+         j += (long long)gridDim.x * blockDim.x) {
         int lo = 0, hi = n;
         while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
+            const int mid = midpoint(lo, hi);
             if (key[mid] < j) lo = mid + 1;
             else hi = mid;
         }
@@ -177,6 +185,7 @@ __global__ void k_gather_entries(const int *__restrict__ pos, int n, const int *
     }
 }
 
+// Pool arrays freed in stream order: by name once they are done with, the rest at the end.
 struct PoolTemps {
     cudaStream_t s;
     std::vector<void *> all;
@@ -187,15 +196,21 @@ struct PoolTemps {
         if (rc == MF_SUCCESS) all.push_back(*p);
         return rc;
     }
-    ~PoolTemps()
+    void free_all()
     {
         for (void *p : all) mf_pool_free(p, s);
+        all.clear();
     }
+    ~PoolTemps() { free_all(); }
 };
 
 }  // namespace
 
-// A handle for A^T, built from A's device CSR copy without leaving the GPU.
+// A handle for A^T, built from A's device CSR copy without leaving the GPU, on the
+// current device as mf_matrix_create does.  Its CSR arrays become the new handle's
+// and the sort's temporaries are freed before the tile build, so the call needs no
+// more device memory than the handle: at most 36 bytes an entry at a time here,
+// where the build goes past 46.
 extern "C" int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *stream)
 {
     if (!out || !A) return MF_ERR_INVALID;
@@ -205,21 +220,37 @@ extern "C" int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *st
     int base = 0;                   // entries of rows [0, m) start here
     MF_CUDA_TRY(cudaMemcpyAsync(&base, A->d_rowptr, sizeof(int), cudaMemcpyDeviceToHost, s));
     MF_CUDA_TRY(cudaStreamSynchronize(s));
-    const int *colidx = A->d_colidx + base;
-    const int nblocks = (nnz + kTTile - 1) / kTTile;
-    PoolTemps tmp{s, {}};
+    PoolTemps tmp{s, {}}, csr{s, {}};
+    const int *rowptr = A->d_rowptr, *colidx = A->d_colidx + base;
+    const double *val = A->d_val + base;
+    const float *low = A->d_val_low ? A->d_val_low + base : nullptr;
+    int rc = MF_SUCCESS, dev = 0;
+    MF_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev != A->dev) {            // kernels do not read another device's memory
+        auto fetch = [&](auto **p, long long count) -> int {
+            using T = std::remove_const_t<std::remove_reference_t<decltype(**p)>>;
+            T *here = nullptr;
+            const int e = tmp.get(&here, count);
+            if (e != MF_SUCCESS) return e;
+            MF_CUDA_TRY(cudaMemcpyAsync(here, *p, (size_t)count * sizeof(T), cudaMemcpyDeviceToDevice, s));
+            *p = here;
+            return MF_SUCCESS;
+        };
+        if ((rc = fetch(&rowptr, (long long)m + 1)) || (rc = fetch(&colidx, nnz)) || (rc = fetch(&val, nnz)) ||
+            (low && (rc = fetch(&low, nnz))))
+            return rc;
+    }
+    const int nblocks = sort_blocks(nnz);
     int *row, *key[2], *pos[2], *hist, *start, *tp, *tc;
     double *tv;
     float *tl = nullptr;
-    int rc = MF_SUCCESS;
-    if ((rc = tmp.get(&row, nnz)) || (rc = tmp.get(&key[0], nnz)) || (rc = tmp.get(&key[1], nnz)) ||
-        (rc = tmp.get(&pos[0], nnz)) || (rc = tmp.get(&pos[1], nnz)) ||
-        (rc = tmp.get(&hist, (long long)kDigits * nblocks)) || (rc = tmp.get(&start, (long long)kDigits * nblocks + 1)) ||
-        (rc = tmp.get(&tp, (long long)n + 1)) || (rc = tmp.get(&tc, nnz)) || (rc = tmp.get(&tv, nnz)) ||
-        (A->d_val_low && (rc = tmp.get(&tl, nnz))))
+    if ((rc = csr.get(&tp, (long long)n + 1)) || (rc = csr.get(&tc, nnz)) || (rc = csr.get(&tv, nnz)) ||
+        (low && (rc = csr.get(&tl, nnz))) || (rc = tmp.get(&row, nnz)) || (rc = tmp.get(&key[0], nnz)) ||
+        (rc = tmp.get(&key[1], nnz)) || (rc = tmp.get(&pos[0], nnz)) || (rc = tmp.get(&pos[1], nnz)) ||
+        (rc = tmp.get(&hist, (long long)kDigits * nblocks)) || (rc = tmp.get(&start, (long long)kDigits * nblocks + 1)))
         return rc;
     if (nnz > 0) {
-        k_entry_rows<<<148 * 8, 256, 0, s>>>(A->d_rowptr, m, row);
+        k_entry_rows<<<148 * 8, 256, 0, s>>>(rowptr, m, row);
         MF_CUDA_TRY(cudaGetLastError());
         const int *kin = colidx, *pin = nullptr;
         int at = 0;
@@ -233,13 +264,14 @@ extern "C" int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *st
             kin = key[at];
             pin = pos[at];
         }
-        k_sorted_rowptr<<<(n + 256) / 256, 256, 0, s>>>(kin, nnz, n, tp);
+        k_sorted_rowptr<<<(unsigned)(((long long)n + 256) / 256), 256, 0, s>>>(kin, nnz, n, tp);
         MF_CUDA_TRY(cudaGetLastError());
-        k_gather_entries<<<148 * 8, 256, 0, s>>>(pin, nnz, row, A->d_val + base,
-                                                 A->d_val_low ? A->d_val_low + base : nullptr, tc, tv, tl);
+        k_gather_entries<<<148 * 8, 256, 0, s>>>(pin, nnz, row, val, low, tc, tv, tl);
         MF_CUDA_TRY(cudaGetLastError());
     } else {
         MF_CUDA_TRY(cudaMemsetAsync(tp, 0, ((size_t)n + 1) * sizeof(int), s));
     }
-    return mf_matrix_create(out, n, m, nnz, tp, tc, tv, tl, 1, stream);
+    tmp.free_all();
+    csr.all.clear();                // the handle's from here on, also when the build fails
+    return mf_matrix_adopt(out, n, m, nnz, tp, tc, tv, tl, s);
 }

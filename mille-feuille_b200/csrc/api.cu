@@ -136,6 +136,20 @@ int stage_get(mf_matrix_s *A, size_t bytes, double **out, cudaStream_t s)
     return MF_SUCCESS;
 }
 
+// An empty handle on the current device.
+int new_matrix(mf_matrix_s **out, int n_rows, int n_cols)
+{
+    int dev = 0;
+    MF_CUDA_TRY(cudaGetDevice(&dev));
+    mf_matrix_s *A = new mf_matrix_s();
+    memset(A, 0, sizeof(*A));
+    A->dev = dev;
+    A->n_rows = n_rows;
+    A->n_cols = n_cols;
+    *out = A;
+    return MF_SUCCESS;
+}
+
 int device_ready()
 {
     int nd = 0;
@@ -159,11 +173,8 @@ extern "C" int mf_matrix_create(mf_matrix *out, int n_rows, int n_cols, long lon
     *out = nullptr;
     MF_TRY(device_ready());
     cudaStream_t s = (cudaStream_t)stream;
-    mf_matrix_s *A = new mf_matrix_s();
-    memset(A, 0, sizeof(*A));
-    MF_CUDA_TRY(cudaGetDevice(&A->dev));
-    A->n_rows = n_rows;
-    A->n_cols = n_cols;
+    mf_matrix_s *A = nullptr;
+    MF_TRY(new_matrix(&A, n_rows, n_cols));
     const cudaMemcpyKind kind = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     int rc = MF_SUCCESS;
     auto fail = [&](int code) { free_matrix(A); return code; };
@@ -180,6 +191,31 @@ extern "C" int mf_matrix_create(mf_matrix *out, int n_rows, int n_cols, long lon
         return fail(MF_ERR_CUDA);
     rc = mf_build_tiles(A, nnz, s);
     if (rc != MF_SUCCESS) return fail(rc);
+    *out = A;
+    return MF_SUCCESS;
+}
+
+// A handle around CSR arrays that already are in pool memory of the current device.
+// They belong to it from here on, also when the build fails.
+int mf_matrix_adopt(mf_matrix *out, int n_rows, int n_cols, long long nnz, int *rowptr, int *colidx, double *val,
+                    float *val_low, cudaStream_t s)
+{
+    mf_matrix_s *A = nullptr;
+    int rc = new_matrix(&A, n_rows, n_cols);
+    if (rc != MF_SUCCESS) {
+        void *all[] = {rowptr, colidx, val, val_low};
+        for (void *p : all) mf_pool_free(p, s);
+        return rc;
+    }
+    A->d_rowptr = rowptr;
+    A->d_colidx = colidx;
+    A->d_val = val;
+    A->d_val_low = val_low;
+    rc = mf_build_tiles(A, nnz, s);
+    if (rc != MF_SUCCESS) {
+        free_matrix(A);
+        return rc;
+    }
     *out = A;
     return MF_SUCCESS;
 }

@@ -161,6 +161,9 @@ int mf_scan_tile_counts(const int *d_ntiles, int *d_tile_ptr, int *d_rb_ptr, int
 
 // tile build (tile_build.cu); nnz: entries of the caller's arrays
 int mf_build_tiles(mf_matrix_s *A, long long nnz, cudaStream_t s);
+// a handle that takes over CSR arrays in pool memory (api.cu)
+int mf_matrix_adopt(mf_matrix *out, int n_rows, int n_cols, long long nnz, int *rowptr, int *colidx, double *val,
+                    float *val_low, cudaStream_t s);
 
 // solver (solver.cu)
 int mf_solver_run(mf_matrix_s *A, const double *d_b, double *d_x, const mf_options *opt,
