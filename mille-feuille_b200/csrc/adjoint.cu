@@ -41,6 +41,7 @@ extern "C" int mf_value_grad(mf_matrix A, int nrhs, const double *lambda, const 
                              int device_ptrs, void *stream)
 {
     if (!A || !lambda || !x || !grad_val || nrhs < 1) return MF_ERR_INVALID;
+    CallMark mark(A);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t nl = (size_t)nrhs * A->n_rows, nx = (size_t)nrhs * A->n_cols, ne = (size_t)A->nnz;
     const double *dl = lambda, *dx = x;
@@ -66,7 +67,7 @@ extern "C" int mf_value_grad(mf_matrix A, int nrhs, const double *lambda, const 
         mf_pool_free(tmp, s);
     }
     MF_CUDA_TRY(cudaStreamSynchronize(s));
-    return MF_SUCCESS;
+    return mark.end(MF_SUCCESS);
 }
 
 // ------------------------------------------------------------ A^T on the GPU
@@ -215,6 +216,7 @@ extern "C" int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *st
 {
     if (!out || !A) return MF_ERR_INVALID;
     *out = nullptr;
+    CallMark mark(A);
     cudaStream_t s = (cudaStream_t)stream;
     const int m = A->n_rows, n = A->n_cols, nnz = (int)A->nnz;
     int base = 0;                   // entries of rows [0, m) start here
@@ -273,5 +275,5 @@ extern "C" int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *st
     }
     tmp.free_all();
     csr.all.clear();                // the handle's from here on, also when the build fails
-    return mf_matrix_adopt(out, n, m, nnz, tp, tc, tv, tl, s);
+    return mark.end(mf_matrix_adopt(out, n, m, nnz, tp, tc, tv, tl, s));
 }

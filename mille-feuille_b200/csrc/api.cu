@@ -93,13 +93,10 @@ void mf_free_host(void *p) { free(p); }
 // ------------------------------------------------------------------ matrices
 namespace {
 
-// Work on any stream may still use the handle's arrays, so the device is
-// synchronised first (as cudaFree does); the frees themselves are then
-// stream-ordered on an idle device.
 void free_matrix(mf_matrix_s *A)
 {
     MfDeviceGuard guard(A->dev);
-    if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+    mf_handle_wait(A);
     mf_solver_free_ws(A);
     void *ptrs[] = {A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, A->d_tile_ptr, A->d_tile_columnidx,
                     A->d_csr_offset, A->d_csrptr_offset, A->d_tval, A->d_tval_low, A->d_tcol, A->d_tptr,
@@ -107,9 +104,8 @@ void free_matrix(mf_matrix_s *A)
                     A->d_blockcsr_ptr_new, A->d_rb_idx, A->d_rb_start, A->d_rb_stop, A->d_val_f16,
                     A->d_val_i8_ref, A->d_val_i8, A->d_i8_scale, A->d_tile_caps, A->d_seg_ptr, A->d_seg_tile0,
                     A->d_seg_off, A->d_seg_hdr, A->d_seg_tile, A->d_seg_kp, A->d_seg_rowlen, A->d_meta, A->d_v64, A->d_v32, A->d_v16,
-                    A->d_v8, A->d_v8ref, A->d_row_cost};
-    for (void *p : ptrs) mf_pool_free(p, 0);
-    mf_pool_free(A->stage, 0);
+                    A->d_v8, A->d_v8ref, A->d_row_cost, A->stage};
+    mf_pool_give_back(ptrs, (int)(sizeof(ptrs) / sizeof(ptrs[0])));
     for (cudaEvent_t e : A->spmv_ev)
         if (e) cudaEventDestroy(e);
     mf_pool_settle(A->dev);
@@ -124,8 +120,8 @@ int stage_get(mf_matrix_s *A, size_t bytes, double **out, cudaStream_t s)
 {
     if (A->stage_bytes < bytes) {
         if (A->stage) {
-            MF_CUDA_TRY(cudaDeviceSynchronize());   // a call on another stream may still read it
-            mf_pool_free(A->stage, 0);
+            mf_handle_wait(A);
+            mf_pool_give_back(&A->stage, 1);
         }
         A->stage = nullptr;
         A->stage_bytes = 0;
@@ -177,7 +173,11 @@ extern "C" int mf_matrix_create(mf_matrix *out, int n_rows, int n_cols, long lon
     MF_TRY(new_matrix(&A, n_rows, n_cols));
     const cudaMemcpyKind kind = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     int rc = MF_SUCCESS;
-    auto fail = [&](int code) { free_matrix(A); return code; };
+    auto fail = [&](int code) {
+        A->unsynced = 1;
+        free_matrix(A);
+        return code;
+    };
     if ((rc = mf_pool_array(&A->d_rowptr, (long long)n_rows + 1, s)) != MF_SUCCESS ||
         (rc = mf_pool_array(&A->d_colidx, nnz, s)) != MF_SUCCESS ||
         (rc = mf_pool_array(&A->d_val, nnz, s)) != MF_SUCCESS)
@@ -213,6 +213,7 @@ int mf_matrix_adopt(mf_matrix *out, int n_rows, int n_cols, long long nnz, int *
     A->d_val_low = val_low;
     rc = mf_build_tiles(A, nnz, s);
     if (rc != MF_SUCCESS) {
+        A->unsynced = 1;
         free_matrix(A);
         return rc;
     }
@@ -354,6 +355,7 @@ extern "C" int mf_solve(mf_matrix A, const double *b, double *x, const mf_option
     if (opt) o = *opt; else mf_options_default(&o);
     if (!(o.tol >= 0.0) || o.max_iter < 0) return MF_ERR_INVALID;
     if (A->n_rows != A->n_cols && A->n_cols < A->n_rows) return MF_ERR_INVALID;
+    CallMark mark(A);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t nb = (size_t)A->n_rows * sizeof(double);
     const double *db = b;
@@ -379,7 +381,7 @@ extern "C" int mf_solve(mf_matrix A, const double *b, double *x, const mf_option
         report->host_ms[0] = std::chrono::duration<double, std::milli>(t1 - t0).count();
         report->host_ms[3] = std::chrono::duration<double, std::milli>(clk::now() - t2).count();
     }
-    return rc;
+    return mark.end(rc);
 }
 
 extern "C" int mf_solve_multi(mf_matrix A, int nrhs, const double *B, double *X, const mf_options *opt,
@@ -395,6 +397,7 @@ extern "C" int mf_solve_multi(mf_matrix A, int nrhs, const double *B, double *X,
         // one column: the single-column kernel
         return mf_solve(A, B, X, &o, reports, device_ptrs, stream);
     }
+    CallMark mark(A);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t bytes = (size_t)nrhs * A->n_rows * sizeof(double);
     const double *dB = B;
@@ -411,7 +414,7 @@ extern "C" int mf_solve_multi(mf_matrix A, int nrhs, const double *B, double *X,
         cudaMemcpyAsync(X, dX, bytes, cudaMemcpyDeviceToHost, s);
         MF_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    return rc;
+    return mark.end(rc);
 }
 
 extern "C" int mf_batch_create(mf_batch *out, int nsys, const mf_matrix *systems, const int *nrhs, void *stream)
@@ -509,6 +512,7 @@ extern "C" int mf_spmv(mf_matrix A, const double *x, double *y, int precision, i
     NvtxRange nvtx_range("mf_spmv");
     if (!A || !x || !y) return MF_ERR_INVALID;
     if (precision != MF_PREC_FP64 && precision != MF_PREC_MIXED) return MF_ERR_INVALID;
+    CallMark mark(A);
     cudaStream_t s = (cudaStream_t)stream;
     const double *dxp = x;
     double *dyp = y;
@@ -524,12 +528,13 @@ extern "C" int mf_spmv(mf_matrix A, const double *x, double *y, int precision, i
         cudaMemcpyAsync(y, dyp, (size_t)A->n_rows * sizeof(double), cudaMemcpyDeviceToHost, s);
         MF_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    return rc;
+    return mark.end(rc);
 }
 
 extern "C" int mf_debug_spmv_tiles(mf_matrix A, const double *x, double *y, int tile_prec, int device_ptrs)
 {
     if (!A || !x || !y || tile_prec < 0 || tile_prec > 3) return MF_ERR_INVALID;
+    CallMark mark(A);
     const double *dxp = x;
     double *dyp = y, *tmp = nullptr;
     if (!device_ptrs) {
@@ -544,13 +549,14 @@ extern "C" int mf_debug_spmv_tiles(mf_matrix A, const double *x, double *y, int 
         if (rc == MF_SUCCESS) cudaMemcpy(y, dyp, (size_t)A->n_rows * sizeof(double), cudaMemcpyDeviceToHost);
         cudaFree(tmp);
     }
-    return rc;
+    return mark.end(rc);
 }
 
 extern "C" int mf_debug_spmm(mf_matrix A, const double *X, double *Y, int tensor_cores, int device_ptrs,
                              double *elapsed_ms)
 {
     if (!A || !X || !Y) return MF_ERR_INVALID;
+    CallMark mark(A);
     const size_t nx = (size_t)8 * A->n_cols, ny = (size_t)8 * A->n_rows;
     const double *dX = X;
     double *dY = Y, *tmp = nullptr;
@@ -562,7 +568,7 @@ extern "C" int mf_debug_spmm(mf_matrix A, const double *X, double *Y, int tensor
     }
     int rc = mf_spmm_run(A, dX, dY, tensor_cores ? 1 : 0, 0, elapsed_ms);
     if (!device_ptrs && rc == MF_SUCCESS) MF_CUDA_TRY(cudaMemcpy(Y, dY, ny * sizeof(double), cudaMemcpyDeviceToHost));
-    return rc;
+    return mark.end(rc);
 }
 
 extern "C" long long mf_debug_build_scratch(mf_matrix A) { return A ? A->build_scratch : -1; }
@@ -577,6 +583,7 @@ extern "C" int mf_spmv_noalloc(mf_matrix A, const double *x, double *y, int prec
 {
     if (!A || !x || !y) return MF_ERR_INVALID;
     if (precision != MF_PREC_FP64 && precision != MF_PREC_MIXED) return MF_ERR_INVALID;
+    A->unsynced = 1;          // returns before its kernel has run
     return mf_spmv_noalloc_run(A, x, y, precision, (cudaStream_t)stream);
 }
 

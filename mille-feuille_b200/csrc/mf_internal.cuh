@@ -93,6 +93,7 @@ struct mf_matrix_s {
     // tile-row ownership cost prefix for partitioning: [tilem+1]
     long long *d_row_cost;
     double build_ms;
+    int unsynced;              // work of an earlier call may still run: wait before arrays go (CallMark)
     long long build_scratch;   // largest global-memory scratch of a launch of the tile build, bytes
     // cached solver workspace
     void *ws;
@@ -138,6 +139,32 @@ void mf_set_last_cuda_error(cudaError_t e, const char *what, const char *file, i
 int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s);
 void mf_pool_free(void *p, cudaStream_t s);
 void mf_pool_settle(int dev);
+// memory of the current device that no work uses any more; mf_device_wait first where
+// some still may
+void mf_pool_give_back(void *const *p, int count);
+void mf_device_wait();
+
+// A call that uses a handle: it returns with its stream synchronised, or the handle
+// is marked and waits for the device before it gives memory back.  (The wait takes
+// 50 us; calls that fail half-way and mf_spmv_noalloc are the only ones that need it.)
+struct CallMark {
+    mf_matrix_s *A;
+    bool done = false;
+    explicit CallMark(mf_matrix_s *handle) : A(handle) {}
+    ~CallMark()
+    {
+        if (!done) A->unsynced = 1;
+    }
+    int end(int rc)
+    {
+        done = rc == MF_SUCCESS;
+        return rc;
+    }
+};
+inline void mf_handle_wait(const mf_matrix_s *A)
+{
+    if (A->unsynced) mf_device_wait();
+}
 template <typename T>
 inline int mf_pool_array(T **p, long long count, cudaStream_t s)
 {

@@ -896,8 +896,8 @@ int ws_multi(mf_matrix_s *A, Workspace *w, int mode, int nr, cudaStream_t s)
 {
     if (w->m_nr == nr && w->m_vec) return MF_SUCCESS;
     void *old[] = {w->m_vec, w->m_mag, w->m_red, w->m_hw_begin};
-    if (w->m_vec) MF_CUDA_TRY(cudaDeviceSynchronize());
-    for (void *p : old) mf_pool_free(p, 0);
+    if (w->m_vec) mf_handle_wait(A);
+    mf_pool_give_back(old, 4);
     w->m_vec = nullptr; w->m_mag = nullptr; w->m_red = nullptr;
     w->m_hw_begin = nullptr;
     w->m_nr = 0;
@@ -931,12 +931,12 @@ int ws_multi(mf_matrix_s *A, Workspace *w, int mode, int nr, cudaStream_t s)
 constexpr int kOutM = 4 * kMaxNR + 8;    // doubles per column group's result record
 
 // Result slots for `groups` column groups (grown, never shrunk).
-int ws_multi_groups(Workspace *w, int groups, cudaStream_t s)
+int ws_multi_groups(const mf_matrix_s *A, Workspace *w, int groups, cudaStream_t s)
 {
     if (w->m_groups >= groups) return MF_SUCCESS;
-    if (w->m_out) MF_CUDA_TRY(cudaDeviceSynchronize());
-    mf_pool_free(w->m_out, 0);
-    mf_pool_free(w->m_err, 0);
+    if (w->m_out) mf_handle_wait(A);
+    void *old[] = {w->m_out, w->m_err};
+    mf_pool_give_back(old, 2);
     w->m_out = nullptr;
     w->m_err = nullptr;
     for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
@@ -991,7 +991,7 @@ int mf_solver_multi_run(mf_matrix_s *A, int nrhs, const double *d_B, double *d_X
     M.mag = w->m_mag;
     M.red = w->m_red;
     const int groups = (nrhs + nr - 1) / nr;
-    MF_TRY(ws_multi_groups(w, groups, s));
+    MF_TRY(ws_multi_groups(A, w, groups, s));
     MF_CUDA_TRY(cudaMemsetAsync(w->m_out, 0, (size_t)groups * kOutM * sizeof(double), s));
     MF_CUDA_TRY(cudaMemsetAsync(w->m_err, 0, (size_t)groups * sizeof(int), s));
     // every column group is enqueued back to back (the interleaved buffers are
@@ -1069,6 +1069,17 @@ struct BatchImpl {
     int graph_mode = -1;
     cudaEvent_t e0 = nullptr, e1 = nullptr, e_in = nullptr;
     double last_ms = 0.0;
+    bool unsynced = false;             // a call failed half-way: its work may still run
+
+    // Ends a call: where it failed, the batch and its systems wait for the device
+    // before they give memory back.
+    int ended(int rc)
+    {
+        if (rc == MF_SUCCESS) return rc;
+        unsynced = true;
+        for (mf_matrix_s *A : sys) A->unsynced = 1;
+        return rc;
+    }
 
     void release_items()
     {
@@ -1077,8 +1088,9 @@ struct BatchImpl {
         graph_key.clear();
         void *p[] = {d_items, d_order, d_bptr, d_blist, d_ctl, d_pool};
         MfDeviceGuard guard(dev);
-        if (d_pool && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
-        for (void *q : p) mf_pool_free(q, 0);
+        if (unsynced) mf_device_wait();
+        unsynced = false;
+        mf_pool_give_back(p, 6);
         d_items = nullptr; d_order = nullptr; d_bptr = nullptr; d_blist = nullptr; d_ctl = nullptr;
         d_pool = nullptr;
     }
@@ -1392,6 +1404,7 @@ int mf_batch_create_impl(mf_batch_s **out, int nsys, mf_matrix_s *const *systems
         rc = MF_ERR_CUDA;
     if (rc == MF_SUCCESS) rc = batch_build_items(B, 8, 1, s ? s : B.own);
     if (rc != MF_SUCCESS) {
+        B.ended(rc);
         mf_batch_destroy_impl(b);
         return rc;
     }
@@ -1415,8 +1428,8 @@ void mf_batch_destroy_impl(mf_batch_s *b)
 // Solve every system's right-hand sides.  Bd[k] / Xd[k]: device arrays of
 // nrhs[k] x n_k doubles.  With use_graph the sequence is captured into a CUDA
 // graph on first use and replayed while pointers, options and items stay the same.
-int mf_batch_solve_impl(mf_batch_s *b, const double *const *Bd, double *const *Xd, const mf_options *opt,
-                        mf_report *reps, int use_graph, cudaStream_t s)
+static int batch_solve(mf_batch_s *b, const double *const *Bd, double *const *Xd, const mf_options *opt,
+                       mf_report *reps, int use_graph, cudaStream_t s)
 {
     BatchImpl &B = b->impl;
     if (opt->method != MF_METHOD_CG || opt->precision == MF_PREC_PARITY) return MF_ERR_UNSUPPORTED;
@@ -1536,6 +1549,12 @@ int mf_batch_solve_impl(mf_batch_s *b, const double *const *Bd, double *const *X
     return status;
 }
 
+int mf_batch_solve_impl(mf_batch_s *b, const double *const *Bd, double *const *Xd, const mf_options *opt,
+                        mf_report *reps, int use_graph, cudaStream_t s)
+{
+    return b->impl.ended(batch_solve(b, Bd, Xd, opt, reps, use_graph, s));
+}
+
 // Right-hand sides per work item chosen by timing: each candidate cap runs
 // `iters` fixed iterations of the real batch with all-ones right-hand sides.
 // A given (columns per item, blocks per SM), e.g. what mf_batch_tune chose for
@@ -1546,7 +1565,7 @@ int mf_batch_configure_impl(mf_batch_s *b, int cap, int lb, cudaStream_t s)
     if (cap != 1 && cap != 2 && cap != 4 && cap != 8) return MF_ERR_INVALID;
     // two blocks per SM only for items of up to 4 columns, as the tuner's candidates
     if (lb != 1 && !(lb == 2 && cap <= 4 && B.max_res[2] >= 1)) return MF_ERR_INVALID;
-    return batch_build_items(B, cap, lb, s ? s : B.own);
+    return B.ended(batch_build_items(B, cap, lb, s ? s : B.own));
 }
 
 void mf_batch_config_impl(const mf_batch_s *b, int *cap, int *lb)
@@ -1610,5 +1629,5 @@ int mf_batch_tune_impl(mf_batch_s *b, int precision, int iters, int *chosen, cud
         mf_pool_free(bufB[k], run);
     if (rc == MF_SUCCESS) rc = batch_build_items(B, best, best_lb, run);
     if (chosen) *chosen = best;
-    return rc;
+    return B.ended(rc);
 }

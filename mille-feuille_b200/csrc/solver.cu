@@ -100,7 +100,7 @@ int ws_get(mf_matrix_s *A, int blocks_per_sm, Workspace **out, cudaStream_t s)
     const int need = (A->tilem + kWarps * 2 - 1) / (kWarps * 2);
     if (need < G) G = need > 0 ? need : 1;
     if (w) {
-        MF_CUDA_TRY(cudaDeviceSynchronize());
+        mf_handle_wait(A);
         mf_solver_free_ws(A);
     }
     w = new Workspace();
@@ -281,13 +281,14 @@ VecWindow vec_window(const Workspace *w, int mode, int method, size_t matrix_byt
 
 }  // namespace
 
-// (the caller has synchronised the device)
+// (after mf_handle_wait)
 void mf_solver_free_ws(mf_matrix_s *A)
 {
     Workspace *w = (Workspace *)A->ws;
     if (!w) return;
-    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->hw_begin_cl, w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
-    for (void *p : ptrs) mf_pool_free(p, 0);
+    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->hw_begin_cl,
+                    w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
+    mf_pool_give_back(ptrs, (int)(sizeof(ptrs) / sizeof(ptrs[0])));
     for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
     delete[] w->m_ev;
     cudaEventDestroy(w->e0);
