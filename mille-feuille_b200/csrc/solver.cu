@@ -522,13 +522,31 @@ int spmv_launch(mf_matrix_s *A, const double *x, double *y, int tile_prec, cudaS
     return MF_SUCCESS;
 }
 
-// Whether x's n_cols doubles and y's n_rows doubles share memory: the product
-// is then formed from a copy of x.
-bool spmv_overlap(const mf_matrix_s *A, const double *x, const double *y)
+// Whether the product reads the caller's x where it is.  A kernel needs what a copy
+// does not: x on the handle's own device (or managed), on an 8-byte boundary, and
+// apart from y.  Otherwise x is copied first, which takes any alignment, another
+// GPU's memory and pinned host memory (whose gathers would each cross PCIe), and
+// refuses a pageable host pointer with an error where a kernel would fault.
+// (Asking costs 0.06 us.)
+bool spmv_in_place(const mf_matrix_s *A, const double *x, const double *y)
 {
     const uintptr_t x0 = (uintptr_t)x, x1 = x0 + (size_t)A->n_cols * sizeof(double);
     const uintptr_t y0 = (uintptr_t)y, y1 = y0 + (size_t)A->n_rows * sizeof(double);
-    return x0 < y1 && y0 < x1;
+    if ((x0 < y1 && y0 < x1) || x0 % sizeof(double) != 0) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, x) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == A->dev);
+}
+
+// x copied for a product; a refusal is this call's error, not the next launch's.
+cudaError_t spmv_copy(const mf_matrix_s *A, double *to, const double *x, cudaStream_t s)
+{
+    const cudaError_t e = cudaMemcpyAsync(to, x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 }  // namespace
@@ -536,7 +554,7 @@ bool spmv_overlap(const mf_matrix_s *A, const double *x, const double *y)
 // y = A x with every tile in one entry precision (MF_P64 .. MF_P8).  The kernel
 // reads the caller's x in place: it gathers no column past n_cols, so the padded
 // copy made before (33 MB moved and a 16.8 MB fill for 128^3: 20 of 75 us) is
-// needed only when y overlaps x.
+// needed only where spmv_in_place says so.
 int mf_spmv_tiles_run(mf_matrix_s *A, const double *d_x, double *d_y, int tile_prec, cudaStream_t s,
                       double *elapsed_ms)
 {
@@ -544,10 +562,9 @@ int mf_spmv_tiles_run(mf_matrix_s *A, const double *d_x, double *d_y, int tile_p
     for (cudaEvent_t &e : A->spmv_ev)
         if (!e) MF_CUDA_TRY(cudaEventCreate(&e));
     double *copy = nullptr;
-    if (spmv_overlap(A, d_x, d_y)) {
+    if (!spmv_in_place(A, d_x, d_y)) {
         MF_TRY(mf_pool_array(&copy, A->n_cols, s));
-        const cudaError_t e =
-            cudaMemcpyAsync(copy, d_x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s);
+        const cudaError_t e = spmv_copy(A, copy, d_x, s);
         if (e != cudaSuccess) mf_pool_free(copy, s);
         MF_CUDA_TRY(e);
         d_x = copy;
@@ -799,9 +816,9 @@ int mf_spmv_noalloc_run(mf_matrix_s *A, const double *d_x, double *d_y, int prec
     if (dev != A->dev) return MF_ERR_INVALID;
     double *x = nullptr;
     MF_TRY(noalloc_scratch(dev, &x));
-    // the scratch is needed only when y overlaps x
-    if (spmv_overlap(A, d_x, d_y)) {
-        MF_CUDA_TRY(cudaMemcpyAsync(x, d_x, (size_t)A->n_cols * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    // the scratch is needed only where x cannot be read in place
+    if (!spmv_in_place(A, d_x, d_y)) {
+        MF_CUDA_TRY(spmv_copy(A, x, d_x, s));
         d_x = x;
     }
     return spmv_launch(A, d_x, d_y, precision == MF_PREC_FP64 ? MF_P64 : MF_P32, s);
