@@ -476,68 +476,64 @@ __global__ void k_seg_shape(const int *__restrict__ tile_ptr, const int *__restr
     if (lane == 0 && longest > 0) atomicMax(&shape[0], longest);
 }
 
-// The slices' payload: lane i collects row i's next 8 entries (tile by tile) and
-// stores them as the 16-byte groups the solver loads (mf_slot), with zeros past the
-// row's end.  One entry at a time, with a warp per tile-row whose halves took alternate
-// slices (one of them idle on one-slice tile-rows), made 1- to 8-byte stores of six
-// arrays: 91 us for 7.1 M padded entries, 59 us now for 120 MB written and 92 MB read.
-__global__ void k_seg_fill(const int *__restrict__ tile_ptr, const int *__restrict__ seg_ptr,
-                           const int *__restrict__ seg_kp, const long long *__restrict__ seg_off,
-                           const int *__restrict__ csr_offset, const int *__restrict__ csrptr_offset,
-                           const unsigned char *__restrict__ tptr, const unsigned char *__restrict__ tcol,
-                           const double *__restrict__ tval, const float *__restrict__ tval_low,
-                           const int8_t *__restrict__ q8, const int8_t *__restrict__ q8ref, int tilem, int rowA,
+// The slices' payload, a half-warp per slice: lane i collects row i's next 8 entries
+// (tile by tile) and stores them as the 16-byte groups the solver loads (mf_slot),
+// with zeros past the row's end.  One entry at a time, with a warp per tile-row whose
+// halves took alternate slices (one of them idle on one-slice tile-rows), made 1- to
+// 8-byte stores of six arrays: 91 us for 7.1 M padded entries, 59 us now for 120 MB
+// written and 92 MB read.  By slice and not by tile-row: a tile-row of many slices
+// would be one half-warp's serial work.
+__global__ void k_seg_fill(const int4 *__restrict__ seg_hdr, const int *__restrict__ csr_offset,
+                           const int *__restrict__ csrptr_offset, const unsigned char *__restrict__ tptr,
+                           const unsigned char *__restrict__ tcol, const double *__restrict__ tval,
+                           const float *__restrict__ tval_low, const int8_t *__restrict__ q8,
+                           const int8_t *__restrict__ q8ref, int nseg, int tilem, int rowA,
                            unsigned char *__restrict__ meta, double *__restrict__ v64, float *__restrict__ v32,
                            __half *__restrict__ v16, int8_t *__restrict__ v8, int8_t *__restrict__ v8ref)
 {
-    const int nhw = (gridDim.x * blockDim.x) >> 4;      // a half-warp per tile-row
+    const int nhw = (gridDim.x * blockDim.x) >> 4;
     const int i = threadIdx.x & 15;
-    for (int R = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; R < tilem; R += nhw) {
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; s < nseg; s += nhw) {
+        const int4 h = seg_hdr[s];
+        const int R = h.y, ta = h.x, tb = ta + ((h.z >> 16) & 0xFF), kp = h.z & 0xFFFF;
         const int rowlen = (R == tilem - 1) ? rowA - R * MF_BS : MF_BS;
-        const int t0 = tile_ptr[R], t1 = tile_ptr[R + 1];
-        const int s0 = seg_ptr[R], s1 = seg_ptr[R + 1];
-        for (int s = s0; s < s1; s++) {
-            const int ta = t0 + (s - s0) * MF_SEG_TILES;
-            const int tb = min(t1, ta + MF_SEG_TILES);
-            const int kp = seg_kp[s];
-            const long long off = seg_off[s];
-            int t = i < rowlen ? ta : tb, e = 0, end = 0;
-            for (int k0 = 0; k0 < kp; k0 += 8) {
-                double d[8];
-                float f[8];
-                unsigned short hf[8];
-                unsigned long long m = 0, a8 = 0, r8 = 0;
+        const long long off = (long long)h.w << 7;
+        int t = i < rowlen ? ta : tb, e = 0, end = 0;
+        for (int k0 = 0; k0 < kp; k0 += 8) {
+            double d[8];
+            float f[8];
+            unsigned short hf[8];
+            unsigned long long m = 0, a8 = 0, r8 = 0;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    while (e >= end && t < tb) {          // the row's entries in the next tile
-                        const int cc = csrptr_offset[t], o = csr_offset[t], nnzt = csr_offset[t + 1] - o;
-                        e = o + tptr[cc + i];
-                        end = o + ((i == rowlen - 1) ? nnzt : (int)tptr[cc + i + 1]);
-                        t++;
-                    }
-                    d[j] = 0.0;
-                    f[j] = 0.0f;
-                    if (e < end) {
-                        d[j] = tval[e];
-                        f[j] = tval_low[e];
-                        m |= (unsigned long long)(unsigned char)(((t - 1 - ta) << 4) | tcol[e]) << (8 * j);
-                        a8 |= (unsigned long long)(unsigned char)q8[e] << (8 * j);
-                        r8 |= (unsigned long long)(unsigned char)q8ref[e] << (8 * j);
-                        e++;
-                    }
-                    hf[j] = __half_as_ushort(__float2half_rn(f[j]));
+            for (int j = 0; j < 8; j++) {
+                while (e >= end && t < tb) {          // the row's entries in the next tile
+                    const int cc = csrptr_offset[t], o = csr_offset[t], nnzt = csr_offset[t + 1] - o;
+                    e = o + tptr[cc + i];
+                    end = o + ((i == rowlen - 1) ? nnzt : (int)tptr[cc + i + 1]);
+                    t++;
                 }
-                const long long cb = off + (long long)(k0 >> 3) * 128;
-#pragma unroll
-                for (int q = 0; q < 4; q++) ((double2 *)(v64 + cb + 32 * q))[i] = make_double2(d[2 * q], d[2 * q + 1]);
-                ((float4 *)(v32 + cb))[i] = make_float4(f[0], f[1], f[2], f[3]);
-                ((float4 *)(v32 + cb + 64))[i] = make_float4(f[4], f[5], f[6], f[7]);
-                ((uint4 *)(v16 + cb))[i] = make_uint4(hf[0] | (unsigned)hf[1] << 16, hf[2] | (unsigned)hf[3] << 16,
-                                                      hf[4] | (unsigned)hf[5] << 16, hf[6] | (unsigned)hf[7] << 16);
-                ((unsigned long long *)(meta + cb))[i] = m;
-                ((unsigned long long *)(v8 + cb))[i] = a8;
-                ((unsigned long long *)(v8ref + cb))[i] = r8;
+                d[j] = 0.0;
+                f[j] = 0.0f;
+                if (e < end) {
+                    d[j] = tval[e];
+                    f[j] = tval_low[e];
+                    m |= (unsigned long long)(unsigned char)(((t - 1 - ta) << 4) | tcol[e]) << (8 * j);
+                    a8 |= (unsigned long long)(unsigned char)q8[e] << (8 * j);
+                    r8 |= (unsigned long long)(unsigned char)q8ref[e] << (8 * j);
+                    e++;
+                }
+                hf[j] = __half_as_ushort(__float2half_rn(f[j]));
             }
+            const long long cb = off + (long long)(k0 >> 3) * 128;
+#pragma unroll
+            for (int q = 0; q < 4; q++) ((double2 *)(v64 + cb + 32 * q))[i] = make_double2(d[2 * q], d[2 * q + 1]);
+            ((float4 *)(v32 + cb))[i] = make_float4(f[0], f[1], f[2], f[3]);
+            ((float4 *)(v32 + cb + 64))[i] = make_float4(f[4], f[5], f[6], f[7]);
+            ((uint4 *)(v16 + cb))[i] = make_uint4(hf[0] | (unsigned)hf[1] << 16, hf[2] | (unsigned)hf[3] << 16,
+                                                  hf[4] | (unsigned)hf[5] << 16, hf[6] | (unsigned)hf[7] << 16);
+            ((unsigned long long *)(meta + cb))[i] = m;
+            ((unsigned long long *)(v8 + cb))[i] = a8;
+            ((unsigned long long *)(v8ref + cb))[i] = r8;
         }
     }
 }
@@ -824,10 +820,10 @@ int mf_build_tiles(mf_matrix_s *A, long long nnz_given, cudaStream_t s)
         MF_CUDA_TRY(cudaGetLastError());
     }
     if (tilem > 0 && nseg > 0) {
-        k_seg_fill<<<grid_for((long long)tilem * MF_BS, kThreads), kThreads, 0, s>>>(A->d_tile_ptr, A->d_seg_ptr, A->d_seg_kp, A->d_seg_off,
-                                              A->d_csr_offset, A->d_csrptr_offset, A->d_tptr, A->d_tcol, A->d_tval,
-                                              A->d_tval_low, A->d_val_i8, A->d_val_i8_ref, tilem, rowA, A->d_meta,
-                                              A->d_v64, A->d_v32, A->d_v16, A->d_v8, A->d_v8ref);
+        k_seg_fill<<<grid_for((long long)nseg * MF_BS, kThreads), kThreads, 0, s>>>(
+            A->d_seg_hdr, A->d_csr_offset, A->d_csrptr_offset, A->d_tptr, A->d_tcol, A->d_tval, A->d_tval_low,
+            A->d_val_i8, A->d_val_i8_ref, nseg, tilem, rowA, A->d_meta, A->d_v64, A->d_v32, A->d_v16, A->d_v8,
+            A->d_v8ref);
         MF_CUDA_TRY(cudaGetLastError());
     }
     MF_CUDA_TRY(cudaStreamSynchronize(s));

@@ -111,6 +111,23 @@ def test_gpu_tiles_long_rows_have_bounded_scratch(mf, oracle_mod, cuda, n, rows)
     assert (scratch == 0) == (n == 2700)
 
 
+def test_gpu_slices_of_long_rows(mf, cuda):
+    """Tile-rows of one, two and many slices beside each other: products with the FP64,
+    FP32 and FP16 payload against the same stored values, within k eps of sum |a||x|
+    for a row of k entries (FP64 products and sums)."""
+    import scipy.sparse as sp
+    n = 20003
+    rowptr, colidx, val = _long_rows(n, [(5, 400), (40, 240), (41, 241), (9000, 700), (20001, n)],
+                                     np.random.default_rng(7))
+    G = mf.Matrix.from_csr(n, n, rowptr, colidx, val)
+    x = np.random.default_rng(8).standard_normal(n)
+    low = val.astype(np.float32)
+    for prec, stored in ((0, val), (1, low.astype(np.float64)), (2, low.astype(np.float16).astype(np.float64))):
+        S = sp.csr_matrix((stored, colidx, rowptr), shape=(n, n), copy=True)     # SciPy sorts its rows in place
+        bound = (np.diff(rowptr) + 1) * np.finfo(np.float64).eps * (abs(S) @ np.abs(x))
+        assert np.all(np.abs(G.spmv_tiles(x, prec) - S @ x) <= 2 * bound), prec
+
+
 def test_gpu_tiles_from_device_pointers(mf, oracle_mod, cuda):
     import torch
     from millefeuille import matrices as M
