@@ -96,6 +96,11 @@ namespace {
 void free_matrix(mf_matrix_s *A)
 {
     MfDeviceGuard guard(A->dev);
+    if (mf_context_gone(A->ctx)) {
+        mf_solver_free_ws(A, true);
+        delete A;
+        return;
+    }
     mf_handle_wait(A);
     mf_solver_free_ws(A);
     void *ptrs[] = {A->d_rowptr, A->d_colidx, A->d_val, A->d_val_low, A->d_tile_ptr, A->d_tile_columnidx,
@@ -140,6 +145,7 @@ int new_matrix(mf_matrix_s **out, int n_rows, int n_cols)
     mf_matrix_s *A = new mf_matrix_s();
     memset(A, 0, sizeof(*A));
     A->dev = dev;
+    A->ctx = mf_context();
     A->n_rows = n_rows;
     A->n_cols = n_cols;
     *out = A;

@@ -46,8 +46,16 @@
 #define MF_P8 3
 #define MF_PSKIP 4
 
+// The context a handle's memory belongs to: the driver's object and its id.  A
+// cudaDeviceReset keeps the object and changes the id.
+struct MfContext {
+    void *object;
+    unsigned long long id;
+};
+
 struct mf_matrix_s {
     int dev;
+    MfContext ctx;
     int n_rows, n_cols;        // as given
     long long nnz;             // entries in rows [0, n_rows)
     int tilem, tilen, tilenum;
@@ -139,6 +147,10 @@ void mf_set_last_cuda_error(cudaError_t e, const char *what, const char *file, i
 int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s);
 void mf_pool_free(void *p, cudaStream_t s);
 void mf_pool_settle(int dev);
+// the current device's context (pool.cu), and whether `c` has ended there with a
+// cudaDeviceReset, which has taken its memory, events and streams along
+MfContext mf_context();
+bool mf_context_gone(const MfContext &c);
 // memory of the current device that no work uses any more; mf_device_wait first where
 // some still may
 void mf_pool_give_back(void *const *p, int count);
@@ -231,7 +243,7 @@ int mf_spmm_run(mf_matrix_s *A, const double *d_X, double *d_Y, int tensor_cores
 int mf_spmv_noalloc_run(mf_matrix_s *A, const double *d_x, double *d_y, int precision, cudaStream_t s);
 int mf_ref_labels_run(const double *d_pold, const double *d_pnew, int nseg, int *d_vis,
                       cudaStream_t s);
-void mf_solver_free_ws(mf_matrix_s *A);
+void mf_solver_free_ws(mf_matrix_s *A, bool gone = false);   // gone: the device memory no longer exists
 int mf_ws_get(mf_matrix_s *A, int blocks_per_sm, void **out, cudaStream_t s);
 // solve_rows.cu: the solve kernel of a one-chunk matrix (mode: FP64 / mixed; its
 // longest row), and that file's bounds-check report

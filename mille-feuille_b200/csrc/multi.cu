@@ -1046,6 +1046,7 @@ int mf_solver_multi_run(mf_matrix_s *A, int nrhs, const double *d_B, double *d_X
 namespace {
 
 struct BatchImpl {
+    MfContext ctx = {nullptr, 0};
     int dev = 0, cap = 8, lb = 1, nitems = 0, nsm = 0;
     int max_res[3] = {0, 0, 0};        // co-resident blocks of the k_batch<*, lb> launch, lb = 1, 2
     std::vector<mf_matrix_s *> sys;
@@ -1083,14 +1084,16 @@ struct BatchImpl {
 
     void release_items()
     {
-        if (graph) cudaGraphExecDestroy(graph);
+        MfDeviceGuard guard(dev);
+        if (!mf_context_gone(ctx)) {
+            if (graph) cudaGraphExecDestroy(graph);
+            void *p[] = {d_items, d_order, d_bptr, d_blist, d_ctl, d_pool};
+            if (unsynced) mf_device_wait();
+            mf_pool_give_back(p, 6);
+        }
+        unsynced = false;
         graph = nullptr;
         graph_key.clear();
-        void *p[] = {d_items, d_order, d_bptr, d_blist, d_ctl, d_pool};
-        MfDeviceGuard guard(dev);
-        if (unsynced) mf_device_wait();
-        unsynced = false;
-        mf_pool_give_back(p, 6);
         d_items = nullptr; d_order = nullptr; d_bptr = nullptr; d_blist = nullptr; d_ctl = nullptr;
         d_pool = nullptr;
     }
@@ -1377,6 +1380,7 @@ int mf_batch_create_impl(mf_batch_s **out, int nsys, mf_matrix_s *const *systems
     if (cudaGetDevice(&B.dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&B.nsm, cudaDevAttrMultiProcessorCount, B.dev) != cudaSuccess)
         rc = MF_ERR_CUDA;
+    B.ctx = mf_context();
     if (rc == MF_SUCCESS) {
         // co-resident blocks of the cooperative launch (both precisions, both register budgets)
         int o[4] = {0, 0, 0, 0};
@@ -1417,11 +1421,14 @@ void mf_batch_destroy_impl(mf_batch_s *b)
     if (!b) return;
     BatchImpl &B = b->impl;
     B.release_items();
-    if (B.e0) cudaEventDestroy(B.e0);
-    if (B.e1) cudaEventDestroy(B.e1);
-    if (B.e_in) cudaEventDestroy(B.e_in);
-    if (B.own) cudaStreamDestroy(B.own);
-    mf_pool_settle(B.dev);
+    MfDeviceGuard guard(B.dev);
+    if (!mf_context_gone(B.ctx)) {
+        if (B.e0) cudaEventDestroy(B.e0);
+        if (B.e1) cudaEventDestroy(B.e1);
+        if (B.e_in) cudaEventDestroy(B.e_in);
+        if (B.own) cudaStreamDestroy(B.own);
+        mf_pool_settle(B.dev);
+    }
     delete b;
 }
 

@@ -24,25 +24,34 @@
 #include "mf_internal.cuh"
 
 #include <mutex>
+#include <vector>
 
 namespace {
 
 constexpr int kMaxDevices = 64;
 constexpr unsigned long long kKeepBytes = 1ull << 30;
 
+// One pool per device and context: a cudaDeviceReset ends the context's pool, and
+// the next handle makes another (entries of ended contexts stay, 32 bytes each).
 struct DevicePool {
+    int dev;
+    MfContext ctx;
     cudaMemPool_t pool;
     void *keep;                 // holds the small-allocation block that mf_device_wait uses
 };
 std::mutex g_mu;
-DevicePool g_pool[kMaxDevices];
+std::vector<DevicePool> g_pools;
 
-// The current device's pool, made on first use.
+// The pool of the current device `dev`, made on first use.
 int pool_of(int dev, DevicePool *out)
 {
     if (dev < 0 || dev >= kMaxDevices) return MF_ERR_UNSUPPORTED;
+    const MfContext ctx = mf_context();
     std::lock_guard<std::mutex> lock(g_mu);
-    if (!g_pool[dev].pool) {
+    const DevicePool *found = nullptr;
+    for (const DevicePool &d : g_pools)
+        if (d.dev == dev && d.ctx.object == ctx.object && d.ctx.id == ctx.id) found = &d;
+    if (!found) {
         cudaMemPoolProps pr = {};
         pr.allocType = cudaMemAllocationTypePinned;
         pr.location.type = cudaMemLocationTypeDevice;
@@ -57,9 +66,10 @@ int pool_of(int dev, DevicePool *out)
             cudaMemPoolDestroy(p);
             MF_CUDA_TRY(e);
         }
-        g_pool[dev] = {p, block};
+        g_pools.push_back({dev, ctx, p, block});
+        found = &g_pools.back();
     }
-    *out = g_pool[dev];
+    *out = *found;
     return MF_SUCCESS;
 }
 
@@ -79,7 +89,47 @@ void follow(cudaMemPool_t pool)
 
 constexpr size_t kFollowBytes = 4u << 20;    // allocations that move the threshold
 
+// The driver's calls for a context and its id (null where the driver has none).
+struct DriverCalls {
+    int (*current)(void **) = nullptr;
+    int (*id)(void *, unsigned long long *) = nullptr;
+    DriverCalls()
+    {
+        cudaDriverEntryPointQueryResult q;
+        void *f = nullptr, *g = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess && f &&
+            cudaGetDriverEntryPointByVersion("cuCtxGetId", &g, 12000, cudaEnableDefault, &q) == cudaSuccess && g) {
+            current = (int (*)(void **))f;
+            id = (int (*)(void *, unsigned long long *))g;
+        }
+        cudaGetLastError();
+    }
+};
+
 }  // namespace
+
+// 14 ns a driver call.  Where there is no context yet, or a reset has ended it,
+// cudaSetDevice makes one (no call that a stream capture forbids).
+MfContext mf_context()
+{
+    static const DriverCalls driver;
+    MfContext c = {nullptr, 0};
+    if (!driver.id) return c;
+    int dev = 0;
+    if (driver.id(nullptr, &c.id) != 0 &&
+        (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || driver.id(nullptr, &c.id) != 0)) {
+        cudaGetLastError();
+        return {nullptr, 0};
+    }
+    if (driver.current(&c.object) != 0) return {nullptr, 0};
+    return c;
+}
+
+bool mf_context_gone(const MfContext &c)
+{
+    const MfContext now = mf_context();
+    return now.id != c.id && (now.object == c.object || now.id == 0);
+}
 
 int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s)
 {
@@ -128,6 +178,7 @@ void mf_pool_give_back(void *const *p, int count)
 
 void mf_pool_settle(int dev)
 {
+    MfDeviceGuard guard(dev);
     DevicePool dp;
     unsigned long long used = 0, high = 0, held = 0, zero = 0;
     if (pool_of(dev, &dp) != MF_SUCCESS) return;

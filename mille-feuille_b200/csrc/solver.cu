@@ -282,17 +282,19 @@ VecWindow vec_window(const Workspace *w, int mode, int method, size_t matrix_byt
 }  // namespace
 
 // (after mf_handle_wait)
-void mf_solver_free_ws(mf_matrix_s *A)
+void mf_solver_free_ws(mf_matrix_s *A, bool gone)
 {
     Workspace *w = (Workspace *)A->ws;
     if (!w) return;
-    void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->hw_begin_cl,
-                    w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
-    mf_pool_give_back(ptrs, (int)(sizeof(ptrs) / sizeof(ptrs[0])));
-    for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
+    if (!gone) {
+        void *ptrs[] = {w->vecs, w->mag_p, w->mag_s, w->lab_p, w->lab_s, w->red, w->ctl, w->hw_begin, w->hw_begin_cl,
+                        w->m_vec, w->m_mag, w->m_red, w->m_out, w->m_err, w->m_hw_begin};
+        mf_pool_give_back(ptrs, (int)(sizeof(ptrs) / sizeof(ptrs[0])));
+        for (int k = 0; k < 2 * w->m_groups; k++) cudaEventDestroy(w->m_ev[k]);
+        cudaEventDestroy(w->e0);
+        cudaEventDestroy(w->e1);
+    }
     delete[] w->m_ev;
-    cudaEventDestroy(w->e0);
-    cudaEventDestroy(w->e1);
     delete w;
     A->ws = nullptr;
 }
