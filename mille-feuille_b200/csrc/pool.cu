@@ -10,8 +10,9 @@
 //
 // What the pool holds beyond live allocations is bounded: at most kKeepBytes
 // (the release threshold follows what is live, see follow(); more goes back at
-// the next synchronisation), and once nothing is live, at most what was live
-// since it was last empty (mf_pool_settle).  A failed allocation gives the rest back and tries again.
+// the next synchronisation and when a handle is destroyed), and once nothing is
+// live, at most what was live since it was last empty (mf_pool_settle).  A failed
+// allocation gives the rest back and tries again.
 // The pool is stream-ordered and safe with any number of threads.
 //
 // A handle's memory is given back the way cudaFree would, which the rest of a
@@ -23,7 +24,9 @@
 // stream, each was reused through an event: 55 us more a build).
 #include "mf_internal.cuh"
 
+#include <memory>
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 namespace {
@@ -32,44 +35,51 @@ constexpr int kMaxDevices = 64;
 constexpr unsigned long long kKeepBytes = 1ull << 30;
 
 // One pool per device and context: a cudaDeviceReset ends the context's pool, and
-// the next handle makes another (entries of ended contexts stay, 32 bytes each).
+// the next handle makes another (the entries of ended contexts stay).
 struct DevicePool {
     int dev;
     MfContext ctx;
     cudaMemPool_t pool;
-    void *keep;                 // holds the small-allocation block that mf_device_wait uses
+    void *keep;                      // holds the small-allocation block that mf_device_wait uses
+    unsigned long long live, high;   // bytes allocated now, and at most since none were
 };
-std::mutex g_mu;
-std::vector<DevicePool> g_pools;
+struct Allocation {
+    DevicePool *from;
+    size_t bytes;
+};
+std::mutex g_mu;                     // of all that follows
+std::vector<std::unique_ptr<DevicePool>> g_pools;
+// What is live is counted here: the driver's own count (UsedMemCurrent) leaves out
+// what cudaFree gives back.
+std::unordered_map<void *, Allocation> g_live;
 
 // The pool of the current device `dev`, made on first use.
-int pool_of(int dev, DevicePool *out)
+int pool_of(int dev, DevicePool **out)
 {
     if (dev < 0 || dev >= kMaxDevices) return MF_ERR_UNSUPPORTED;
     const MfContext ctx = mf_context();
     std::lock_guard<std::mutex> lock(g_mu);
-    const DevicePool *found = nullptr;
-    for (const DevicePool &d : g_pools)
-        if (d.dev == dev && d.ctx.object == ctx.object && d.ctx.id == ctx.id) found = &d;
-    if (!found) {
-        cudaMemPoolProps pr = {};
-        pr.allocType = cudaMemAllocationTypePinned;
-        pr.location.type = cudaMemLocationTypeDevice;
-        pr.location.id = dev;
-        cudaMemPool_t p = nullptr;
-        MF_CUDA_TRY(cudaMemPoolCreate(&p, &pr));
-        unsigned long long keep = kKeepBytes;
-        void *block = nullptr;
-        cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);   // nothing live yet
-        if (e == cudaSuccess) e = cudaMalloc(&block, 1);
-        if (e != cudaSuccess) {
-            cudaMemPoolDestroy(p);
-            MF_CUDA_TRY(e);
+    for (const auto &d : g_pools)
+        if (d->dev == dev && d->ctx.object == ctx.object && d->ctx.id == ctx.id) {
+            *out = d.get();
+            return MF_SUCCESS;
         }
-        g_pools.push_back({dev, ctx, p, block});
-        found = &g_pools.back();
+    cudaMemPoolProps pr = {};
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    MF_CUDA_TRY(cudaMemPoolCreate(&p, &pr));
+    unsigned long long keep = kKeepBytes;
+    void *block = nullptr;
+    cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);   // nothing live yet
+    if (e == cudaSuccess) e = cudaMalloc(&block, 1);
+    if (e != cudaSuccess) {
+        cudaMemPoolDestroy(p);
+        MF_CUDA_TRY(e);
     }
-    *out = *found;
+    g_pools.emplace_back(new DevicePool{dev, ctx, p, block, 0, 0});
+    *out = g_pools.back().get();
     return MF_SUCCESS;
 }
 
@@ -77,17 +87,22 @@ int pool_of(int dev, DevicePool *out)
 // live allocations included.  With a fixed one, handles above it (three 128^3
 // systems) had every freed array unmapped at the next synchronisation and mapped
 // again for the next solve (first solve of a handle 4.9 -> 8.5 ms).
-void follow(cudaMemPool_t pool)
+void follow(DevicePool *d)
 {
-    unsigned long long used = 0;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
-        used += kKeepBytes;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &used);
-    }
-    cudaGetLastError();
+    unsigned long long keep = d->live + kKeepBytes;
+    if (cudaMemPoolSetAttribute(d->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
 }
 
 constexpr size_t kFollowBytes = 4u << 20;    // allocations that move the threshold
+
+void count_free(void *p)
+{
+    std::lock_guard<std::mutex> lock(g_mu);
+    const auto it = g_live.find(p);
+    if (it == g_live.end()) return;
+    it->second.from->live -= it->second.bytes;
+    g_live.erase(it);
+}
 
 // The driver's calls for a context and its id (null where the driver has none).
 struct DriverCalls {
@@ -136,29 +151,36 @@ int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s)
     *p = nullptr;
     int dev = 0;
     MF_CUDA_TRY(cudaGetDevice(&dev));
-    DevicePool dp;
-    const int rc = pool_of(dev, &dp);
+    DevicePool *d = nullptr;
+    const int rc = pool_of(dev, &d);
     if (rc != MF_SUCCESS) return rc;
-    cudaMemPool_t pool = dp.pool;
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, s);
+    if (bytes == 0) bytes = 1;
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d->pool, s);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         mf_device_wait();
-        if (cudaMemPoolTrimTo(pool, 0) == cudaSuccess)
-            e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, s);
+        if (cudaMemPoolTrimTo(d->pool, 0) == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes, d->pool, s);
     }
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
     }
     MF_CUDA_TRY(e);
-    if (bytes >= kFollowBytes) follow(pool);
+    std::lock_guard<std::mutex> lock(g_mu);
+    g_live[*p] = {d, bytes};
+    d->live += bytes;
+    if (d->live > d->high) d->high = d->live;
+    if (bytes >= kFollowBytes) follow(d);
     return MF_SUCCESS;
 }
 
+// An address is taken off the list before it goes back: from then on another
+// thread may get it.
 void mf_pool_free(void *p, cudaStream_t s)
 {
-    if (p && cudaFreeAsync(p, s) != cudaSuccess) cudaGetLastError();
+    if (!p) return;
+    count_free(p);
+    if (cudaFreeAsync(p, s) != cudaSuccess) cudaGetLastError();
 }
 
 // cudaFree of an allocation of cudaMalloc waits for the whole device.
@@ -172,26 +194,26 @@ void mf_device_wait()
 
 void mf_pool_give_back(void *const *p, int count)
 {
-    for (int k = 0; k < count; k++)
-        if (p[k] && cudaFree(p[k]) != cudaSuccess) cudaGetLastError();
+    for (int k = 0; k < count; k++) {
+        if (!p[k]) continue;
+        count_free(p[k]);
+        if (cudaFree(p[k]) != cudaSuccess) cudaGetLastError();
+    }
 }
 
 void mf_pool_settle(int dev)
 {
     MfDeviceGuard guard(dev);
-    DevicePool dp;
-    unsigned long long used = 0, high = 0, held = 0, zero = 0;
-    if (pool_of(dev, &dp) != MF_SUCCESS) return;
-    cudaMemPool_t pool = dp.pool;
-    follow(pool);
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > 0 ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &high) != cudaSuccess ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    if (held > high) cudaMemPoolTrimTo(pool, (size_t)high);
-    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &zero);
+    DevicePool *d = nullptr;
+    unsigned long long held = 0;
+    if (pool_of(dev, &d) != MF_SUCCESS) return;
+    std::lock_guard<std::mutex> lock(g_mu);
+    follow(d);
+    const unsigned long long keep =
+        d->live > 0 ? d->live + kKeepBytes : d->high < kKeepBytes ? d->high : kKeepBytes;
+    if (cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess && held > keep)
+        cudaMemPoolTrimTo(d->pool, (size_t)keep);
+    if (d->live == 0) d->high = 0;
     cudaGetLastError();
 }
 
