@@ -328,24 +328,29 @@ int mf_spmv(mf_matrix A, const double *x, double *y, int precision, int device_p
  *    MF_PREC_FP64 or MF_PREC_MIXED (every tile in FP32), as for mf_spmv.
  *  - The call is asynchronous on `stream` (NULL: default stream); y is ready
  *    when the stream reaches that point.
- *  - Scratch: the padded copy of x lives in a fixed device buffer compiled
- *    into the library, MF_SPMV_NOALLOC_MAX_LEN doubles (16 MB per device).  Matrices whose padded vector length,
- *    16 * ceil(max(n_rows, n_cols) / 16), exceeds it are rejected with
- *    MF_ERR_UNSUPPORTED before anything is launched.
- *  - Nothing has to start at zero: each call writes every scratch entry the
- *    kernel reads (x, then zeros up to the padded length).
+ *  - x is read in place when it is memory of the matrix's device (or managed),
+ *    on an 8-byte boundary and apart from y; it must then stay valid and
+ *    unchanged until the stream has passed the call.  Otherwise (y over x among
+ *    others) it is first copied on the stream into a fixed device buffer compiled
+ *    into the library, MF_SPMV_NOALLOC_MAX_LEN doubles (16 MB per device).
+ *    Matrices whose padded vector length, 16 * ceil(max(n_rows, n_cols) / 16),
+ *    exceeds it are rejected with MF_ERR_UNSUPPORTED before anything is launched,
+ *    whichever way x goes.
  *  - The current device must be the one the matrix was created on
  *    (mf_matrix_info.device); otherwise the call returns MF_ERR_INVALID.
  *  - The first call on a device looks the buffer up (cudaGetSymbolAddress,
  *    which may load the library's device code); make that first call before
- *    any stream capture.  Later calls only issue a copy, a memset and the
- *    kernel.  The address is kept for the life of the loaded library: a
+ *    any stream capture.  Later calls only issue the kernel, and the copy where
+ *    one is needed.  The address is kept for the life of the loaded library: a
  *    cudaDeviceReset in the caller's process unloads the device code and
  *    leaves it stale, so after a reset the library must be unloaded and
- *    loaded again before this entry point is called.
- *  - One buffer per device is shared by all handles and threads: calls on
- *    the same device must not overlap in time (issue them on one stream, or
- *    order the streams), otherwise they race on the scratch.
+ *    loaded again before this entry point is called.  (All other entry points
+ *    work again after a reset, on handles and batches made after it; those made
+ *    before it can only be destroyed.)
+ *  - One buffer per device is shared by all handles and threads: calls on the
+ *    same device that copy x must not overlap in time (issue them on one stream,
+ *    or order the streams), otherwise they race on it.  Calls that read x in
+ *    place may overlap.
  */
 #define MF_SPMV_NOALLOC_MAX_LEN (1 << 21)
 int mf_spmv_noalloc(mf_matrix A, const double *x, double *y, int precision, void *stream);
@@ -364,8 +369,9 @@ int mf_spmv_noalloc(mf_matrix A, const double *x, double *y, int precision, void
 int mf_value_grad(mf_matrix A, int nrhs, const double *lambda, const double *x, double *grad_val,
                   int device_ptrs, void *stream);
 
-/* A handle for A^T (n_cols x n_rows), built from A's CSR; rows of A^T keep
- * A's row order (stable, deterministic).  Destroy it with mf_matrix_destroy. */
+/* A handle for A^T (n_cols x n_rows), built from A's CSR on the current device;
+ * rows of A^T keep A's row order (stable, deterministic).  Needs no more device
+ * memory than the handle itself does.  Destroy it with mf_matrix_destroy. */
 int mf_matrix_create_transposed(mf_matrix *out, mf_matrix A, void *stream);
 
 /* Test hook: segment labels of the reference rule for (p_old, p_new) device or
