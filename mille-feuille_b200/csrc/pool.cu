@@ -47,11 +47,12 @@ struct Allocation {
     DevicePool *from;
     size_t bytes;
 };
+// (Never destroyed: a program's static objects may give handles back at exit.)
 std::mutex g_mu;                     // of all that follows
-std::vector<std::unique_ptr<DevicePool>> g_pools;
+std::vector<std::unique_ptr<DevicePool>> &g_pools = *new std::vector<std::unique_ptr<DevicePool>>;
 // What is live is counted here: the driver's own count (UsedMemCurrent) leaves out
 // what cudaFree gives back.
-std::unordered_map<void *, Allocation> g_live;
+std::unordered_map<void *, Allocation> &g_live = *new std::unordered_map<void *, Allocation>;
 
 // The pool of the current device `dev`, made on first use.
 int pool_of(int dev, DevicePool **out)
@@ -151,6 +152,13 @@ int mf_pool_alloc(void **p, size_t bytes, cudaStream_t s)
     *p = nullptr;
     int dev = 0;
     MF_CUDA_TRY(cudaGetDevice(&dev));
+    // On a captured stream the allocation would become a node of the graph: an address
+    // without memory, kept by a handle whose call then fails at its synchronisation.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t cap = cudaStreamIsCapturing(s, &capture);
+    if (cap == cudaSuccess && capture != cudaStreamCaptureStatusNone) cap = cudaErrorStreamCaptureUnsupported;
+    if (cap != cudaSuccess) cudaGetLastError();
+    MF_CUDA_TRY(cap);
     DevicePool *d = nullptr;
     const int rc = pool_of(dev, &d);
     if (rc != MF_SUCCESS) return rc;
