@@ -145,9 +145,10 @@ struct SharedT {
 // One-cluster solves: the hardware's cluster barrier, with release / acquire of
 // everything the blocks wrote.  It waits for the threads of the cluster that
 // have not exited, and all of them run through the same barriers, so it needs no
-// limit of its own.
+// limit of its own.  `aligned` asks for whole warps: their lanes meet first.
 __device__ __forceinline__ void cluster_barrier()
 {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

@@ -35,6 +35,13 @@ def test_cluster_kernels_meet_before_the_first_remote_store():
     assert "if constexpr (CL) cluster_barrier();" in body[:first_use]
 
 
+def test_cluster_barrier_takes_whole_warps():
+    """`.aligned` barriers need every lane of a warp at the same instruction; lanes that
+    come from a branch (the stores of the first few) are not known to be."""
+    body = _body(_code("solver_dev.cuh"), "__device__ __forceinline__ void cluster_barrier()")
+    assert body.index("__syncwarp();") < body.index(".aligned")
+
+
 def test_multi_column_reductions_leave_between_two_barriers():
     """Every reduction over several columns copies its sums to registers between two
     block barriers, after its warps' half-warps have met."""
